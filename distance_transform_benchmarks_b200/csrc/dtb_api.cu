@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
     old = __shfl_sync(~0u, old, 0);
     const uint32_t img = old >> ST_IMG_SHIFT;
     const ImgDesc dd = descs[img];
-    const VisitBufs vb{sm.box[k], sm.Wh, sm.Wv, &sm.bar[k], &sm.mbar, 1u << k, 4u, &pbits};
+    const VisitBufs vb{sm.box[k], sm.Wh, sm.Wv, sm.E, &sm.bar[k], &sm.mbar, 1u << k, 4u, &pbits};
     uint32_t nph, nact;
     visit_ns<true>(dd, tmaps + 2 * img, tmaps + 2 * img + 1, cur, old, vb, sch, &nph, &nact);
     count_visit(ws, q, nph, nact);

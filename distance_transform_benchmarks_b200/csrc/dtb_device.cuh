@@ -103,34 +103,36 @@ struct Queue {
 };
 constexpr uint32_t KEY_NONE = 0xFFFFFFFFu;
 
-// Per-warp shared memory slot (14 KB: 12 warps per SM, the 168-register launch, fit in 228 KB).
-// Weight and tile buffers keep 36 floats a row.  A lane-per-column access ([k * 36 + lane]) is conflict-free; a
-// lane-per-row access ([lane * 36 + k]) is conflict-free as 16-byte vectors (the rows of a quarter-warp start in
-// 8 different 16-byte bank groups), so the row-layout phase moves its weights and the tile in 128-bit accesses:
-// 17 loads of weights instead of 65, 8 accesses instead of 32 on its side of each transpose (4 % faster than
-// 33-float rows with scalar accesses on the 1024-image batch).
-constexpr int W_STRIDE = TILE + 4;
+// Per-warp shared memory slot (13.4 KB: 16 warps per SM fit in 228 KB).
+// Weight and tile buffers keep 34 floats a row: a lane-per-column access ([k * 34 + lane]) is conflict-free, and so
+// is the sweeps' diagonal access ([lane * 34 + ((k +- lane) & 31)]: consecutive lanes are 33 or 35 words apart);
+// a lane-per-row access of one column, used only at the tile's borders, costs two wavefronts.
+constexpr int W_STRIDE = TILE + 2;
 constexpr int TILE_BUF_BYTES = TILE * W_STRIDE * 4;
 constexpr int IMG_REGION = IMG_BOX_ROWS * IMG_BOX_RGB > TILE_BUF_BYTES ? IMG_BOX_ROWS * IMG_BOX_RGB : TILE_BUF_BYTES;
+// Halo edge weights: 32 floats a side.
+constexpr int E_LEFT = 0, E_RIGHT = TILE, E_TOP = 2 * TILE, E_BOTTOM = 3 * TILE;
 struct alignas(128) WarpSmem {
   uint8_t img[IMG_REGION];                   // TMA destination of the image box (gray uses IMG_BOX_ROWS x 64); once
-                                             // the weights are computed, the tile buffer B[y * 36 + x]
-  float Wh[TILE * W_STRIDE];                 // ns-mode: Wh[y * 36 + x] = weight of edge (x-1, x) on row y, x = 0..32
-  float Wv[(TILE + 1) * W_STRIDE];           // ns-mode: Wv[y * 36 + x] = weight of edge (y-1, y) on column x, y = 0..32;
-                                             // its first 1 KB receives the seed-mask TMA box before the weights
+                                             // the weights are computed, the tile buffer B[y * 34 + x]
+  float Wh[TILE * W_STRIDE];                 // ns-mode: Wh[y * 34 + x] = weight of edge (x-1, x) on row y; INF at x = 0
+  float Wv[TILE * W_STRIDE];                 // ns-mode: Wv[y * 34 + x] = weight of edge (y-1, y) on column x; INF at
+                                             // y = 0; its first 1 KB receives the seed-mask TMA box before the weights
+  float E[4 * TILE];                         // ns-mode: weights of the edges to the halo, per side
   uint64_t bar;                              // TMA mbarrier
   uint32_t keep;                             // tile this warp keeps for its next visit (POP_NONE: none)
 };
 __device__ __forceinline__ uint8_t* mask_box(WarpSmem& sm) { return reinterpret_cast<uint8_t*>(sm.Wv); }
 
-// Per-warp shared memory of the staged-ahead tile kernel (17 KB: 12 warps per SM fit in 228 KB): the image
+// Per-warp shared memory of the staged-ahead tile kernel (18 KB: 12 warps per SM fit in 228 KB): the image
 // boxes of the tile being visited and of the warp's next tile, each the tile buffer B of its own visit once its
 // weights are computed; the weights; a barrier per box and one for the seed-mask box.
 constexpr int IMG_BOX_BYTES = IMG_REGION;
 struct alignas(128) WarpSmemP {
   uint8_t box[2][IMG_BOX_BYTES];
   float Wh[TILE * W_STRIDE];
-  float Wv[(TILE + 1) * W_STRIDE];   // its first 1 KB receives the seed-mask TMA box before the weights
+  float Wv[TILE * W_STRIDE];         // its first 1 KB receives the seed-mask TMA box before the weights
+  float E[4 * TILE];
   uint64_t bar[2];                   // image box k
   uint64_t mbar;                     // seed-mask box
 };
@@ -435,47 +437,61 @@ __device__ __forceinline__ float ref_relax(float dq, float eucl_d, float l_eucl,
 }
 
 // ------------------------------------------------------------------------------------------------------
-// One phase of the warp's tile in either layout.  Lane l holds a line of 32 pixels d[0..31] (a row in the
-// row layout, a column in the column layout); lanes l-1 / l+1 hold the neighbouring lines.
-//   chain edges  wc[k]: between positions k-1 and k of the own line (wc[0]: lo -> d[0], wc[32]: d[31] -> hi,
-//                where lo / hi are the halo pixels before and after the line);
-//   cross edges  wx[k]: between position k of line l-1 and position k of line l.
-// A forward chain walks k = 0..31 and a backward chain k = 31..0, interleaved (two independent dependency
-// chains).  At each step the chain pixel is first relaxed along the line (from its predecessor on the
-// chain), then across the lines from both neighbouring lanes, whose values at the same position are
-// exchanged by warp shuffles.  Every step is a set of single-edge relaxations fl(D + w): no two edge weights
-// are ever added before meeting a distance, so the result is the exact fixpoint whatever the order.  A chain
-// therefore follows any staircase path that moves at most one line per position, in both cross directions,
-// so one phase covers every monotone path of slope <= 1 along its axis.  Every internal edge of the tile is
-// relaxed in both directions during a phase: a phase that changes nothing proves the tile internally
-// converged.  The halo lines of the cross direction are not read here (lane 0 / 31 shuffle with themselves,
-// which never lowers a value); they are the chain halo of the other layout's phase.
+// One round of diagonal sweeps over the warp's tile.  Lane l holds row l of the tile, skewed: register j is pixel
+// x = (j + off_l) mod 32, with off_l = -l (layout A) or +l (layout B), so that register j runs over one
+// (anti)diagonal of the tile across the lanes.  The forward sweep walks j = 0..31: pixel (x, l) takes its
+// predecessor along the row from register j - 1 of its own lane and its predecessor along the column, which is
+// register j - 1 of lane `src_f` (l - 1 in layout A: down-right; l + 1 in layout B: up-right), by one shuffle.  The
+// reverse sweep walks j = 31..0 towards the opposite corner (from lane `src_r`), interleaved with the forward one
+// (two independent dependency chains).  The registers wrap: a lane whose row has reached its end goes on at its
+// start, so two rounds in a row complete both full sweeps (63 steps) for every lane, and no lane is idle.
+//   wh[j]: edge between pixels x - 1 and x of the row (INF at x = 0, which cuts the wrap);
+//   wv[j]: edge between this row and the row of lane `src_f` at x (INF where that row is across the tile's border,
+//          which also cuts the shuffles that wrap around the warp).
+// A path that moves only right and down (in any order, any slope) is followed from end to end by one forward sweep
+// in layout A, and likewise the other three quadrants.  Shortest paths inside a tile are nearly always of that kind,
+// so a visit needs about 3 rounds (of 32 steps) where sweeps along rows and columns alone, which follow
+// slopes up to 1, needed 6.4 phases of the same length (1024-image batch).
+// Every step is a set of single-edge relaxations fl(D + w): no two edge weights are ever added before meeting a
+// distance, so the fixpoint is exact whatever the order.  In one round every internal edge is relaxed in both
+// directions: a round that changes nothing proves the tile internally converged.
 // ------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool sweep_phase(float (&d)[TILE], const float (&wc)[TILE + 1], const float (&wx)[TILE], float lo,
-                                            float hi) {
+__device__ __forceinline__ bool skew_round(float (&d)[TILE], const float (&wh)[TILE], const float (&wv)[TILE], int src_f,
+                                           int src_r) {
   bool ch = false;
-  float f = lo, b = hi;
 #pragma unroll
-  for (int k = 0; k < TILE; ++k) {
-    const int i = k, j = TILE - 1 - k;
-    const float di = d[i];
-    const float a = fminf(di, __fadd_rn(f, wc[i]));
-    const float from_prev = __shfl_up_sync(~0u, a, 1);
-    const float from_next = __shfl_down_sync(~0u, __fadd_rn(a, wx[i]), 1);
-    const float c = fminf(a, fminf(__fadd_rn(from_prev, wx[i]), from_next));
-    ch |= c < di;
-    d[i] = c;
-    f = c;
-    const float dj = d[j];
-    const float e = fminf(dj, __fadd_rn(b, wc[j + 1]));
-    const float from_prev2 = __shfl_up_sync(~0u, e, 1);
-    const float from_next2 = __shfl_down_sync(~0u, __fadd_rn(e, wx[j]), 1);
-    const float g = fminf(e, fminf(__fadd_rn(from_prev2, wx[j]), from_next2));
-    ch |= g < dj;
-    d[j] = g;
-    b = g;
+  for (int s = 0; s < TILE; ++s) {
+    {
+      const int j = s, p = (s + TILE - 1) % TILE;
+      const float q = d[p];
+      const float up = __shfl_sync(~0u, q, src_f);
+      const float c = fminf(fminf(d[j], __fadd_rn(q, wh[j])), __fadd_rn(up, wv[j]));
+      ch |= c < d[j];
+      d[j] = c;
+    }
+    {
+      const int j = TILE - 1 - s, n = (TILE - s) % TILE;
+      const float q = d[n];
+      const float dn = __shfl_sync(~0u, __fadd_rn(q, wv[n]), src_r);
+      const float c = fminf(fminf(d[j], __fadd_rn(q, wh[n])), dn);
+      ch |= c < d[j];
+      d[j] = c;
+    }
   }
   return ch;
+}
+
+// A lane's row of a W_STRIDE buffer in the skewed order (register j = element (j + off) mod 32, 0 <= off < 32).
+__device__ __forceinline__ void load_skew(float (&r)[TILE], const float* row, int off) {
+  const float* p = row + off;
+#pragma unroll
+  for (int j = 0; j < TILE; ++j) r[j] = (off >= TILE - j ? p - TILE : p)[j];
+}
+__device__ __forceinline__ void store_skew(float* row, int off, const float (&r)[TILE]) {
+  asm("" : "+r"(off) : "f"(r[0]));  // or the addresses of the loads would be kept in registers through the rounds
+  float* p = row + off;
+#pragma unroll
+  for (int j = 0; j < TILE; ++j) (off >= TILE - j ? p - TILE : p)[j] = r[j];
 }
 
 }  // namespace dtb

@@ -198,6 +198,7 @@ struct VisitBufs {
   uint8_t* box;       // image box (TMA destination), the tile buffer B once the weights are computed
   float* Wh;
   float* Wv;          // its first 1 KB receives the seed-mask box before the weights
+  float* E;
   uint64_t* bar;
   uint64_t* mbar;
   uint32_t pmask;     // bit of *pbits holding bar's phase parity
@@ -206,7 +207,7 @@ struct VisitBufs {
 };
 
 __device__ __forceinline__ VisitBufs visit_bufs(WarpSmem& sm, uint32_t& pbits) {
-  return VisitBufs{sm.img, sm.Wh, sm.Wv, &sm.bar, &sm.bar, 1u, 1u, &pbits};
+  return VisitBufs{sm.img, sm.Wh, sm.Wv, sm.E, &sm.bar, &sm.bar, 1u, 1u, &pbits};
 }
 
 // Issues one 2-D TMA box into this warp's shared memory on `bar` (whole warp; lane 0 issues).  Orders this
@@ -265,44 +266,29 @@ __device__ __forceinline__ uint32_t box_pix(const uint8_t* box, bool rgb, int r,
   return __funnelshift_r(wp[0], wp[1], (off & 3) * 8) & 0xFFFFFFu;
 }
 
-// A lane's row of 32 floats of a W_STRIDE buffer (16-byte aligned), as 8 vector loads / stores.
-__device__ __forceinline__ void load_row(float (&d)[TILE], const float* row) {
-  const float4* p = reinterpret_cast<const float4*>(row);
-#pragma unroll
-  for (int j = 0; j < TILE / 4; ++j) {
-    const float4 v4 = p[j];
-    d[4 * j] = v4.x; d[4 * j + 1] = v4.y; d[4 * j + 2] = v4.z; d[4 * j + 3] = v4.w;
-  }
-}
-__device__ __forceinline__ void store_row(float* row, const float (&d)[TILE]) {
-  float4* p = reinterpret_cast<float4*>(row);
-#pragma unroll
-  for (int j = 0; j < TILE / 4; ++j) p[j] = make_float4(d[4 * j], d[4 * j + 1], d[4 * j + 2], d[4 * j + 3]);
-}
-
 // ------------------------------------------------------------------------------------------------------
 // ns-mode visit (C4, w = sqrt(1 + g2 * dI2)), gray or rgb8.
 //
-// Layouts: "column" (lane = x, d[y]) and "row" (lane = y, d[x]).  Each phase (sweep_phase) relaxes every
-// internal edge of the tile and the halo edges of its own axis; the halo edges of the other axis were relaxed
-// by an earlier phase and stay satisfied, because tile values only decrease while the halo is fixed.  So the
-// visit stops at the first phase that changes nothing once both layouts have run: every edge of the tile and
-// its halo is then satisfied.  The halo is an upper bound of the neighbours' values (values only decrease;
-// never-visited neighbours read as v), so the visit never undershoots the fixpoint.  A neighbour is
-// re-activated only if some border pixel plus its edge weight is below the halo value it was compared with.
+// The tile's distances are relaxed from the halo once (values only decrease while the halo is fixed, so the halo
+// edges stay satisfied), then by rounds of diagonal sweeps (skew_round) until a round changes nothing: every edge
+// of the tile and its halo is then satisfied.  A visit whose halo lowers nothing runs no round unless it applies
+// seeds.  The halo is an upper bound of the neighbours' values (values only decrease; never-visited neighbours read
+// as v), so the visit never undershoots the fixpoint.  A neighbour is re-activated only if some border pixel plus
+// its edge weight is below the halo value it was compared with.
 //
-// One code path serves both layouts (the phase loop is small enough to stay in the instruction cache): the
-// weights live in shared memory as Wh / Wv (stride 36: scalar lane-per-column reads and 16-byte lane-per-row
-// reads are conflict-free) and are loaded into registers for the phase's layout; the tile changes layout through
-// B.  Element k of lane l is at [k * 36 + l] of the row-major arrays in the column layout (scalar loads), at
-// [l * 36 + k] in the row layout (16-byte vectors).
-// Returns the number of phases and activations through *nph / *nact.
+// The rounds run in one of two skewed layouts (A: the down-right and up-left quadrants, B: the other two); the visit
+// starts in the one whose corners hold the smallest border value, where the front comes in, and changes after
+// LAYOUT_ROUNDS rounds without convergence (about one visit in five; changing after 2 rounds saved 5 % of the
+// rounds and cost four times the reloads).
+// Returns the number of rounds and activations through *nph / *nact.
 //
 // rerun: the warp visits again the tile it has just visited (its halo dropped while it ran, and the visit kept
-// it).  The warp's shared memory still holds that tile's edge weights (Wh / Wv) and its final distances (the
+// it).  The warp's shared memory still holds that tile's edge weights (Wh / Wv / E) and its final distances (the
 // tile buffer B, equal to the tile in global memory: no other warp can have visited it in between), so the
 // re-run reloads only the neighbour states and halos: no bulk copy, no weights, no tile loads.
 // ------------------------------------------------------------------------------------------------------
+constexpr int LAYOUT_ROUNDS = 3;
+
 template <bool PRESTAGED, class Sched>
 __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* tm_img, const CUtensorMap* tm_mask,
                                          uint32_t tile, uint32_t old_state, const VisitBufs& vb, const Sched& sch,
@@ -370,24 +356,24 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
 
   // Seeds first: the mask box shares memory with Wv.
   if (first) {
+    const bool in = lane < vw;
 #pragma unroll
-    for (int y = 0; y < TILE; ++y) {
-      const bool in = lane < vw && y < vh;
-      const bool s = seed && mbox[y * TILE + lane] != 0;
-      d[y] = in ? (s ? 0.0f : v) : INF;
-    }
-  } else if (seed) {
+    for (int y = 0; y < TILE; ++y) d[y] = in && y < vh ? v : INF;
+  }
+  if (seed) {
 #pragma unroll
     for (int y = 0; y < TILE; ++y)
       if (lane < vw && y < vh && mbox[y * TILE + lane] != 0) d[y] = 0.0f;
   }
   __syncwarp();
 
-  // Edge weights into Wh / Wv (computed in column layout, lane = x).  Edges touching a pixel outside the image
-  // are INF.  A re-run has them from its previous visit.
+  // Edge weights into Wh / Wv / E (lane = x; the left and right halo edges lane = y).  A re-run has them.
+  const uint32_t img_idx = old_state >> ST_IMG_SHIFT;
+  float wsum = 0.0f;
   if (!rerun) {
     const float g2 = dd.g2;
     const uint8_t* box = vb.box;
+    float et, eb, el, er;
     if (!rgb) {
       // Gray: the weight depends on |dI| in [0, 255] only.  A 256-entry table of the same expression (so the
       // same bits) costs 8 square roots per lane instead of 65; it sits in the part of the image box that the
@@ -400,69 +386,76 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
       }
       __syncwarp();
       const uint8_t* col = box + 16 + lane;  // column `lane` of the box, row r at col[r * IMG_BOX_GRAY]
-      int pprev = col[0];
-      // Unrolled 2: the 1024-image batch ran 0.7 % faster than with 4 (8 was 2.4 % slower).
+      int pprev = col[IMG_BOX_GRAY];
+      et = lut[abs(pprev - (int)col[0])];
+      vb.Wv[lane] = INF;
+      vb.Wh[lane] = lane == 0 ? INF : lut[abs(pprev - (int)col[IMG_BOX_GRAY - 1])];
 #pragma unroll 2
-      for (int y = 0; y <= TILE; ++y) {  // edge (y-1, y); y == 32 is the bottom halo edge
+      for (int y = 1; y < TILE; ++y) {
         const int pcur = col[(y + 1) * IMG_BOX_GRAY];
-        float w = lut[abs(pcur - pprev)];
-        if (lane >= vw || (y < TILE ? y >= vh : TILE - 1 >= vh)) w = INF;
+        const float w = lut[abs(pcur - pprev)];
+        const float wx = lut[abs(pcur - (int)col[(y + 1) * IMG_BOX_GRAY - 1])];
         vb.Wv[y * W_STRIDE + lane] = w;
-        if (y < TILE) {
-          float wx = lut[abs(pcur - (int)col[(y + 1) * IMG_BOX_GRAY - 1])];
-          if (lane >= vw || y >= vh) wx = INF;
-          vb.Wh[y * W_STRIDE + lane] = wx;
-        }
+        vb.Wh[y * W_STRIDE + lane] = lane == 0 ? INF : wx;
+        if (lane < vw && y < vh) wsum += w;
         pprev = pcur;
       }
+      eb = lut[abs((int)col[(TILE + 1) * IMG_BOX_GRAY] - pprev)];
       const uint8_t* row = box + (lane + 1) * IMG_BOX_GRAY + 16;
-      float er = lut[abs((int)row[TILE - 1] - (int)row[TILE])];
-      if (lane >= vh || TILE - 1 >= vw) er = INF;
-      vb.Wh[lane * W_STRIDE + TILE] = er;
+      el = lut[abs((int)row[0] - (int)row[-1])];
+      er = lut[abs((int)row[TILE] - (int)row[TILE - 1])];
     } else {
-      uint32_t pprev = box_pix(box, rgb, 0, lane);
-#pragma unroll 1
-      for (int y = 0; y <= TILE; ++y) {  // edge (y-1, y); y == 32 is the bottom halo edge
-        const uint32_t pcur = box_pix(box, rgb, y + 1, lane);
-        float w = ns_weight(pprev, pcur, g2);
-        if (lane >= vw || (y < TILE ? y >= vh : TILE - 1 >= vh)) w = INF;
+      uint32_t pprev = box_pix(box, true, 1, lane);
+      et = ns_weight(box_pix(box, true, 0, lane), pprev, g2);
+      vb.Wv[lane] = INF;
+      {
+        const float wx = ns_weight(__shfl_up_sync(~0u, pprev, 1), pprev, g2);
+        vb.Wh[lane] = lane == 0 ? INF : wx;
+      }
+#pragma unroll 2
+      for (int y = 1; y < TILE; ++y) {
+        const uint32_t pcur = box_pix(box, true, y + 1, lane);
+        const float w = ns_weight(pprev, pcur, g2);
+        const float wx = ns_weight(__shfl_up_sync(~0u, pcur, 1), pcur, g2);
         vb.Wv[y * W_STRIDE + lane] = w;
-        if (y < TILE) {
-          float wx = ns_weight(box_pix(box, rgb, y + 1, lane - 1), pcur, g2);
-          if (lane >= vw || y >= vh) wx = INF;
-          vb.Wh[y * W_STRIDE + lane] = wx;
-        }
+        vb.Wh[y * W_STRIDE + lane] = lane == 0 ? INF : wx;
+        if (lane < vw && y < vh) wsum += w;
         pprev = pcur;
       }
-      // Edge (x = 31, x = 32) of row `lane`.
-      float er = ns_weight(box_pix(box, rgb, lane + 1, TILE - 1), box_pix(box, rgb, lane + 1, TILE), g2);
-      if (lane >= vh || TILE - 1 >= vw) er = INF;
-      vb.Wh[lane * W_STRIDE + TILE] = er;
+      eb = ns_weight(pprev, box_pix(box, true, TILE + 1, lane), g2);
+      el = ns_weight(box_pix(box, true, lane + 1, -1), box_pix(box, true, lane + 1, 0), g2);
+      er = ns_weight(box_pix(box, true, lane + 1, TILE - 1), box_pix(box, true, lane + 1, TILE), g2);
     }
+    if (vw < TILE || vh < TILE) {  // edges touching a pixel outside the image are INF
+#pragma unroll 1
+      for (int y = 0; y < TILE; ++y)
+        if (lane >= vw || y >= vh) {
+          vb.Wh[y * W_STRIDE + lane] = INF;
+          vb.Wv[y * W_STRIDE + lane] = INF;
+        }
+      if (lane >= vw) et = INF;
+      if (lane >= vw || vh < TILE) eb = INF;
+      if (lane >= vh) el = INF;
+      if (lane >= vh || vw < TILE) er = INF;
+    }
+    vb.E[E_LEFT + lane] = el;
+    vb.E[E_RIGHT + lane] = er;
+    vb.E[E_TOP + lane] = et;
+    vb.E[E_BOTTOM + lane] = eb;
   }
   __syncwarp();
 
   // Bucket width of this image: one tile-width of path cost, 32 x the mean internal edge weight seen so far by
   // first visits (each first visit adds its column edges).
-  const uint32_t img_idx = old_state >> ST_IMG_SHIFT;
   float inv_width = 0.0f;
   if (sch.q.wacc) {
     float* wa = sch.q.wacc + 2 * img_idx;
     if (first) {
-      float wsum = 0.0f, wcnt = 0.0f;
-#pragma unroll 4
-      for (int y = 1; y < TILE; ++y) {
-        const float w = vb.Wv[y * W_STRIDE + lane];
-        if (w < INF) { wsum += w; wcnt += 1.0f; }
-      }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        wsum += __shfl_xor_sync(~0u, wsum, o);
-        wcnt += __shfl_xor_sync(~0u, wcnt, o);
-      }
-      if (lane == 0 && wcnt > 0.0f) {
+      for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(~0u, wsum, o);
+      if (lane == 0 && vh > 1) {
         atomicAdd(&wa[0], wsum);
-        atomicAdd(&wa[1], wcnt);
+        atomicAdd(&wa[1], (float)(vw * (vh - 1)));
       }
     }
     const float s_ = *(volatile float*)&wa[0], c_ = *(volatile float*)&wa[1];
@@ -470,81 +463,64 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     inv_width = (c_ > 0.0f && s_ > 0.0f) ? c_ / (bt * (float)TILE * s_) : 1.0f / (bt * (float)TILE);
   }
 
-  // Local fixpoint.  B overlays the image box, which is no longer needed.
+  // The tile buffer B overlays the image box, which is no longer needed.  Relax the halo edges in it: top and bottom
+  // lane = x, then left and right lane = y.
   float* B = reinterpret_cast<float*>(vb.box);
-  // Start in the layout whose chains begin at the halo sides that can lower the tile now: a column phase
-  // never reads the left / right halo, so a tile reached only from the side would spend its first column
-  // phase without any effect.
-  bool col = true;
-  // hside / vside: whether the left / right (top / bottom) halo can lower the tile as it stands.  A phase that
-  // changes nothing proves every internal edge and its own axis's halo edges satisfied; if the first phase
-  // changes nothing and the other axis's halo could not lower the unchanged tile, the tile is at its fixpoint
-  // and the visit ends after that one phase (a false-positive activation costs one phase, not two).
-  bool hside, vside;
-  {
+  const float* E = vb.E;
+  if (!rerun) {
     float* pb = B + lane;
 #pragma unroll
     for (int k = 0; k < TILE; ++k) pb[k * W_STRIDE] = d[k];
     __syncwarp();
-    const float dl = B[lane * W_STRIDE], dr = B[lane * W_STRIDE + TILE - 1];
-    hside = __any_sync(~0u, __fadd_rn(lft, vb.Wh[lane * W_STRIDE]) < dl ||
-                                 __fadd_rn(rgt, vb.Wh[lane * W_STRIDE + TILE]) < dr);
-    vside = __any_sync(~0u, __fadd_rn(top, vb.Wv[lane]) < d[0] ||
-                                 __fadd_rn(bot, vb.Wv[TILE * W_STRIDE + lane]) < d[TILE - 1]);
-    if (hside && !vside) {
-      col = false;
-      load_row(d, B + lane * W_STRIDE);
-    }
+  }
+  bool any, layout_a;
+  {
+    const float ct = __fadd_rn(top, E[E_TOP + lane]), cb = __fadd_rn(bot, E[E_BOTTOM + lane]);
+    float dt = B[lane], db = B[(TILE - 1) * W_STRIDE + lane];
+    bool low = ct < dt || cb < db;
+    dt = fminf(dt, ct);
+    db = fminf(db, cb);
+    B[lane] = dt;
+    B[(TILE - 1) * W_STRIDE + lane] = db;
+    __syncwarp();
+    const float cl = __fadd_rn(lft, E[E_LEFT + lane]), cr = __fadd_rn(rgt, E[E_RIGHT + lane]);
+    float dl = B[lane * W_STRIDE], dr = B[lane * W_STRIDE + TILE - 1];
+    low |= cl < dl || cr < dr;
+    dl = fminf(dl, cl);
+    dr = fminf(dr, cr);
+    B[lane * W_STRIDE] = dl;
+    B[lane * W_STRIDE + TILE - 1] = dr;
+    any = __any_sync(~0u, low);
+    // The smallest border value near the corners of either diagonal (float bits order like the values, all >= 0).
+    const float tl = fminf(dt, dl), br = fminf(db, dr);
+    const uint32_t ka = __reduce_min_sync(~0u, __float_as_uint(lane < TILE / 2 ? tl : br));
+    const uint32_t kb = __reduce_min_sync(~0u, __float_as_uint(lane < TILE / 2 ? fminf(db, dr) : fminf(dt, dl)));
+    layout_a = ka <= kb;
     __syncwarp();
   }
-  bool any = false, ran_col = false, ran_row = false;
   uint32_t nph = 0;
-  for (;;) {
-    float wc[TILE + 1], wx[TILE];
-    if (col) {  // element k of lane x: [k * 36 + x]
-      const float* pc = vb.Wv + lane;
-      const float* px = vb.Wh + lane;
-#pragma unroll
-      for (int k = 0; k <= TILE; ++k) wc[k] = pc[k * W_STRIDE];
-#pragma unroll
-      for (int k = 0; k < TILE; ++k) wx[k] = px[k * W_STRIDE];
-    } else {    // element k of lane y: [y * 36 + k], as 16-byte vectors
-      const float4* pc = reinterpret_cast<const float4*>(vb.Wh + lane * W_STRIDE);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 v4 = pc[j];
-        wc[4 * j] = v4.x; wc[4 * j + 1] = v4.y; wc[4 * j + 2] = v4.z; wc[4 * j + 3] = v4.w;
-      }
-      wc[TILE] = pc[8].x;
-      load_row(wx, vb.Wv + lane * W_STRIDE);
-    }
-    bool ch = sweep_phase(d, wc, wx, col ? top : lft, col ? bot : rgt);
-    ch = __any_sync(~0u, ch);
-    any |= ch;
-    ran_col |= col;
-    ran_row |= !col;
-    ++nph;
-    const bool stop = (!ch && ((ran_col && ran_row) || (nph == 1 && !(col ? hside : vside)))) ||
-                      nph >= (uint32_t)PHASE_LIMIT;
-    if (col) {
-      float* pb = B + lane;
-#pragma unroll
-      for (int k = 0; k < TILE; ++k) pb[k * W_STRIDE] = d[k];
+  if (any || seed) {
+    for (;;) {
+      const int off = layout_a ? (TILE - lane) % TILE : lane;
+      const int src_f = (layout_a ? lane + TILE - 1 : lane + 1) % TILE, src_r = (layout_a ? lane + 1 : lane + TILE - 1) % TILE;
+      float wh[TILE], wv[TILE];
+      load_skew(wh, vb.Wh + lane * W_STRIDE, off);
+      load_skew(wv, vb.Wv + (layout_a ? lane : src_f) * W_STRIDE, off);
+      load_skew(d, B + lane * W_STRIDE, off);
+      bool ch;
+      int r = 0;
+      do {
+        ch = __any_sync(~0u, skew_round(d, wh, wv, src_f, src_r));
+        any |= ch;
+        ++nph;
+      } while (ch && ++r < LAYOUT_ROUNDS);
+      store_skew(B + lane * W_STRIDE, off, d);
       __syncwarp();
-      if (stop) break;
-      load_row(d, B + lane * W_STRIDE);
-    } else {
-      store_row(B + lane * W_STRIDE, d);
-      __syncwarp();
-      if (stop) break;
-      const float* qb = B + lane;
-#pragma unroll
-      for (int k = 0; k < TILE; ++k) d[k] = qb[k * W_STRIDE];
+      if (!ch || nph >= (uint32_t)PHASE_LIMIT) break;
+      layout_a = !layout_a;
     }
-    col = !col;
-    __syncwarp();
+    if (nph >= (uint32_t)PHASE_LIMIT && lane == 0) set_error(sch.q, DERR_PHASE_LIMIT, tile);
   }
-  if (nph >= (uint32_t)PHASE_LIMIT && lane == 0) set_error(sch.q, DERR_PHASE_LIMIT, tile);
 
   // Neighbours that can still decrease (bit 0 left, 1 right, 2 top, 3 bottom).
   uint32_t act = 0;
@@ -552,8 +528,7 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   if (any || seed) {
     const float dt = B[lane], db = B[(TILE - 1) * W_STRIDE + lane];               // column layout
     const float dl = B[lane * W_STRIDE], dr = B[lane * W_STRIDE + TILE - 1];      // row layout
-    const float wt = vb.Wv[lane], wb = vb.Wv[TILE * W_STRIDE + lane];
-    const float wl = vb.Wh[lane * W_STRIDE], wr = vb.Wh[lane * W_STRIDE + TILE];
+    const float wt = E[E_TOP + lane], wb = E[E_BOTTOM + lane], wl = E[E_LEFT + lane], wr = E[E_RIGHT + lane];
     // The activation value of a side: the smallest border value it can bring (its priority in the queue).
     const float vl = __fadd_rn(dl, wl), vr = __fadd_rn(dr, wr), vt = __fadd_rn(dt, wt), vb = __fadd_rn(db, wb);
     const uint32_t kl = __reduce_min_sync(~0u, vl < lft ? __float_as_uint(vl) : KEY_NONE);
