@@ -22,6 +22,7 @@
 
 #include "dtb.h"
 #include "dtb_internal.h"
+#include "dtb_block.cuh"
 #include "dtb_kernels.cuh"
 
 using namespace dtb;
@@ -47,16 +48,7 @@ __global__ void __launch_bounds__(128) ggdt_scan(const ImgDesc* __restrict__ des
     const int x0 = tx * TILE, y0 = ty * TILE;
     const int vw = min(TILE, dd.width - x0), vh = min(TILE, dd.height - y0);
     bool nz = false;
-    if (lane < vh) {
-      const uint8_t* row = dd.mask + (int64_t)(y0 + lane) * dd.mask_pitch + x0;
-      if (vw == TILE && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
-        const uint4 a = reinterpret_cast<const uint4*>(row)[0];
-        const uint4 b = reinterpret_cast<const uint4*>(row)[1];
-        nz = (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) != 0u;
-      } else {
-        for (int c = 0; c < vw; ++c) nz |= row[c] != 0;
-      }
-    }
+    if (lane < vh) nz = mask_row_any(dd, x0, y0 + lane, vw);
     nz = __any_sync(~0u, nz);
     if (lane == 0) {
       uint32_t st = (img << ST_IMG_SHIFT) | (warm ? ST_VISITED : 0u);
@@ -349,6 +341,7 @@ ScratchLayout layout_for(int n, uint32_t total, uint32_t workers, bool rounds, u
   L.nb = std::max<uint32_t>(1u, std::min<uint32_t>(next_pow2(std::max<uint32_t>(buckets, 1u)), NBUCKET_MAX));
   size_t off = 0;
   L.o_hdr = off;    off = align_up(off + sizeof(QueueHdr), 256);
+  L.o_msg = off;    off = align_up(off + 32ull * std::min<uint32_t>(total, BLOCK_RUN_MAX), 256);  // right after the header
   L.o_states = off; off = align_up(off + 4ull * std::max<uint32_t>(total, 1), 256);
   L.o_ring = off;   off = align_up(off + L.ring_bytes(), 256);
   L.o_keys = off;   off = align_up(off + (L.nb > 1 ? 4ull * std::max<uint32_t>(total, 1) : 0), 256);
@@ -356,13 +349,15 @@ ScratchLayout layout_for(int n, uint32_t total, uint32_t workers, bool rounds, u
   L.o_desc = off;   off = align_up(off + sizeof(ImgDesc) * (size_t)std::max(n, 1), 256);
   L.o_tmap = off;   off = align_up(off + sizeof(CUtensorMap) * 2 * (size_t)std::max(n, 1), 256);
   L.o_base = off;   off = align_up(off + 4ull * (n + 1), 256);
+  L.o_bbase = off;  off = align_up(off + 4ull * (n + 1), 256);
   L.o_act = off;    off = align_up(off + (rounds ? 2ull * std::max<uint32_t>(total, 1) : 0), 256);
   L.o_chg = off;    off = align_up(off + 4, 256);
   L.bytes = off;
   return L;
 }
 
-dtb_status fill_desc(dtb_context ctx, const Job& j, uint32_t tile_base, int index, ImgDesc* d, CUtensorMap* tm) {
+dtb_status fill_desc(dtb_context ctx, const Job& j, uint32_t tile_base, uint32_t block_base, int index, ImgDesc* d,
+                     CUtensorMap* tm) {
   d->img = j.img;
   d->mask = j.mask;
   d->dist = j.dist;
@@ -381,6 +376,9 @@ dtb_status fill_desc(dtb_context ctx, const Job& j, uint32_t tile_base, int inde
   d->l_grad = j.l_grad;
   d->mode = j.mode;
   d->ref_fma = j.ref_fma;
+  d->blocks_x = j.blocks_x();
+  d->blocks_y = j.blocks_y();
+  d->block_base = block_base;
   if (j.width > 0 && j.height > 0) {
     const uint32_t bw = j.channels == 3 ? IMG_BOX_RGB : IMG_BOX_GRAY;
     if (!encode_u8_2d(ctx, &tm[0], j.img, (uint64_t)j.width * j.channels, (uint64_t)j.height, (uint64_t)j.img_pitch, bw,
@@ -398,14 +396,18 @@ dtb_status build_tables(dtb_context ctx, const std::vector<Job>& jobs, const Scr
   ImgDesc* hdesc = reinterpret_cast<ImgDesc*>(out.data());
   CUtensorMap* htm = reinterpret_cast<CUtensorMap*>(out.data() + (L.o_tmap - L.o_desc));
   uint32_t* hbase = reinterpret_cast<uint32_t*>(out.data() + (L.o_base - L.o_desc));
-  uint32_t base = 0;
+  uint32_t* hbbase = reinterpret_cast<uint32_t*>(out.data() + (L.o_bbase - L.o_desc));
+  uint32_t base = 0, bbase = 0;
   for (int i = 0; i < n; ++i) {
-    const dtb_status s = fill_desc(ctx, jobs[i], base, i, &hdesc[i], &htm[2 * i]);
+    const dtb_status s = fill_desc(ctx, jobs[i], base, bbase, i, &hdesc[i], &htm[2 * i]);
     if (s != DTB_OK) return s;
     hbase[i] = base;
     base += (uint32_t)(hdesc[i].tiles_x * hdesc[i].tiles_y);
+    hbbase[i] = bbase;
+    bbase += (uint32_t)(hdesc[i].blocks_x * hdesc[i].blocks_y);
   }
   hbase[n] = base;
+  hbbase[n] = bbase;
   return DTB_OK;
 }
 
@@ -466,8 +468,62 @@ dtb_status reset_queue(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, 
   return DTB_OK;
 }
 
+uint32_t count_blocks(const std::vector<Job>& jobs) {
+  uint64_t t = 0;
+  for (const Job& j : jobs) t += (uint64_t)j.blocks_x() * j.blocks_y();
+  return (uint32_t)t;
+}
+
+// Whether a run takes the block kernel: ns-mode under the default tuning, up to as many blocks as its CTAs may own
+// (9472 on 148 SMs, 38 Mpx).  Up to there chains of dependent visits bound the run and the block kernel is faster or as
+// fast (tile against block kernel: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze
+// 4.2 / 4.1, 6016^2 rgb8 1.19 / 1.18, 48 images of 7 Mpx 0.80 / 0.75); with more work than warps the tile kernel's finer
+// units win (128 images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5).
+bool use_blocks(dtb_context ctx, int mode, const LaunchTuning& t, uint32_t blocks) {
+  return mode == MODE_NS && !t.chosen && blocks > 0 &&
+         blocks <= std::min((uint32_t)(ctx->num_sms * BLOCK_CTAS * BLOCK_OWNED_MAX), BLOCK_RUN_MAX);
+}
+
+// A run of the block kernel: one memset (header, block states, keys) and one launch.
+static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, cudaStream_t stream, cudaEvent_t ev0,
+                                 cudaEvent_t ev1) {
+  const uint64_t stall_ns = ctx->inject_stall_ns;
+  ctx->inject_stall_ns = 0;
+  const ImgDesc* ddesc = reinterpret_cast<const ImgDesc*>(dbase + L.o_desc);
+  const CUtensorMap* dtm = reinterpret_cast<const CUtensorMap*>(dbase + L.o_tmap);
+  BlockRun a{};
+  a.hdr = reinterpret_cast<QueueHdr*>(dbase + L.o_hdr);
+  a.msg = reinterpret_cast<uint2*>(dbase + L.o_msg);
+  a.base = reinterpret_cast<const uint32_t*>(dbase + L.o_bbase);
+  a.n = L.n;
+  a.total = L.blocks;
+  a.max_visits = (uint32_t)std::min<uint64_t>(0xF0000000ull, 4096ull * L.total + (1ull << 20));
+  a.timeout_ns = stall_ns ? stall_ns : DEFAULT_TIMEOUT_NS;
+  DTB_CUDA(ctx, cudaMemsetAsync(dbase + L.o_hdr, 0, L.o_msg - L.o_hdr + 32ull * L.blocks, stream));
+  if (stall_ns) {
+    ggdt_phantom_pending<<<1, 1, 0, stream>>>(a.hdr);
+    DTB_CUDA(ctx, cudaGetLastError());
+  }
+  if (ev0) DTB_CUDA(ctx, cudaEventRecord(ev0, stream));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, (uint32_t)(ctx->num_sms * BLOCK_CTAS)));
+  cfg.blockDim = dim3(BLOCK_WARPS * 32);
+  cfg.dynamicSmemBytes = BLOCK_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;  // all CTAs resident: a CTA waits for blocks that the others activate
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[3] = {(void*)&ddesc, (void*)&dtm, (void*)&a};
+  DTB_CUDA(ctx, cudaLaunchKernelExC(&cfg, (const void*)ggdt_block, args));
+  if (ev1) DTB_CUDA(ctx, cudaEventRecord(ev1, stream));
+  return DTB_OK;
+}
+
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
                               cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, QueueHdr* fold) {
+  if (!fold && L.total && use_blocks(ctx, mode, t, L.blocks)) return enqueue_blocks(ctx, dbase, L, stream, ev0, ev1);
   const uint64_t stall_ns = ctx->inject_stall_ns;
   ctx->inject_stall_ns = 0;
   Queue q = make_queue(dbase, L, stall_ns ? stall_ns : DEFAULT_TIMEOUT_NS, &t);
@@ -673,8 +729,9 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
   LaunchTuning tuning = ctx->tuning;
   auto it = ctx->tuned.find(tuning_key(n, total));
   if (it != ctx->tuned.end()) tuning = it->second;
-  const ScratchLayout L = layout_for(n, total, resident_workers(ctx, mode, tuning), rounds,
-                                     rounds ? 1u : (uint32_t)tuning.buckets);
+  ScratchLayout L = layout_for(n, total, resident_workers(ctx, mode, tuning), rounds,
+                               rounds ? 1u : (uint32_t)tuning.buckets);
+  L.blocks = count_blocks(jobs);
   if ((s = grow(ctx, &ctx->dscratch, &ctx->dscratch_size, L.bytes)) != DTB_OK) return s;
   uint8_t* dbase = reinterpret_cast<uint8_t*>(ctx->dscratch);
   if ((s = build_tables(ctx, jobs, L, ctx->hstage)) != DTB_OK) return s;
@@ -829,6 +886,12 @@ DTB_API dtb_status dtb_context_create(int32_t device, dtb_context* out) {
                                                        ctx->ns_smem[k]) == cudaSuccess &&
          ctx->ns_blocks_per_sm[k] >= 1;
   }
+  int block_bps = 0;
+  ok = ok && cudaFuncSetAttribute((const void*)ggdt_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLOCK_SMEM) ==
+                 cudaSuccess &&
+       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&block_bps, (const void*)ggdt_block, BLOCK_WARPS * 32, BLOCK_SMEM) ==
+           cudaSuccess &&
+       block_bps >= BLOCK_CTAS;
   int ref_bps_nofma = 0;
   ok = ok && cudaFuncSetAttribute(kref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM) == cudaSuccess &&
        cudaFuncSetAttribute(kref_nofma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM) == cudaSuccess &&
@@ -851,7 +914,10 @@ DTB_API dtb_status dtb_context_create(int32_t device, dtb_context* out) {
   }
   if (const char* e = getenv("DTB_NS_VARIANT")) {  // index into NS_VARIANT_TABLE
     const int k = atoi(e);
-    if (k >= 0 && k < NS_VARIANTS) ctx->tuning.variant = k;
+    if (k >= 0 && k < NS_VARIANTS) {
+      ctx->tuning.variant = k;
+      ctx->tuning.chosen = true;
+    }
   }
   if (const char* e = getenv("DTB_AUTOTUNE_CACHE")) {  // autotuner cache of earlier processes
     ctx->tune_cache_path = e;
@@ -926,6 +992,7 @@ DTB_API dtb_status dtb_context_set_tuning(dtb_context ctx, const dtb_tuning* t) 
   nt.grid_percent = pct;
   nt.buckets = buckets;
   nt.bucket_tiles = width;
+  nt.chosen = true;
   ctx->tuning = nt;
   if (t->host_chunk_kpx > 0) ctx->host_chunk_px = (uint64_t)t->host_chunk_kpx * 1024ull;
   ctx->tuned.clear();

@@ -25,6 +25,13 @@ static_assert(GRAY_LUT_OFFSET >= IMG_BOX_ROWS * IMG_BOX_GRAY && GRAY_LUT_OFFSET 
               "gray weight table must fit the unused part of the image box");
 constexpr int S_STRIDE = TILE + 1;        // padded transpose buffer stride (floats): conflict-free both ways
 
+// Block kernel: tiles of a block (one warp each), its size in pixels, and CTAs per SM.  Two CTAs of four warps leave
+// 255 registers a thread, so a warp holds its tile and weights without spills; measured against 3 CTAs of 2x2, and one
+// of 4x2, 4x3 and 4x4 tiles, on 512^2 gray, 2048^2 gray and 4096^2 rgb8: 0.17 / 0.45 / 1.10 ms against 0.19 / 0.51 / 1.18,
+// 0.17 / 0.46 / 1.13, 0.20 / 0.53 / 1.14 and 0.25 / 0.69 / 1.34 ms.
+constexpr int BLOCK_TX = 2, BLOCK_TY = 2, BLOCK_CTAS = 2;
+constexpr int BLOCK_W = BLOCK_TX * TILE, BLOCK_H = BLOCK_TY * TILE;
+
 // Tile state word: flags in the low byte, image index of the tile in the upper 24 bits.
 constexpr uint32_t ST_PENDING = 1u;   // queued (or: re-run requested while running)
 constexpr uint32_t ST_RUNNING = 2u;   // a warp is visiting the tile
@@ -64,6 +71,8 @@ struct alignas(64) ImgDesc {
   float l_grad;   // ref-mode: lambda
   int32_t mode;
   int32_t ref_fma;  // ref-mode: 1 = fma(l_grad, dI, fma(l_eucl, d, D)), 0 = left-to-right rounding
+  int32_t blocks_x, blocks_y;  // block kernel: blocks of 4 x 4 tiles
+  uint32_t block_base;
 };
 
 // Counters live on separate 128-byte lines.
@@ -417,11 +426,26 @@ __device__ __forceinline__ uint32_t queue_try_pop(const Queue& q) {
 // ------------------------------------------------------------------------------------------------------
 // Edge weights
 // ------------------------------------------------------------------------------------------------------
+// Correctly rounded square root of x >= 1 (or infinite), without branches.  The hardware approximation s is within one
+// ulp, and Tuckerman's test picks the right neighbour: the rounded root r is the float with r * pred(r) < x <= r * succ(r),
+// whose two products a fused multiply-add compares with x exactly.  Equal to __fsqrt_rn for every float from 1 up
+// (checked exhaustively); __fsqrt_rn's special cases are a branch per root, which kept the roots of a tile from overlapping
+// (59 cycles a root in a row of independent ones, 21 here).
+__device__ __forceinline__ float sqrt_ge1(float x) {
+  float s;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(x));
+  const float lo = __uint_as_float(__float_as_uint(s) - 1u), hi = __uint_as_float(__float_as_uint(s) + 1u);
+  float r = s;
+  if (__fmaf_rn(s, lo, -x) >= 0.0f) r = lo;
+  if (__fmaf_rn(s, hi, -x) < 0.0f) r = hi;
+  return r;
+}
+
 // ns-mode: w = sqrt(1 + g2 * dI2), dI2 = sum_c (I_c(p) - I_c(q))^2.  Pixels are packed little-endian in a
 // u32 (gray: byte 0; rgb8: bytes 0..2), unused bytes zero.  dI2 <= 3 * 255^2 is exact in fp32; each of the
 // three float operations is rounded separately (no contraction), the square root correctly rounded.
 __device__ __forceinline__ float ns_weight_sq(uint32_t dI2, float g2) {
-  return __fsqrt_rn(__fadd_rn(1.0f, __fmul_rn(g2, __uint2float_rn(dI2))));
+  return sqrt_ge1(__fadd_rn(1.0f, __fmul_rn(g2, __uint2float_rn(dI2))));
 }
 __device__ __forceinline__ float ns_weight(uint32_t pa, uint32_t pb, float g2) {
   const uint32_t ad = __vabsdiffu4(pa, pb);

@@ -22,6 +22,7 @@ constexpr size_t PERSIST_SMEM = PERSIST_WPC * sizeof(WarpSmem) + 128;
 constexpr size_t PERSIST_SMEM_AHEAD = PERSIST_WPC * sizeof(WarpSmemP) + 128;
 constexpr size_t ROUND_SMEM = ROUND_WPC * sizeof(WarpSmem) + 128;
 constexpr uint64_t DEFAULT_TIMEOUT_NS = 2000000000ull;
+constexpr uint32_t BLOCK_RUN_MAX = 16384;  // blocks of a block kernel run at most (room for its messages)
 constexpr int REF_CTAS = 3;  // resident CTAs per SM of the ref-mode tile kernels (168 registers)
 // ns-mode tile kernel variants: CTAs per SM, whether a warp stages its next tile ahead (17 KB of shared memory a
 // warp instead of 13 KB, so at most 3 CTAs of 4 warps per SM), and warps per CTA.  Registers per thread follow
@@ -60,6 +61,8 @@ struct Job {
 
   int tiles_x() const { return (width + 31) / 32; }
   int tiles_y() const { return (height + 31) / 32; }
+  int blocks_x() const { return (width + BLOCK_W - 1) / BLOCK_W; }  // of the block kernel
+  int blocks_y() const { return (height + BLOCK_H - 1) / BLOCK_H; }
 
   static Job from(const dtb_image* img, const dtb_image* mask, const dtb_image* dist) {
     Job j;
@@ -87,9 +90,10 @@ inline float gamma_to_g2(float gamma) {
 struct ScratchLayout {
   int n = 0;
   uint32_t total = 0;  // tiles
+  uint32_t blocks = 0;  // blocks of the block kernel (0: the run does not use it)
   uint32_t cap = 0;    // ring slots per bucket (power of two)
   uint32_t nb = 1;     // priority-bucket rings allocated (a power of two <= NBUCKET_MAX; 1 = one FIFO ring)
-  size_t o_hdr = 0, o_states = 0, o_ring = 0, o_keys = 0, o_wacc = 0, o_desc = 0, o_tmap = 0, o_base = 0, o_act = 0,
+  size_t o_hdr = 0, o_msg = 0, o_states = 0, o_ring = 0, o_keys = 0, o_wacc = 0, o_desc = 0, o_tmap = 0, o_base = 0, o_bbase = 0, o_act = 0,
          o_chg = 0, bytes = 0;
   size_t ring_bytes() const { return 4ull * cap * nb; }
 };
@@ -104,6 +108,7 @@ struct LaunchTuning {
   int grid_percent = 100; // share of the co-resident CTAs that is launched
   int buckets = DEFAULT_BUCKETS;              // 1 = FIFO, else 2 / 4 / 8 / 16 distance-ordered buckets
   float bucket_tiles = DEFAULT_BUCKET_TILES;  // bucket width in tile-widths of path cost
+  bool chosen = false;    // set by the caller or the autotuner: the tile kernel runs as given, whatever the size
 };
 
 }  // namespace dtb
@@ -201,14 +206,19 @@ ScratchLayout layout_for(int n, uint32_t total, uint32_t workers, bool rounds, u
 dtb_status reset_queue(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, cudaStream_t stream);
 // Host image of [descriptors | tensor maps | tile prefix] (bytes o_desc .. o_act of the layout).
 dtb_status build_tables(dtb_context ctx, const std::vector<Job>& jobs, const ScratchLayout& L, std::vector<uint8_t>& out);
-// Descriptor and tensor maps (image box, mask tile) of one image whose tile ids start at tile_base; `index`
+// Descriptor and tensor maps (image box, mask tile) of one image whose tile and block ids start at the given bases; `index`
 // names the image in error messages.
-dtb_status fill_desc(dtb_context ctx, const Job& j, uint32_t tile_base, int index, ImgDesc* d, CUtensorMap* tm);
+dtb_status fill_desc(dtb_context ctx, const Job& j, uint32_t tile_base, uint32_t block_base, int index, ImgDesc* d,
+                     CUtensorMap* tm);
+// Blocks of the jobs for the block kernel, and whether a run of that many takes it.
+uint32_t count_blocks(const std::vector<Job>& jobs);
+bool use_blocks(dtb_context ctx, int mode, const LaunchTuning& t, uint32_t blocks);
 // Total tiles of the jobs (error if beyond the 31-bit tile id space).
 dtb_status count_tiles(dtb_context ctx, const std::vector<Job>& jobs, uint32_t* total);
 // Resident warps of the tile kernel of `mode` under `t`.
 uint32_t resident_workers(dtb_context ctx, int mode, const LaunchTuning& t);
-// Enqueues queue reset, seed scan, the persistent tile kernel and finalize on `stream` (capturable).
+// Enqueues queue reset, seed scan, the persistent tile kernel and finalize on `stream` (capturable); or the block
+// kernel, where use_blocks says so and there is nothing to fold.
 // ev0 / ev1 (optional) are recorded around the tile kernel; `fold` (optional) receives the run's status and
 // counters, added by finalize.
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,

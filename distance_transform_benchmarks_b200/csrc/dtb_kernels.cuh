@@ -174,6 +174,19 @@ __device__ __forceinline__ float ld_dist_at(const uint8_t* base, int64_t pitch, 
   return __ldcg(reinterpret_cast<const float*>(base + (int64_t)y * pitch));
 }
 
+// Whether the seed mask holds a nonzero byte in columns x0 .. x0 + vw - 1 of row y (x0 a multiple of 32, vw <= 32).
+__device__ __forceinline__ bool mask_row_any(const ImgDesc& dd, int x0, int y, int vw) {
+  const uint8_t* row = dd.mask + (int64_t)y * dd.mask_pitch + x0;
+  if (vw == TILE && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
+    const uint4 a = reinterpret_cast<const uint4*>(row)[0];
+    const uint4 b = reinterpret_cast<const uint4*>(row)[1];
+    return (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) != 0u;
+  }
+  bool nz = false;
+  for (int c = 0; c < vw; ++c) nz |= row[c] != 0;
+  return nz;
+}
+
 // Waits for the TMA transactions on `bar`; its phase parity is bit `pmask` of `pbits`.  Bounded: after
 // TMA_TIMEOUT_NS the error word is set and the wait goes on for as long again, to give a slow copy the chance
 // to land before the warp leaves; after that the wait gives up, and a copy may then still be pending.  The
@@ -266,6 +279,84 @@ __device__ __forceinline__ uint32_t box_pix(const uint8_t* box, bool rgb, int r,
   return __funnelshift_r(wp[0], wp[1], (off & 3) * 8) & 0xFFFFFFu;
 }
 
+// Edge weights of a tile from its staged image box into Wh / Wv / E (lane = x; the left and right halo edges
+// lane = y).  Returns this lane's sum of the tile's internal column edges (x < vw, 0 < y < vh).
+__device__ __forceinline__ float tile_weights(float g2, bool rgb, int vw, int vh, uint8_t* box, float* Wh, float* Wv, float* E) {
+  const int lane = threadIdx.x & 31;
+  const float INF = f_inf();
+  float wsum = 0.0f;
+  float et, eb, el, er;
+  if (!rgb) {
+    // Gray: the weight depends on |dI| in [0, 255] only.  A 256-entry table of the same expression (so the
+    // same bits) costs 8 square roots per lane instead of 65; it sits in the part of the image box that the
+    // 64-byte gray rows leave unused.
+    float* lut = reinterpret_cast<float*>(box + GRAY_LUT_OFFSET);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t a = (uint32_t)(lane + 32 * k);
+      lut[a] = ns_weight_sq(a * a, g2);
+    }
+    __syncwarp();
+    const uint8_t* col = box + 16 + lane;  // column `lane` of the box, row r at col[r * IMG_BOX_GRAY]
+    int pprev = col[IMG_BOX_GRAY];
+    et = lut[abs(pprev - (int)col[0])];
+    Wv[lane] = INF;
+    Wh[lane] = lane == 0 ? INF : lut[abs(pprev - (int)col[IMG_BOX_GRAY - 1])];
+#pragma unroll 2
+    for (int y = 1; y < TILE; ++y) {
+      const int pcur = col[(y + 1) * IMG_BOX_GRAY];
+      const float w = lut[abs(pcur - pprev)];
+      const float wx = lut[abs(pcur - (int)col[(y + 1) * IMG_BOX_GRAY - 1])];
+      Wv[y * W_STRIDE + lane] = w;
+      Wh[y * W_STRIDE + lane] = lane == 0 ? INF : wx;
+      if (lane < vw && y < vh) wsum += w;
+      pprev = pcur;
+    }
+    eb = lut[abs((int)col[(TILE + 1) * IMG_BOX_GRAY] - pprev)];
+    const uint8_t* row = box + (lane + 1) * IMG_BOX_GRAY + 16;
+    el = lut[abs((int)row[0] - (int)row[-1])];
+    er = lut[abs((int)row[TILE] - (int)row[TILE - 1])];
+  } else {
+    uint32_t pprev = box_pix(box, true, 1, lane);
+    et = ns_weight(box_pix(box, true, 0, lane), pprev, g2);
+    Wv[lane] = INF;
+    {
+      const float wx = ns_weight(__shfl_up_sync(~0u, pprev, 1), pprev, g2);
+      Wh[lane] = lane == 0 ? INF : wx;
+    }
+#pragma unroll 2
+    for (int y = 1; y < TILE; ++y) {
+      const uint32_t pcur = box_pix(box, true, y + 1, lane);
+      const float w = ns_weight(pprev, pcur, g2);
+      const float wx = ns_weight(__shfl_up_sync(~0u, pcur, 1), pcur, g2);
+      Wv[y * W_STRIDE + lane] = w;
+      Wh[y * W_STRIDE + lane] = lane == 0 ? INF : wx;
+      if (lane < vw && y < vh) wsum += w;
+      pprev = pcur;
+    }
+    eb = ns_weight(pprev, box_pix(box, true, TILE + 1, lane), g2);
+    el = ns_weight(box_pix(box, true, lane + 1, -1), box_pix(box, true, lane + 1, 0), g2);
+    er = ns_weight(box_pix(box, true, lane + 1, TILE - 1), box_pix(box, true, lane + 1, TILE), g2);
+  }
+  if (vw < TILE || vh < TILE) {  // edges touching a pixel outside the image are INF
+#pragma unroll 1
+    for (int y = 0; y < TILE; ++y)
+      if (lane >= vw || y >= vh) {
+        Wh[y * W_STRIDE + lane] = INF;
+        Wv[y * W_STRIDE + lane] = INF;
+      }
+    if (lane >= vw) et = INF;
+    if (lane >= vw || vh < TILE) eb = INF;
+    if (lane >= vh) el = INF;
+    if (lane >= vh || vw < TILE) er = INF;
+  }
+  E[E_LEFT + lane] = el;
+  E[E_RIGHT + lane] = er;
+  E[E_TOP + lane] = et;
+  E[E_BOTTOM + lane] = eb;
+  return wsum;
+}
+
 // ------------------------------------------------------------------------------------------------------
 // ns-mode visit (C4, w = sqrt(1 + g2 * dI2)), gray or rgb8.
 //
@@ -338,13 +429,9 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     if (nexist & 2u) rgt = (nvis & 2u) ? ld_dist(dd, y0 + lane, x0 + TILE) : v;
   }
 
-  // Tile distances in column layout.
+  // Tile distances (lane = x).
   float d[TILE];
-  if (rerun) {
-    const float* pb = reinterpret_cast<const float*>(vb.box) + lane;  // B[y * 36 + x]
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = pb[y * W_STRIDE];
-  } else if (!first) {
+  if (!rerun && !first) {
     const uint8_t* lb = dist_base(dd, y0, x0 + lane, 0u);
 #pragma unroll
     for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
@@ -352,18 +439,13 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
 
   if (!rerun && !tma_wait(vb.bar, *vb.pbits, vb.pmask, sch.q, tile)) return;
   if (PRESTAGED && seed && !tma_wait(vb.mbar, *vb.pbits, vb.mmask, sch.q, tile)) return;
-  const uint8_t* mbox = reinterpret_cast<const uint8_t*>(vb.Wv);
 
   // Seeds first: the mask box shares memory with Wv.
-  if (first) {
-    const bool in = lane < vw;
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = in && y < vh ? v : INF;
-  }
+  uint32_t seeds = 0;  // this lane's column of the mask tile
   if (seed) {
-#pragma unroll
-    for (int y = 0; y < TILE; ++y)
-      if (lane < vw && y < vh && mbox[y * TILE + lane] != 0) d[y] = 0.0f;
+    const uint8_t* mbox = reinterpret_cast<const uint8_t*>(vb.Wv);
+#pragma unroll 4
+    for (int y = 0; y < TILE; ++y) seeds |= (lane < vw && y < vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
   }
   __syncwarp();
 
@@ -371,77 +453,7 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   const uint32_t img_idx = old_state >> ST_IMG_SHIFT;
   float wsum = 0.0f;
   if (!rerun) {
-    const float g2 = dd.g2;
-    const uint8_t* box = vb.box;
-    float et, eb, el, er;
-    if (!rgb) {
-      // Gray: the weight depends on |dI| in [0, 255] only.  A 256-entry table of the same expression (so the
-      // same bits) costs 8 square roots per lane instead of 65; it sits in the part of the image box that the
-      // 64-byte gray rows leave unused.
-      float* lut = reinterpret_cast<float*>(vb.box + GRAY_LUT_OFFSET);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t a = (uint32_t)(lane + 32 * k);
-        lut[a] = ns_weight_sq(a * a, g2);
-      }
-      __syncwarp();
-      const uint8_t* col = box + 16 + lane;  // column `lane` of the box, row r at col[r * IMG_BOX_GRAY]
-      int pprev = col[IMG_BOX_GRAY];
-      et = lut[abs(pprev - (int)col[0])];
-      vb.Wv[lane] = INF;
-      vb.Wh[lane] = lane == 0 ? INF : lut[abs(pprev - (int)col[IMG_BOX_GRAY - 1])];
-#pragma unroll 2
-      for (int y = 1; y < TILE; ++y) {
-        const int pcur = col[(y + 1) * IMG_BOX_GRAY];
-        const float w = lut[abs(pcur - pprev)];
-        const float wx = lut[abs(pcur - (int)col[(y + 1) * IMG_BOX_GRAY - 1])];
-        vb.Wv[y * W_STRIDE + lane] = w;
-        vb.Wh[y * W_STRIDE + lane] = lane == 0 ? INF : wx;
-        if (lane < vw && y < vh) wsum += w;
-        pprev = pcur;
-      }
-      eb = lut[abs((int)col[(TILE + 1) * IMG_BOX_GRAY] - pprev)];
-      const uint8_t* row = box + (lane + 1) * IMG_BOX_GRAY + 16;
-      el = lut[abs((int)row[0] - (int)row[-1])];
-      er = lut[abs((int)row[TILE] - (int)row[TILE - 1])];
-    } else {
-      uint32_t pprev = box_pix(box, true, 1, lane);
-      et = ns_weight(box_pix(box, true, 0, lane), pprev, g2);
-      vb.Wv[lane] = INF;
-      {
-        const float wx = ns_weight(__shfl_up_sync(~0u, pprev, 1), pprev, g2);
-        vb.Wh[lane] = lane == 0 ? INF : wx;
-      }
-#pragma unroll 2
-      for (int y = 1; y < TILE; ++y) {
-        const uint32_t pcur = box_pix(box, true, y + 1, lane);
-        const float w = ns_weight(pprev, pcur, g2);
-        const float wx = ns_weight(__shfl_up_sync(~0u, pcur, 1), pcur, g2);
-        vb.Wv[y * W_STRIDE + lane] = w;
-        vb.Wh[y * W_STRIDE + lane] = lane == 0 ? INF : wx;
-        if (lane < vw && y < vh) wsum += w;
-        pprev = pcur;
-      }
-      eb = ns_weight(pprev, box_pix(box, true, TILE + 1, lane), g2);
-      el = ns_weight(box_pix(box, true, lane + 1, -1), box_pix(box, true, lane + 1, 0), g2);
-      er = ns_weight(box_pix(box, true, lane + 1, TILE - 1), box_pix(box, true, lane + 1, TILE), g2);
-    }
-    if (vw < TILE || vh < TILE) {  // edges touching a pixel outside the image are INF
-#pragma unroll 1
-      for (int y = 0; y < TILE; ++y)
-        if (lane >= vw || y >= vh) {
-          vb.Wh[y * W_STRIDE + lane] = INF;
-          vb.Wv[y * W_STRIDE + lane] = INF;
-        }
-      if (lane >= vw) et = INF;
-      if (lane >= vw || vh < TILE) eb = INF;
-      if (lane >= vh) el = INF;
-      if (lane >= vh || vw < TILE) er = INF;
-    }
-    vb.E[E_LEFT + lane] = el;
-    vb.E[E_RIGHT + lane] = er;
-    vb.E[E_TOP + lane] = et;
-    vb.E[E_BOTTOM + lane] = eb;
+    wsum = tile_weights(dd.g2, rgb, vw, vh, vb.box, vb.Wh, vb.Wv, vb.E);
   }
   __syncwarp();
 
@@ -469,8 +481,13 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   const float* E = vb.E;
   if (!rerun) {
     float* pb = B + lane;
+    if (first) {
+#pragma unroll 4
+      for (int y = 0; y < TILE; ++y) pb[y * W_STRIDE] = (lane < vw && y < vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
+    } else {
 #pragma unroll
-    for (int k = 0; k < TILE; ++k) pb[k * W_STRIDE] = d[k];
+      for (int y = 0; y < TILE; ++y) pb[y * W_STRIDE] = ((seeds >> y) & 1u) ? 0.0f : d[y];
+    }
     __syncwarp();
   }
   bool any, layout_a;

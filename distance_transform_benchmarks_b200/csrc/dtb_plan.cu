@@ -66,6 +66,7 @@ struct CacheEntry {
   std::string gpu;
   uint64_t images = 0, tiles = 0;
   int ctas = 0, staging = 0, grid = 0, buckets = 0, width_pct = 0, wpc = 4;  // wpc: 4 in caches written without it
+  int blocks = 0;  // the block kernel where the size allows it; 0 in caches written without it
   double ms = 0.0;
 };
 
@@ -110,6 +111,7 @@ std::vector<CacheEntry> parse_cache(const std::string& text) {
       else if (key == "grid_percent") c.grid = std::atoi(val.c_str());
       else if (key == "queue_buckets") c.buckets = std::atoi(val.c_str());
       else if (key == "bucket_width_pct") c.width_pct = std::atoi(val.c_str());
+      else if (key == "blocks") c.blocks = std::atoi(val.c_str());
       else if (key == "ms") c.ms = std::atof(val.c_str());
     }
     out.push_back(c);
@@ -148,6 +150,7 @@ dtb_status load_tuning_cache(dtb_context ctx) {
     t.grid_percent = c.grid;
     t.buckets = c.buckets;
     t.bucket_tiles = (float)c.width_pct / 100.0f;
+    t.chosen = c.blocks == 0;
     ctx->tuned[key_of(c)] = t;
   }
   return DTB_OK;
@@ -169,6 +172,7 @@ dtb_status save_tuning_cache(dtb_context ctx, uint64_t key, const LaunchTuning& 
   n.grid = t.grid_percent;
   n.buckets = t.buckets;
   n.width_pct = (int)lrintf(t.bucket_tiles * 100.0f);
+  n.blocks = t.chosen ? 0 : 1;
   n.ms = ms;
   bool replaced = false;
   for (CacheEntry& c : entries)
@@ -185,9 +189,9 @@ dtb_status save_tuning_cache(dtb_context ctx, uint64_t key, const LaunchTuning& 
     const CacheEntry& c = entries[i];
     std::fprintf(f,
                  "%s\n  {\"gpu\": \"%s\", \"images_pow2\": %llu, \"tiles_pow2\": %llu, \"ctas_per_sm\": %d, \"staging\": %d, "
-                 "\"warps_per_cta\": %d, \"grid_percent\": %d, \"queue_buckets\": %d, \"bucket_width_pct\": %d, \"ms\": %.4f}",
+                 "\"warps_per_cta\": %d, \"blocks\": %d, \"grid_percent\": %d, \"queue_buckets\": %d, \"bucket_width_pct\": %d, \"ms\": %.4f}",
                  i ? "," : "", c.gpu.c_str(), (unsigned long long)c.images, (unsigned long long)c.tiles, c.ctas, c.staging,
-                 c.wpc, c.grid, c.buckets, c.width_pct, c.ms);
+                 c.wpc, c.blocks, c.grid, c.buckets, c.width_pct, c.ms);
   }
   std::fprintf(f, "\n]}\n");
   const bool ok = std::fclose(f) == 0 && std::rename(tmp.c_str(), ctx->tune_cache_path.c_str()) == 0;
@@ -238,6 +242,7 @@ DTB_API dtb_status dtb_plan_create(dtb_context ctx, int32_t n, const dtb_image* 
   uint32_t workers = 0;
   for (int k = 0; k < NS_VARIANTS; ++k) workers = std::max(workers, resident_workers(ctx, MODE_NS, LaunchTuning{k, 100}));
   p->L = layout_for(n, total, workers, false, NBUCKET_MAX);  // room for every queue policy of the autotuner
+  p->L.blocks = count_blocks(p->jobs);
   p->key = tuning_key(n, total);
   auto it = ctx->tuned.find(p->key);
   p->tuning = it != ctx->tuned.end() ? it->second : ctx->tuning;
@@ -316,11 +321,13 @@ DTB_API dtb_status dtb_plan_autotune(dtb_plan p, void* stream, int32_t reps, dtb
   // (3) the variants again under the best policy.
   static const int kPercent[3] = {100, 75, 50};
   const LaunchTuning start = p->tuning;
+  if (use_blocks(ctx, MODE_NS, start, p->L.blocks)) trial(start);  // the block kernel
   for (int v = 0; v < NS_VARIANTS; ++v)
     for (int pc = 0; pc < 3; ++pc) {
       LaunchTuning t = start;
       t.variant = v;
       t.grid_percent = kPercent[pc];
+      t.chosen = true;
       trial(t);
     }
   {

@@ -1070,7 +1070,7 @@ dtb_status live_publish(dtb_server s, LiveFlight& f, const Resident& r) {
     ImgDesc* d = reinterpret_cast<ImgDesc*>(stg + LST_DESC);
     CUtensorMap* tm = reinterpret_cast<CUtensorMap*>(stg + LST_TMAP);
     std::memset(stg, 0, LST_ENTRY);
-    dtb_status ds = fill_desc(ctx, j, r.tile_base, 0, d, tm);
+    dtb_status ds = fill_desc(ctx, j, r.tile_base, 0, 0, d, tm);
     if (ds != DTB_OK) return ds;
     DTB_CUDA(ctx, cudaMemcpyAsync(L->descs + r.slot, d, sizeof(ImgDesc), cudaMemcpyHostToDevice, st));
     DTB_CUDA(ctx, cudaMemcpyAsync(L->tmaps + 2 * r.slot, tm, 2 * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st));

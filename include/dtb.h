@@ -107,7 +107,9 @@ DTB_API dtb_status dtb_sync(dtb_context ctx, void* stream);
  * by the distance an activation can bring (default 8); bucket_width_pct: width of one bucket in percent of
  * one tile-width of path cost of the image (32 x its mean edge weight), 1..6400 (default 50);
  * staging: 1 = a visit stages its own tile, 2 = a warp stages the image box of its next tile while it visits
- * the current one (double-buffered shared memory; ctas_per_sm 2 or 3 only). */
+ * the current one (double-buffered shared memory; ctas_per_sm 2 or 3 only).
+ * A context whose tuning was never set runs calls and plans of up to about 38 Mpx in another kernel (one CTA per 64 x 64
+ * block); setting any field selects the tile kernel for every size. */
 typedef struct dtb_tuning {
   int32_t ctas_per_sm;
   int32_t grid_percent;
@@ -161,7 +163,9 @@ DTB_API dtb_status dtb_gdt_batch(dtb_context ctx, int32_t n, const dtb_image* im
  * distance-ordered buckets of 1/4, 1/2 or 1 tile-width of path cost): variants x grid shares first, then the
  * queue policies under the best launch, then the variants again under the best policy.  It keeps the fastest
  * in the plan and, for batches of the same size class (image count and tile count, each rounded up to a power
- * of two), in the context and in its autotuner cache file if one is set; and reports it.  dtb_plan_get_tuning
+ * of two), in the context and in its autotuner cache file if one is set; and reports it.  Where the size allows the
+ * kernel of one CTA per 64 x 64 block (see dtb_tuning), that one competes too and the report names the tile kernel's
+ * unchanged tuning when it wins.  dtb_plan_get_tuning
  * reports the plan's current tuning.  No reference counterpart: the reference fixes these choices
  * (dt/src/task_queue.cuh:23, dt/src/generalised_distance_transform_task.cu:184). */
 typedef struct dtb_plan_s* dtb_plan;
