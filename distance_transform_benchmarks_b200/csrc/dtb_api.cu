@@ -68,7 +68,7 @@ template <int MODE, int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB)
     ggdt_persistent(const ImgDesc* __restrict__ descs, const CUtensorMap* __restrict__ tmaps, uint32_t* states, Queue q) {
   extern __shared__ uint8_t smem_raw[];
-  WarpSmem& sm = warp_slot(smem_raw);
+  TileSmem<MODE>& sm = warp_slot<TileSmem<MODE>>(smem_raw);
   warp_slot_init(sm);
   uint32_t parity = 0;
   const int lane = threadIdx.x & 31;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(WPC * 32)
     ggdt_round(const ImgDesc* __restrict__ descs, const CUtensorMap* __restrict__ tmaps, uint32_t* states,
                const uint8_t* __restrict__ active, uint8_t* next_active, uint32_t* changed, uint32_t total, Queue q) {
   extern __shared__ uint8_t smem_raw[];
-  WarpSmem& sm = warp_slot(smem_raw);
+  TileSmem<MODE>& sm = warp_slot<TileSmem<MODE>>(smem_raw);
   const uint32_t t = blockIdx.x * WPC + (threadIdx.x >> 5);
   if (t >= total || !active[t]) return;
   warp_slot_init(sm);
@@ -341,7 +341,7 @@ ScratchLayout layout_for(int n, uint32_t total, uint32_t workers, bool rounds, u
   L.nb = std::max<uint32_t>(1u, std::min<uint32_t>(next_pow2(std::max<uint32_t>(buckets, 1u)), NBUCKET_MAX));
   size_t off = 0;
   L.o_hdr = off;    off = align_up(off + sizeof(QueueHdr), 256);
-  L.o_msg = off;    off = align_up(off + 32ull * std::min<uint32_t>(total, BLOCK_RUN_MAX), 256);  // right after the header
+  L.o_msg = off;    off = align_up(off + 64ull * std::min<uint32_t>(total, BLOCK_RUN_MAX), 256);  // right after the header
   L.o_states = off; off = align_up(off + 4ull * std::max<uint32_t>(total, 1), 256);
   L.o_ring = off;   off = align_up(off + L.ring_bytes(), 256);
   L.o_keys = off;   off = align_up(off + (L.nb > 1 ? 4ull * std::max<uint32_t>(total, 1) : 0), 256);
@@ -474,18 +474,19 @@ uint32_t count_blocks(const std::vector<Job>& jobs) {
   return (uint32_t)t;
 }
 
-// Whether a run takes the block kernel: ns-mode under the default tuning, up to as many blocks as its CTAs may own
-// (9472 on 148 SMs, 38 Mpx).  Up to there chains of dependent visits bound the run and the block kernel is faster or as
-// fast (tile against block kernel: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze
-// 4.2 / 4.1, 6016^2 rgb8 1.19 / 1.18, 48 images of 7 Mpx 0.80 / 0.75); with more work than warps the tile kernel's finer
-// units win (128 images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5).
+// Whether a run takes the block kernel: under the default tuning, up to as many blocks as its CTAs may own (9472 on 148
+// SMs, 38 Mpx).  Up to there chains of dependent visits bound the run.  ns-mode: the block kernel is faster or as fast
+// (tile against block kernel: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze 4.2 / 4.1,
+// 6016^2 rgb8 1.19 / 1.18, 48 images of 7 Mpx 0.80 / 0.75); with more work than warps the tile kernel's finer units win (128
+// images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5).  ref-mode, lambda 0 / 0.5 / 1: 1023x777 0.40 / 0.69 / 0.91 ms
+// against 0.23 / 0.56 / 0.80, 3648x2432 1.21 / 2.02 / 1.74 against 0.98 / 2.30 / 1.67, 6000^2 2.8 / 4.7 / 3.2 against 2.3 / 5.9 / 2.5.
 bool use_blocks(dtb_context ctx, int mode, const LaunchTuning& t, uint32_t blocks) {
-  return mode == MODE_NS && !t.chosen && blocks > 0 &&
+  return !t.chosen && blocks > 0 &&
          blocks <= std::min((uint32_t)(ctx->num_sms * BLOCK_CTAS * BLOCK_OWNED_MAX), BLOCK_RUN_MAX);
 }
 
 // A run of the block kernel: one memset (header, block states, keys) and one launch.
-static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, cudaStream_t stream, cudaEvent_t ev0,
+static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, cudaStream_t stream, cudaEvent_t ev0,
                                  cudaEvent_t ev1) {
   const uint64_t stall_ns = ctx->inject_stall_ns;
   ctx->inject_stall_ns = 0;
@@ -499,7 +500,7 @@ static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchL
   a.total = L.blocks;
   a.max_visits = (uint32_t)std::min<uint64_t>(0xF0000000ull, 4096ull * L.total + (1ull << 20));
   a.timeout_ns = stall_ns ? stall_ns : DEFAULT_TIMEOUT_NS;
-  DTB_CUDA(ctx, cudaMemsetAsync(dbase + L.o_hdr, 0, L.o_msg - L.o_hdr + 32ull * L.blocks, stream));
+  DTB_CUDA(ctx, cudaMemsetAsync(dbase + L.o_hdr, 0, L.o_msg - L.o_hdr + (mode == MODE_NS ? 32ull : 64ull) * L.blocks, stream));
   if (stall_ns) {
     ggdt_phantom_pending<<<1, 1, 0, stream>>>(a.hdr);
     DTB_CUDA(ctx, cudaGetLastError());
@@ -508,22 +509,25 @@ static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchL
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, (uint32_t)(ctx->num_sms * BLOCK_CTAS)));
   cfg.blockDim = dim3(BLOCK_WARPS * 32);
-  cfg.dynamicSmemBytes = BLOCK_SMEM;
+  cfg.dynamicSmemBytes = mode == MODE_NS ? BLOCK_SMEM<MODE_NS> : BLOCK_SMEM<MODE_REF>;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;  // all CTAs resident: a CTA waits for blocks that the others activate
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  const void* fn = mode == MODE_NS ? (const void*)ggdt_block<MODE_NS>
+                   : mode == MODE_REF ? (const void*)ggdt_block<MODE_REF>
+                                      : (const void*)ggdt_block<MODE_REF_NOFMA>;
   void* args[3] = {(void*)&ddesc, (void*)&dtm, (void*)&a};
-  DTB_CUDA(ctx, cudaLaunchKernelExC(&cfg, (const void*)ggdt_block, args));
+  DTB_CUDA(ctx, cudaLaunchKernelExC(&cfg, fn, args));
   if (ev1) DTB_CUDA(ctx, cudaEventRecord(ev1, stream));
   return DTB_OK;
 }
 
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
                               cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, QueueHdr* fold) {
-  if (!fold && L.total && use_blocks(ctx, mode, t, L.blocks)) return enqueue_blocks(ctx, dbase, L, stream, ev0, ev1);
+  if (!fold && L.total && use_blocks(ctx, mode, t, L.blocks)) return enqueue_blocks(ctx, dbase, L, mode, stream, ev0, ev1);
   const uint64_t stall_ns = ctx->inject_stall_ns;
   ctx->inject_stall_ns = 0;
   Queue q = make_queue(dbase, L, stall_ns ? stall_ns : DEFAULT_TIMEOUT_NS, &t);
@@ -558,7 +562,7 @@ dtb_status launch_tile_kernel(dtb_context ctx, int mode, const LaunchTuning& t, 
   const int wpc = mode == MODE_NS ? NS_VARIANT_TABLE[t.variant].wpc : PERSIST_WPC;
   cfg.gridDim = dim3(resident_workers(ctx, mode, t) / (uint32_t)wpc);
   cfg.blockDim = dim3((uint32_t)wpc * 32u);
-  cfg.dynamicSmemBytes = mode == MODE_NS ? ctx->ns_smem[t.variant] : PERSIST_SMEM;
+  cfg.dynamicSmemBytes = mode == MODE_NS ? ctx->ns_smem[t.variant] : REF_SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -613,9 +617,9 @@ static dtb_status run_rounds(dtb_context ctx, uint8_t* dbase, const ScratchLayou
     if (mode == MODE_NS)
       ggdt_round<MODE_NS, ROUND_WPC><<<blocks, ROUND_WPC * 32, ROUND_SMEM, stream>>>(ddesc, dtm, states, cur, nxt, changed, total, q);
     else if (mode == MODE_REF)
-      ggdt_round<MODE_REF, ROUND_WPC><<<blocks, ROUND_WPC * 32, ROUND_SMEM, stream>>>(ddesc, dtm, states, cur, nxt, changed, total, q);
+      ggdt_round<MODE_REF, ROUND_WPC><<<blocks, ROUND_WPC * 32, REF_SMEM, stream>>>(ddesc, dtm, states, cur, nxt, changed, total, q);
     else
-      ggdt_round<MODE_REF_NOFMA, ROUND_WPC><<<blocks, ROUND_WPC * 32, ROUND_SMEM, stream>>>(ddesc, dtm, states, cur, nxt, changed,
+      ggdt_round<MODE_REF_NOFMA, ROUND_WPC><<<blocks, ROUND_WPC * 32, REF_SMEM, stream>>>(ddesc, dtm, states, cur, nxt, changed,
                                                                                            total, q);
     DTB_CUDA(ctx, cudaGetLastError());
     uint32_t err_prog[2] = {0, 0};
@@ -886,18 +890,23 @@ DTB_API dtb_status dtb_context_create(int32_t device, dtb_context* out) {
                                                        ctx->ns_smem[k]) == cudaSuccess &&
          ctx->ns_blocks_per_sm[k] >= 1;
   }
-  int block_bps = 0;
-  ok = ok && cudaFuncSetAttribute((const void*)ggdt_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLOCK_SMEM) ==
-                 cudaSuccess &&
-       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&block_bps, (const void*)ggdt_block, BLOCK_WARPS * 32, BLOCK_SMEM) ==
-           cudaSuccess &&
-       block_bps >= BLOCK_CTAS;
+  const struct {
+    const void* fn;
+    size_t smem;
+  } block_fns[3] = {{(const void*)ggdt_block<MODE_NS>, BLOCK_SMEM<MODE_NS>},
+                    {(const void*)ggdt_block<MODE_REF>, BLOCK_SMEM<MODE_REF>},
+                    {(const void*)ggdt_block<MODE_REF_NOFMA>, BLOCK_SMEM<MODE_REF>}};
+  for (const auto& f : block_fns) {
+    int bps = 0;
+    ok = ok && cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, f.fn, BLOCK_WARPS * 32, f.smem) == cudaSuccess && bps >= BLOCK_CTAS;
+  }
   int ref_bps_nofma = 0;
-  ok = ok && cudaFuncSetAttribute(kref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM) == cudaSuccess &&
-       cudaFuncSetAttribute(kref_nofma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM) == cudaSuccess &&
-       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->ref_blocks_per_sm, kref, PERSIST_WPC * 32, PERSIST_SMEM) ==
+  ok = ok && cudaFuncSetAttribute(kref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REF_SMEM) == cudaSuccess &&
+       cudaFuncSetAttribute(kref_nofma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REF_SMEM) == cudaSuccess &&
+       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->ref_blocks_per_sm, kref, PERSIST_WPC * 32, REF_SMEM) ==
            cudaSuccess &&
-       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ref_bps_nofma, kref_nofma, PERSIST_WPC * 32, PERSIST_SMEM) ==
+       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ref_bps_nofma, kref_nofma, PERSIST_WPC * 32, REF_SMEM) ==
            cudaSuccess;
   ctx->ref_blocks_per_sm = std::min(ctx->ref_blocks_per_sm, ref_bps_nofma);  // one grid size for both roundings
   ok = ok && ctx->ref_blocks_per_sm >= 1;
@@ -905,9 +914,9 @@ DTB_API dtb_status dtb_context_create(int32_t device, dtb_context* out) {
        cudaFuncSetAttribute((const void*)ggdt_round<MODE_NS, ROUND_WPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)ROUND_SMEM) == cudaSuccess &&
        cudaFuncSetAttribute((const void*)ggdt_round<MODE_REF, ROUND_WPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)ROUND_SMEM) == cudaSuccess &&
+                            (int)REF_SMEM) == cudaSuccess &&
        cudaFuncSetAttribute((const void*)ggdt_round<MODE_REF_NOFMA, ROUND_WPC>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROUND_SMEM) == cudaSuccess;
+                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REF_SMEM) == cudaSuccess;
   if (!ok) {
     delete ctx;
     return DTB_ERR_NO_DEVICE;

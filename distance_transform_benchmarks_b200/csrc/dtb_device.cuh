@@ -23,7 +23,6 @@ constexpr int IMG_BOX_RGB = 128;          // rgb8 box width (bytes): 3*x0-16 .. 
 constexpr int GRAY_LUT_OFFSET = 2304;
 static_assert(GRAY_LUT_OFFSET >= IMG_BOX_ROWS * IMG_BOX_GRAY && GRAY_LUT_OFFSET + 1024 <= IMG_BOX_ROWS * IMG_BOX_RGB,
               "gray weight table must fit the unused part of the image box");
-constexpr int S_STRIDE = TILE + 1;        // padded transpose buffer stride (floats): conflict-free both ways
 
 // Block kernel: tiles of a block (one warp each), its size in pixels, and CTAs per SM.  Two CTAs of four warps leave
 // 255 registers a thread, so a warp holds its tile and weights without spills; measured against 3 CTAs of 2x2, and one
@@ -131,7 +130,24 @@ struct alignas(128) WarpSmem {
   uint64_t bar;                              // TMA mbarrier
   uint32_t keep;                             // tile this warp keeps for its next visit (POP_NONE: none)
 };
-__device__ __forceinline__ uint8_t* mask_box(WarpSmem& sm) { return reinterpret_cast<uint8_t*>(sm.Wv); }
+
+// Per-warp shared memory of a ref-mode visit (23.6 KB: 8 warps per SM).  The edge words (|dI|, or l_grad * |dI| without
+// FMA; INF where there is no edge inside the tile) and the tile keep 33 floats a row: conflict-free with a lane per
+// column and with a lane per row.
+constexpr int RS = TILE + 1;
+struct alignas(128) RefTile {
+  uint8_t img[TILE * RS * 4];   // TMA destination of the image box, then the tile T[y * 33 + x]
+  float V[TILE * RS];           // (x, y - 1) - (x, y); its first 1 KB receives the seed-mask TMA box before
+  float Hh[TILE * RS];          // (x - 1, y) - (x, y)
+  float DL[TILE * RS];          // (x - 1, y - 1) - (x, y)
+  float DR[(TILE + 1) * RS];    // (x + 1, y - 1) - (x, y)
+  float E[12 * TILE];           // edges to the halo: side (as E_LEFT..), offset -1, 0, 1 along it, position
+  float B0[4 * TILE];           // host-driven rounds: the border before the visit
+  float H[4 * TILE + 4];        // block kernel: halo on the block's border (INF elsewhere), sides, then corners
+  uint64_t bar;
+  uint32_t keep;
+};
+static_assert(sizeof(RefTile::img) >= IMG_BOX_ROWS * IMG_BOX_GRAY, "the gray image box must fit");
 
 // Per-warp shared memory of the staged-ahead tile kernel (18 KB: 12 warps per SM fit in 228 KB): the image
 // boxes of the tile being visited and of the warp's next tile, each the tile buffer B of its own visit once its
@@ -450,14 +466,6 @@ __device__ __forceinline__ float ns_weight_sq(uint32_t dI2, float g2) {
 __device__ __forceinline__ float ns_weight(uint32_t pa, uint32_t pb, float g2) {
   const uint32_t ad = __vabsdiffu4(pa, pb);
   return ns_weight_sq(__dp4a(ad, ad, 0u), g2);
-}
-
-// ref-mode relaxation of one edge, reference dt/src/dt_block_passes.cuh:45-46:
-//   D(q) + l_eucl * local_dist2d[k] + l_grad * |I(p) - I(q)|
-template <bool FMA>
-__device__ __forceinline__ float ref_relax(float dq, float eucl_d, float l_eucl, float l_grad, float absdi) {
-  if (FMA) return __fmaf_rn(l_grad, absdi, __fmaf_rn(l_eucl, eucl_d, dq));
-  return __fadd_rn(__fadd_rn(dq, __fmul_rn(l_eucl, eucl_d)), __fmul_rn(l_grad, absdi));
 }
 
 // ------------------------------------------------------------------------------------------------------

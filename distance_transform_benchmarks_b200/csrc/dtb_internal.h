@@ -21,9 +21,12 @@ constexpr int ROUND_WPC = 4;
 constexpr size_t PERSIST_SMEM = PERSIST_WPC * sizeof(WarpSmem) + 128;
 constexpr size_t PERSIST_SMEM_AHEAD = PERSIST_WPC * sizeof(WarpSmemP) + 128;
 constexpr size_t ROUND_SMEM = ROUND_WPC * sizeof(WarpSmem) + 128;
+static_assert(ROUND_WPC == PERSIST_WPC, "one size for the ref-mode kernels");
+constexpr size_t REF_SMEM = PERSIST_WPC * sizeof(RefTile) + 128;  // ref-mode kernels
 constexpr uint64_t DEFAULT_TIMEOUT_NS = 2000000000ull;
 constexpr uint32_t BLOCK_RUN_MAX = 16384;  // blocks of a block kernel run at most (room for its messages)
-constexpr int REF_CTAS = 3;  // resident CTAs per SM of the ref-mode tile kernels (168 registers)
+constexpr int REF_CTAS = 2;  // resident CTAs per SM of the ref-mode tile kernels (the tile and its edges take 128
+                             // registers a thread; 94 KB of shared memory a CTA)
 // ns-mode tile kernel variants: CTAs per SM, whether a warp stages its next tile ahead (17 KB of shared memory a
 // warp instead of 13 KB, so at most 3 CTAs of 4 warps per SM), and warps per CTA.  Registers per thread follow
 // the warps per SM: 8 -> 255, 12 -> 168, 16 -> 128.  The 12- and 16-warp shapes come in several CTA sizes

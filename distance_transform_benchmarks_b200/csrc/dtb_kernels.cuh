@@ -13,6 +13,8 @@
 //   ggdt_finalize    writes v into tiles that were never reached (their memory was never initialised).
 #pragma once
 
+#include <type_traits>
+
 #include "dtb_device.cuh"
 
 namespace dtb {
@@ -29,6 +31,7 @@ struct WarpStats {
 };
 
 struct QueueSched {
+  static constexpr bool any_change = false;  // ref-mode: activate the neighbours that the border can lower
   Queue q;
   uint32_t* states;
   // Optional: the warp's word for a tile it keeps.  Of the tiles a visit queues, one in the lowest bucket
@@ -112,6 +115,7 @@ struct QueueSched {
 };
 
 struct RoundSched {
+  static constexpr bool any_change = true;  // ref-mode: activate the neighbours whose facing border changed
   Queue q;  // only the counters and error word are used
   uint32_t* states;
   uint8_t* next_active;
@@ -579,40 +583,278 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
 // ------------------------------------------------------------------------------------------------------
 // ref-mode visit (C8, reference weight), gray only.
 //
-// Mirrors the reference's in-tile passes (dt/src/dt_block_passes.cuh:12-127): a row phase relaxes every
-// pixel from its three predecessors in the previous column (forward and backward chains interleaved), a
-// column phase from the three predecessors in the previous row.  The three rows (columns) move in lockstep,
-// so the predecessors of lane l come from lanes l-1 / l+1 by shuffle, or from the halo for the edge lanes.
-// Each relaxation is a single edge with the reference's arithmetic (ref_relax).  Neighbours (8 of them)
-// are re-activated when a border pixel facing them decreased, as in dt_block_passes.cuh:50-63, and on
-// visits that applied seeds.
+// The edges' |dI| are computed once per visit into four shared arrays (RefTile); the tile's distances are relaxed from
+// the halo once (values only decrease while the halo is fixed), then by phases that alternate between two layouts.
+// Column phase: lane = x, position k = y; every pixel is relaxed from its three predecessors in the row above (forward
+// chain) and below (backward chain).  Row phase: lane = y, position k = x, likewise from the columns beside it.  These are
+// the passes of the reference (dt/src/dt_block_passes.cuh:12-127) with the reference's arithmetic per edge; all edges of
+// a phase are in registers, so a step of a chain is two shuffles, five fused multiply-adds and three minima.
+// The visit ends at a phase that changes nothing if the edges along the other layout's chains, which it does not see,
+// hold too (the diagonal edges belong to both layouts).
 // ------------------------------------------------------------------------------------------------------
-constexpr int PIMG_STRIDE = 36;  // padded image copies: 34 lines x 36 bytes (9 words a line, odd word stride)
+constexpr float REF_SQ2 = 1.41421354f;  // sqrtf(2.f), reference generalised_distance_transform.cu:111
 
-// Pixel at position pos (-1..32) of an image line packed 4 per word (byte (pos + 1) & 3 of word (pos + 1) >> 2)
-// as a float.  pos is a constant after unrolling, so this is one bit-field extract and one conversion.
-__device__ __forceinline__ float line_px(const uint32_t (&w)[9], int pos) {
-  const int i = pos + 1;
-  return (float)((w[i >> 2] >> ((i & 3) * 8)) & 0xFFu);
+// D + l_eucl * {1, sqrt2} + l_grad * |dI| (ref_relax) with the parts that depend on the source alone taken out: `axial` /
+// `diagonal` of the source's distance, then `grad` with the edge's word (|dI|, or l_grad * |dI| rounded by itself
+// without FMA).  An edge that does not exist has an infinite word, so its candidate is infinite, or NaN when l_grad is
+// 0, and fminf and < pass over both.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+template <bool FMA>
+struct RefEdge {
+  float le, lg, le2;
+  __device__ __forceinline__ RefEdge(float l_eucl, float l_grad) : le(l_eucl), lg(l_grad), le2(mul_rn(l_eucl, REF_SQ2)) {}
+  __device__ __forceinline__ float axial(float q) const { return __fadd_rn(q, le); }  // l_eucl * 1 is exact
+  __device__ __forceinline__ float diagonal(float q) const { return FMA ? __fmaf_rn(le, REF_SQ2, q) : __fadd_rn(q, le2); }
+  __device__ __forceinline__ float grad(float e, float t) const { return FMA ? __fmaf_rn(lg, e, t) : __fadd_rn(t, e); }
+  __device__ __forceinline__ float word(uint32_t absdi) const {
+    const float f = __uint2float_rn(absdi);
+    return FMA ? f : __fmul_rn(lg, f);
+  }
+};
+
+// Edge words of a tile from its staged image box into t.V / Hh / DL / DR / E.  Returns this lane's sum of the axial
+// costs of the tile's internal column edges.
+template <bool FMA>
+__device__ __forceinline__ float ref_tile_weights(const RefEdge<FMA>& re, int vw, int vh, RefTile& t) {
+  const int lane = threadIdx.x & 31;
+  const float INF = f_inf();
+  const uint8_t* col = t.img + 16 + lane;  // column `lane` of the box, row r at col[r * IMG_BOX_GRAY]
+  auto ad = [](int a, int b) { return (uint32_t)abs(a - b); };
+  float wsum = 0.0f;
+  int ul = col[-1], u = col[0], ur = col[1];
+  {
+    const int c = col[IMG_BOX_GRAY];
+    t.E[E_TOP * 3 + lane] = re.word(ad(c, ul));
+    t.E[E_TOP * 3 + TILE + lane] = re.word(ad(c, u));
+    t.E[E_TOP * 3 + 2 * TILE + lane] = re.word(ad(c, ur));
+  }
+#pragma unroll 2
+  for (int y = 0; y < TILE; ++y) {
+    const uint8_t* pc = col + (y + 1) * IMG_BOX_GRAY;
+    const int l = pc[-1], c = pc[0], r = pc[1];
+    const bool in = lane < vw && y < vh;
+    const float wv = re.word(ad(c, u));
+    t.V[y * RS + lane] = in && y > 0 ? wv : INF;
+    t.Hh[y * RS + lane] = in && lane > 0 ? re.word(ad(c, l)) : INF;
+    t.DL[y * RS + lane] = in && y > 0 && lane > 0 ? re.word(ad(c, ul)) : INF;
+    t.DR[y * RS + lane] = in && y > 0 && lane + 1 < vw ? re.word(ad(c, ur)) : INF;
+    if (in && y > 0) wsum += re.grad(wv, re.le);
+    ul = l;
+    u = c;
+    ur = r;
+  }
+  {
+    const uint8_t* pb = col + (TILE + 1) * IMG_BOX_GRAY;
+    t.E[E_BOTTOM * 3 + lane] = re.word(ad(u, pb[-1]));
+    t.E[E_BOTTOM * 3 + TILE + lane] = re.word(ad(u, pb[0]));
+    t.E[E_BOTTOM * 3 + 2 * TILE + lane] = re.word(ad(u, pb[1]));
+  }
+  const uint8_t* row = t.img + (lane + 1) * IMG_BOX_GRAY + 16;  // row `lane`
+  const int cl = row[0], cr = row[TILE - 1];
+#pragma unroll
+  for (int o = 0; o < 3; ++o) {
+    t.E[E_LEFT * 3 + o * TILE + lane] = re.word(ad(cl, row[(o - 1) * IMG_BOX_GRAY - 1]));
+    t.E[E_RIGHT * 3 + o * TILE + lane] = re.word(ad(cr, row[(o - 1) * IMG_BOX_GRAY + TILE]));
+  }
+  t.DR[lane * RS + TILE] = INF;  // read as the word before the next row's first
+  t.DR[TILE * RS + lane] = INF;
+  return wsum;
 }
 
+// Halo of a tile in registers: the sides (lane = position along the side) and the corners (every lane).
+struct RefHalo {
+  float l, r, t, b, tl, tr, bl, br;
+};
+
+// The three halo pixels beside position `lane` of a side whose own pixel is h: before, at and after it.
+__device__ __forceinline__ void halo3(float (&o)[3], float h, float before, float after) {
+  const int lane = threadIdx.x & 31;
+  const float up = __shfl_up_sync(~0u, h, 1), dn = __shfl_down_sync(~0u, h, 1);
+  o[0] = lane == 0 ? before : up;
+  o[1] = h;
+  o[2] = lane == TILE - 1 ? after : dn;
+}
+
+// Relaxes the tile's border pixels in T from the halo; whether one of them fell.
 template <bool FMA>
-__device__ __forceinline__ float ref_min3(float cur, float da, float db, float dc, float le, float lg, float sq2,
-                                          float ia, float ib, float ic, bool diag_a, bool diag_c) {
-  // a and c are the diagonal predecessors, b the axial one
-  const float ra = ref_relax<FMA>(da, diag_a ? sq2 : 1.0f, le, lg, ia);
-  const float rb = ref_relax<FMA>(db, 1.0f, le, lg, ib);
-  const float rc = ref_relax<FMA>(dc, diag_c ? sq2 : 1.0f, le, lg, ic);
-  return fminf(cur, fminf(rb, fminf(ra, rc)));
+__device__ __forceinline__ bool ref_halo_relax(const RefEdge<FMA>& re, float* T, const float* E, const RefHalo& h, int vw, int vh) {
+  const int lane = threadIdx.x & 31;
+  bool low = false;
+  auto side = [&](float hh, float before, float after, const float* e, float* px, bool in) {
+    float o[3];
+    halo3(o, hh, before, after);
+    const float c = fminf(fminf(re.grad(e[lane], re.diagonal(o[0])), re.grad(e[TILE + lane], re.axial(o[1]))),
+                          re.grad(e[2 * TILE + lane], re.diagonal(o[2])));
+    if (in && c < *px) {
+      *px = c;
+      low = true;
+    }
+  };
+  side(h.t, h.tl, h.tr, E + E_TOP * 3, T + lane, lane < vw);
+  side(h.b, h.bl, h.br, E + E_BOTTOM * 3, T + (TILE - 1) * RS + lane, lane < vw && vh == TILE);
+  __syncwarp();
+  side(h.l, h.tl, h.bl, E + E_LEFT * 3, T + lane * RS, lane < vh);
+  side(h.r, h.tr, h.br, E + E_RIGHT * 3, T + lane * RS + TILE - 1, lane < vh && vw == TILE);
+  low = __any_sync(~0u, low);
+  __syncwarp();
+  return low;
+}
+
+// The smallest value the tile's border can bring to each neighbour below the halo it was compared with: lane k returns
+// neighbour k's (left, right, top, bottom, then the corners tl, tr, bl, br) as float bits, KEY_NONE if nothing.
+template <bool FMA>
+__device__ __forceinline__ uint32_t ref_border_keys(const RefEdge<FMA>& re, const float* T, const float* E, const RefHalo& h) {
+  const int lane = threadIdx.x & 31;
+  uint32_t kc[4] = {KEY_NONE, KEY_NONE, KEY_NONE, KEY_NONE};  // tl, tr, bl, br
+  auto side = [&](float hh, float before, float after, const float* e, float px, uint32_t& k0, uint32_t& k2) -> uint32_t {
+    float o[3];
+    halo3(o, hh, before, after);
+    const float c0 = re.grad(e[lane], re.diagonal(px)), c1 = re.grad(e[TILE + lane], re.axial(px)),
+                c2 = re.grad(e[2 * TILE + lane], re.diagonal(px));
+    uint32_t k = c1 < o[1] ? __float_as_uint(c1) : KEY_NONE;
+    const uint32_t u0 = c0 < o[0] ? __float_as_uint(c0) : KEY_NONE, u2 = c2 < o[2] ? __float_as_uint(c2) : KEY_NONE;
+    if (lane == 0) k0 = min(k0, u0); else k = min(k, u0);
+    if (lane == TILE - 1) k2 = min(k2, u2); else k = min(k, u2);
+    return __reduce_min_sync(~0u, k);
+  };
+  const uint32_t kt = side(h.t, h.tl, h.tr, E + E_TOP * 3, T[lane], kc[0], kc[1]);
+  const uint32_t kb = side(h.b, h.bl, h.br, E + E_BOTTOM * 3, T[(TILE - 1) * RS + lane], kc[2], kc[3]);
+  const uint32_t kl = side(h.l, h.tl, h.bl, E + E_LEFT * 3, T[lane * RS], kc[0], kc[2]);
+  const uint32_t kr = side(h.r, h.tr, h.br, E + E_RIGHT * 3, T[lane * RS + TILE - 1], kc[1], kc[3]);
+  const uint32_t ktl = __reduce_min_sync(~0u, kc[0]), ktr = __reduce_min_sync(~0u, kc[1]);
+  const uint32_t kbl = __reduce_min_sync(~0u, kc[2]), kbr = __reduce_min_sync(~0u, kc[3]);
+  return lane == 0 ? kl : lane == 1 ? kr : lane == 2 ? kt : lane == 3 ? kb : lane == 4 ? ktl : lane == 5 ? ktr
+       : lane == 6 ? kbl : lane == 7 ? kbr : KEY_NONE;
+}
+
+// One phase.  c[k]: edge between positions k - 1 and k of the own line; p[k] / n[k]: between position k of the own line and
+// position k - 1 of line l - 1 / l + 1.  The forward chain takes its diagonal predecessors from the neighbouring lanes;
+// in the backward chain the neighbours send their candidates, whose edges they hold.
+template <bool FMA>
+__device__ __forceinline__ bool ref_phase(const RefEdge<FMA>& re, float (&d)[TILE], const float (&c)[TILE], const float (&p)[TILE],
+                                          const float (&n)[TILE]) {
+  const int lane = threadIdx.x & 31;
+  const int lo = (lane + TILE - 1) % TILE, hi = (lane + 1) % TILE;  // edges across the warp's ends are infinite
+  bool ch = false;
+#pragma unroll
+  for (int s = 1; s < TILE; ++s) {
+    {
+      const int k = s;
+      const float q = d[k - 1], g = re.diagonal(q);
+      const float gl = __shfl_sync(~0u, g, lo), gr = __shfl_sync(~0u, g, hi);
+      const float a = fminf(d[k], re.grad(c[k], re.axial(q)));
+      const float v = fminf(a, fminf(re.grad(p[k], gl), re.grad(n[k], gr)));
+      ch |= v < d[k];
+      d[k] = v;
+    }
+    {
+      const int k = TILE - 1 - s;
+      const float q = d[k + 1], g = re.diagonal(q);
+      const float fl = __shfl_sync(~0u, re.grad(n[k + 1], g), lo), fr = __shfl_sync(~0u, re.grad(p[k + 1], g), hi);
+      const float a = fminf(d[k], re.grad(c[k + 1], re.axial(q)));
+      const float v = fminf(a, fminf(fl, fr));
+      ch |= v < d[k];
+      d[k] = v;
+    }
+  }
+  return __any_sync(~0u, ch);
+}
+
+// Loads the tile (and with `edges` the phase's edge words) in the column or row layout.
+__device__ __forceinline__ void ref_load_tile(float (&d)[TILE], const float* T, bool col) {
+  const int lane = threadIdx.x & 31;
+  if (col) {
+#pragma unroll
+    for (int k = 0; k < TILE; ++k) d[k] = T[k * RS + lane];
+  } else {
+#pragma unroll
+    for (int k = 0; k < TILE; ++k) d[k] = T[lane * RS + k];
+  }
+}
+__device__ __forceinline__ void ref_store_tile(float* T, const float (&d)[TILE], bool col) {
+  const int lane = threadIdx.x & 31;
+  if (col) {
+#pragma unroll
+    for (int k = 0; k < TILE; ++k) T[k * RS + lane] = d[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < TILE; ++k) T[lane * RS + k] = d[k];
+  }
+}
+__device__ __forceinline__ void ref_load_edges(float (&c)[TILE], float (&p)[TILE], float (&n)[TILE], const RefTile& t, bool col) {
+  const int lane = threadIdx.x & 31;
+  if (col) {
+#pragma unroll
+    for (int k = 0; k < TILE; ++k) {
+      c[k] = t.V[k * RS + lane];
+      p[k] = t.DL[k * RS + lane];
+      n[k] = t.DR[k * RS + lane];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < TILE; ++k) {
+      c[k] = t.Hh[lane * RS + k];
+      p[k] = t.DL[lane * RS + k];
+      n[k] = t.DR[(lane + 1) * RS + k - 1];  // (x - 1, y + 1) - (x, y), kept with its lower pixel
+    }
+  }
+}
+
+// Whether an edge along the chains (c) of this layout can lower a pixel.
+template <bool FMA>
+__device__ __forceinline__ bool ref_chain_low(const RefEdge<FMA>& re, const float (&d)[TILE], const float* row, int stride) {
+  bool low = false;
+#pragma unroll
+  for (int k = 1; k < TILE; ++k) {
+    const float e = row[k * stride];
+    low |= re.grad(e, re.axial(d[k - 1])) < d[k] || re.grad(e, re.axial(d[k])) < d[k - 1];
+  }
+  return __any_sync(~0u, low);
+}
+
+// Runs phases over the tile in t.img (T) until it is converged or `limit` phases have run; `col` is the layout to start
+// with, and to go on with.  Adds the phases to nph; whether the tile is not converged yet.  `changed` is set when a
+// value fell.
+template <bool FMA>
+__device__ __forceinline__ bool ref_solve(const RefEdge<FMA>& re, RefTile& t, bool& col, uint32_t limit, uint32_t& nph, bool& changed) {
+  const int lane = threadIdx.x & 31;
+  float* T = reinterpret_cast<float*>(t.img);
+  float d[TILE], c[TILE], p[TILE], n[TILE];
+  ref_load_tile(d, T, col);
+  for (uint32_t k = 0;; ) {
+    ref_load_edges(c, p, n, t, col);
+    const bool ch = ref_phase<FMA>(re, d, c, p, n);
+    changed |= ch;
+    ++nph;
+    ++k;
+    if (ch) {
+      ref_store_tile(T, d, col);
+      __syncwarp();
+    }
+    col = !col;
+    if (ch && k >= limit) return true;
+    ref_load_tile(d, T, col);
+    __syncwarp();
+    // A phase without change: the other layout's chain edges decide.
+    if (!ch && !ref_chain_low<FMA>(re, d, col ? t.V + lane : t.Hh + lane * RS, col ? RS : 1)) return false;
+    if (k >= limit) return true;
+  }
+}
+
+// Distances of a neighbour k (left, right, top, bottom, corners) at pixel (gx, gy): INF where there is no pixel, v where
+// the neighbour has not been visited.
+__device__ __forceinline__ float ref_halo_value(const ImgDesc& dd, uint32_t nexist, uint32_t nvis, int k, int gx, int gy, float v) {
+  if (!((nexist >> k) & 1u) || gx >= dd.width || gy >= dd.height) return f_inf();
+  return ((nvis >> k) & 1u) ? ld_dist(dd, gy, gx) : v;
 }
 
 template <bool FMA, class Sched>
 __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* tm_img, const CUtensorMap* tm_mask,
-                                          uint32_t tile, uint32_t old_state, WarpSmem& sm, uint32_t& parity,
+                                          uint32_t tile, uint32_t old_state, RefTile& sm, uint32_t& parity,
                                           const Sched& sch, uint32_t* nph_out, uint32_t* nact_out,
                                           bool rerun = false) {
-  // rerun: as in visit_ns -- the padded image lines (pimg / pimgT) and the tile values (T) of this tile's previous
-  // visit are still in the warp's shared memory; only the neighbour states and halos are read again.
+  // rerun: as in visit_ns -- the edge words and the tile values (T) of this tile's previous visit are still in the warp's
+  // shared memory; only the neighbour states and halos are read again.
   *nph_out = 0;
   *nact_out = 0;
   const int lane = threadIdx.x & 31;
@@ -623,10 +865,10 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
   const int vw = min(TILE, dd.width - x0), vh = min(TILE, dd.height - y0);
   const bool first = !(old_state & ST_VISITED);
   const bool seed = (old_state & ST_SEED) != 0;
-  const float v = dd.v, le = dd.l_eucl, lg = dd.l_grad;
-  const float sq2 = 1.41421354f;  // sqrtf(2.f), reference generalised_distance_transform.cu:111
+  const float v = dd.v;
+  const RefEdge<FMA> re(dd.l_eucl, dd.l_grad);
 
-  const VisitBufs vb = visit_bufs(sm, parity);
+  const VisitBufs vb{sm.img, sm.V, sm.V, sm.E, &sm.bar, &sm.bar, 1u, 1u, &parity};
   if (!rerun) stage_tile(vb, tm_img, tm_mask, false, seed, x0, y0);
 
   // Neighbour k = lane (0..7): (dx, dy) = L, R, T, B, TL, TR, BL, BR.
@@ -647,85 +889,51 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
   }
   fence_acq_rel();
 
-  // Halo rows / columns in shared memory, index = coordinate + 1 (corners appear in both).
-  float* ht = sm.Wh;                // top row   (y0 - 1), x = -1..32
-  float* hb = sm.Wh + 40;           // bottom row (y0 + 32)
-  float* hl = sm.Wv + 256;          // left column (x0 - 1), y = -1..32 (after the 1 KB seed-mask box)
-  float* hr = sm.Wv + 300;          // right column (x0 + 32)
-  auto halo_val = [&](int k, int gx, int gy) -> float {  // neighbour k's pixel (gx, gy)
-    if (!((nexist >> k) & 1u)) return INF;
-    if (gx >= dd.width || gy >= dd.height) return INF;
-    return ((nvis >> k) & 1u) ? ld_dist(dd, gy, gx) : v;
-  };
-  ht[lane + 1] = (lane < vw) ? halo_val(2, x0 + lane, y0 - 1) : INF;
-  hb[lane + 1] = (lane < vw) ? halo_val(3, x0 + lane, y0 + TILE) : INF;
-  hl[lane + 1] = (lane < vh) ? halo_val(0, x0 - 1, y0 + lane) : INF;
-  hr[lane + 1] = (lane < vh) ? halo_val(1, x0 + TILE, y0 + lane) : INF;
-  if (lane == 0) {
-    const float tl = halo_val(4, x0 - 1, y0 - 1), tr = halo_val(5, x0 + TILE, y0 - 1);
-    const float bl = halo_val(6, x0 - 1, y0 + TILE), br = halo_val(7, x0 + TILE, y0 + TILE);
-    ht[0] = tl; hl[0] = tl;
-    ht[TILE + 1] = tr; hr[0] = tr;
-    hb[0] = bl; hl[TILE + 1] = bl;
-    hb[TILE + 1] = br; hr[TILE + 1] = br;
-  }
+  RefHalo h;
+  h.t = lane < vw ? ref_halo_value(dd, nexist, nvis, 2, x0 + lane, y0 - 1, v) : INF;
+  h.b = lane < vw ? ref_halo_value(dd, nexist, nvis, 3, x0 + lane, y0 + TILE, v) : INF;
+  h.l = lane < vh ? ref_halo_value(dd, nexist, nvis, 0, x0 - 1, y0 + lane, v) : INF;
+  h.r = lane < vh ? ref_halo_value(dd, nexist, nvis, 1, x0 + TILE, y0 + lane, v) : INF;
+  h.tl = ref_halo_value(dd, nexist, nvis, 4, x0 - 1, y0 - 1, v);
+  h.tr = ref_halo_value(dd, nexist, nvis, 5, x0 + TILE, y0 - 1, v);
+  h.bl = ref_halo_value(dd, nexist, nvis, 6, x0 - 1, y0 + TILE, v);
+  h.br = ref_halo_value(dd, nexist, nvis, 7, x0 + TILE, y0 + TILE, v);
 
-  // Tile values live in T (column-layout transposes) = sm.img region after staging is consumed.
-  float* T = reinterpret_cast<float*>(sm.img);  // 32 x 33 floats = 4224 bytes <= 4352
-  float d[TILE];
-  if (rerun) {
+  float* T = reinterpret_cast<float*>(sm.img);  // overlays the image box once the edge words are computed
+  float wsum = 0.0f;
+  if (!rerun) {
+    float d[TILE];
+    if (!first) {
+      const uint8_t* lb = dist_base(dd, y0, x0 + lane, 0u);
 #pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = T[y * S_STRIDE + lane];
-  } else if (!first) {
-    const uint8_t* lb = dist_base(dd, y0, x0 + lane, 0u);
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
-  }
-
-  if (!rerun && !tma_wait(&sm.bar, parity, 1u, sch.q, tile)) return;
-
-  // Padded copies of the image box, one line per tile row and one per tile column (position -1..32 at byte
-  // pos + 1): pimg line r = box row r (tile row r - 1), pimgT line c = tile column c - 1.  In either layout
-  // lane l needs lines l, l + 1, l + 2 (its own line and the two beside it) of one of them.  A re-run has them.
-  uint8_t* pimg = reinterpret_cast<uint8_t*>(sm.Wh + 96);    // 34 * 36 = 1224 bytes after the halo rows
-  uint8_t* pimgT = reinterpret_cast<uint8_t*>(sm.Wh + 416);  // 1224 bytes after pimg
-  for (int i = lane; !rerun && i < IMG_BOX_ROWS * PIMG_STRIDE; i += 32) {
-    const int r = i / PIMG_STRIDE, c = i % PIMG_STRIDE;
-    const uint8_t px = (c < TILE + 2) ? sm.img[r * IMG_BOX_GRAY + 15 + c] : 0;
-    pimg[i] = px;
-    if (c < TILE + 2) pimgT[c * PIMG_STRIDE + r] = px;
-  }
-
-  if (first) {
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) {
-      const bool in = lane < vw && y < vh;
-      d[y] = in ? ((seed && mask_box(sm)[y * TILE + lane] != 0) ? 0.0f : v) : INF;
+      for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
     }
-  } else if (seed) {
+    if (!tma_wait(&sm.bar, parity, 1u, sch.q, tile)) return;
+    uint32_t seeds = 0;  // this lane's column of the mask tile (its box shares memory with V)
+    if (seed) {
+      const uint8_t* mbox = reinterpret_cast<const uint8_t*>(sm.V);
+#pragma unroll 4
+      for (int y = 0; y < TILE; ++y) seeds |= (lane < vw && y < vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
+    }
+    __syncwarp();
+    wsum = ref_tile_weights<FMA>(re, vw, vh, sm);
+    __syncwarp();
+    if (first) {
+#pragma unroll 4
+      for (int y = 0; y < TILE; ++y) T[y * RS + lane] = (lane < vw && y < vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
+    } else {
 #pragma unroll
-    for (int y = 0; y < TILE; ++y)
-      if (lane < vw && y < vh && mask_box(sm)[y * TILE + lane] != 0) d[y] = 0.0f;
+      for (int y = 0; y < TILE; ++y) T[y * RS + lane] = ((seeds >> y) & 1u) ? 0.0f : d[y];
+    }
+    __syncwarp();
   }
-  __syncwarp();
-
-  // From here on the image is needed through pimg only; T holds the tile.
-  // Initial border values for the change test, kept in shared memory through the phases (registers are the
-  // scarce resource there): top, bottom, left, right at border0[32 * side + lane].
-  float* border0 = sm.Wv + 352;  // after the halo columns
-  border0[lane] = d[0];
-  border0[32 + lane] = d[TILE - 1];
-#pragma unroll
-  for (int y = 0; y < TILE; ++y) T[y * S_STRIDE + lane] = d[y];
-  __syncwarp();
-  border0[64 + lane] = T[lane * S_STRIDE];
-  border0[96 + lane] = T[lane * S_STRIDE + TILE - 1];
-  __syncwarp();
-
-  auto P = [&](int r, int c) -> float {  // pixel at tile (c, r) as float, r, c in [-1, 32]
-    return (float)pimg[(r + 1) * PIMG_STRIDE + c + 1];
-  };
-  auto absd = [](float a, float b) { return fabsf(a - b); };  // exact for integers in [0, 255]
+  if constexpr (Sched::any_change) {  // the border as it was, lane = position along the side
+    sm.B0[E_TOP + lane] = T[lane];
+    sm.B0[E_BOTTOM + lane] = T[(TILE - 1) * RS + lane];
+    sm.B0[E_LEFT + lane] = T[lane * RS];
+    sm.B0[E_RIGHT + lane] = T[lane * RS + TILE - 1];
+    __syncwarp();
+  }
 
   // Bucket width of this image (priority queue): half a tile-width of the mean axial edge cost
   // l_eucl + l_grad * |dI| seen by first visits (vertical edges of the tile).
@@ -733,22 +941,11 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
   if (sch.q.wacc) {
     float* wa = sch.q.wacc + 2 * (old_state >> ST_IMG_SHIFT);
     if (first) {
-      float wsum = 0.0f, wcnt = 0.0f;
-      if (lane < vw) {
-#pragma unroll 1
-        for (int y = 1; y < vh; ++y) {
-          wsum += le + lg * absd(P(y, lane), P(y - 1, lane));
-          wcnt += 1.0f;
-        }
-      }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        wsum += __shfl_xor_sync(~0u, wsum, o);
-        wcnt += __shfl_xor_sync(~0u, wcnt, o);
-      }
-      if (lane == 0 && wcnt > 0.0f) {
+      for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(~0u, wsum, o);
+      if (lane == 0 && vh > 1) {
         atomicAdd(&wa[0], wsum);
-        atomicAdd(&wa[1], wcnt);
+        atomicAdd(&wa[1], (float)(vw * (vh - 1)));
       }
     }
     const float s_ = *(volatile float*)&wa[0], c_ = *(volatile float*)&wa[1];
@@ -756,139 +953,40 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
     inv_width = (c_ > 0.0f && s_ > 0.0f) ? c_ / (bt * (float)TILE * s_) : 1.0f / (bt * (float)TILE);
   }
 
-  bool any = false;
+  bool any = ref_halo_relax<FMA>(re, T, sm.E, h, vw, vh);
   uint32_t nph = 0;
-  bool col = true;
-  for (;;) {
-    bool ch = false;
-    // One code path for both layouts.  Column phase (lane = x, position k = y): forward over y from the three
-    // predecessors (x-1..x+1, y-1), backward from (x-1..x+1, y+1).  Row phase (lane = y, k = x): forward over x
-    // from (x-1, y-1..y+1), backward from (x+1, y-1..y+1).  Lanes l-1 / l+1 hold the diagonal predecessors (by
-    // shuffle); the edge lanes take them from the halo beside the tile (`side_lo` / `side_hi`), and position
-    // -1 / 32 from the halo across the chain (`lo` / `hi`).  The lane's image lines (its own and the two beside
-    // it) are loaded once per phase.  The forward and the backward chain are interleaved (two independent
-    // dependency chains per warp); every step is the same single-edge relaxation as in the reference passes,
-    // so the order does not change the fixpoint.
-    const float* lo = col ? ht : hl;
-    const float* hi = col ? hb : hr;
-    const float* side_lo = col ? hl : ht;
-    const float* side_hi = col ? hr : hb;
-    const bool lane_in = lane < (col ? vw : vh);
-    const int kmax = col ? vh : vw;
-    uint32_t L0[9], L1[9], L2[9];
-    {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>((col ? pimgT : pimg) + lane * PIMG_STRIDE);
-#pragma unroll
-      for (int j = 0; j < 9; ++j) {
-        L0[j] = w[j];
-        L1[j] = w[9 + j];
-        L2[j] = w[18 + j];
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < TILE; ++k) {
-      {
-        float pa, pb, pc;
-        if (k == 0) { pa = lo[lane]; pb = lo[lane + 1]; pc = lo[lane + 2]; }
-        else {
-          pb = d[k - 1];
-          pa = __shfl_up_sync(~0u, pb, 1);
-          pc = __shfl_down_sync(~0u, pb, 1);
-          if (lane == 0) pa = side_lo[k];
-          if (lane == TILE - 1) pc = side_hi[k];
-        }
-        const float c = line_px(L1, k);
-        const float nd = ref_min3<FMA>(d[k], pa, pb, pc, le, lg, sq2, absd(c, line_px(L0, k - 1)),
-                                       absd(c, line_px(L1, k - 1)), absd(c, line_px(L2, k - 1)), true, true);
-        const bool upd = lane_in && k < kmax && nd < d[k];
-        ch |= upd;
-        d[k] = upd ? nd : d[k];
-      }
-      {
-        const int j = TILE - 1 - k;
-        float pa, pb, pc;
-        if (j == TILE - 1) { pa = hi[lane]; pb = hi[lane + 1]; pc = hi[lane + 2]; }
-        else {
-          pb = d[j + 1];
-          pa = __shfl_up_sync(~0u, pb, 1);
-          pc = __shfl_down_sync(~0u, pb, 1);
-          if (lane == 0) pa = side_lo[j + 2];
-          if (lane == TILE - 1) pc = side_hi[j + 2];
-        }
-        const float c = line_px(L1, j);
-        const float nd = ref_min3<FMA>(d[j], pa, pb, pc, le, lg, sq2, absd(c, line_px(L0, j + 1)),
-                                       absd(c, line_px(L1, j + 1)), absd(c, line_px(L2, j + 1)), true, true);
-        const bool upd = lane_in && j < kmax && nd < d[j];
-        ch |= upd;
-        d[j] = upd ? nd : d[j];
-      }
-    }
-    ch = __any_sync(~0u, ch);
-    any |= ch;
-    ++nph;
-    if (col) {
-#pragma unroll
-      for (int y = 0; y < TILE; ++y) T[y * S_STRIDE + lane] = d[y];
-    } else {
-#pragma unroll
-      for (int x = 0; x < TILE; ++x) T[lane * S_STRIDE + x] = d[x];
-    }
-    __syncwarp();
-    if ((!ch && nph >= 2) || nph >= (uint32_t)PHASE_LIMIT) break;
-    if (col) {
-#pragma unroll
-      for (int x = 0; x < TILE; ++x) d[x] = T[lane * S_STRIDE + x];
-    } else {
-#pragma unroll
-      for (int y = 0; y < TILE; ++y) d[y] = T[y * S_STRIDE + lane];
-    }
-    col = !col;
-    __syncwarp();
+  if (any || seed) {
+    bool col = true;
+    if (ref_solve<FMA>(re, sm, col, (uint32_t)PHASE_LIMIT, nph, any) && lane == 0) set_error(sch.q, DERR_PHASE_LIMIT, tile);
   }
-  if (nph >= (uint32_t)PHASE_LIMIT && lane == 0) set_error(sch.q, DERR_PHASE_LIMIT, tile);
 
-  // Border changes -> neighbours (bit k = neighbour k as in ndx_l / ndy_l), as the reference activates blocks
-  // (dt_block_passes.cuh:50-63).  An exact "can this border lower the neighbour's halo" test (as in ns-mode)
-  // removed only a tenth of the visits here and cost more than it saved: most re-visits in ref-mode carry
-  // last-bit improvements of equally long paths summed in another order, which that test also lets through.
-  // The activation's priority is the smallest border value facing the neighbour.
+  // Neighbours to activate (bit k = neighbour k as in ndx_l / ndy_l) and the value each is activated at: the ones the
+  // border can lower; in host-driven rounds the ones whose facing border changed (dt_block_passes.cuh:50-63), so that
+  // the round counters count what the reference's do.
   uint32_t act = 0;
   float key = 0.0f;
   if (any || seed) {
-    const bool force = seed;
-    const float bt = T[lane], bb = T[(TILE - 1) * S_STRIDE + lane];
-    const float bl = T[lane * S_STRIDE], br = T[lane * S_STRIDE + TILE - 1];
-    const uint32_t ct = __ballot_sync(~0u, force || bt != border0[lane]);
-    const uint32_t cb = __ballot_sync(~0u, force || bb != border0[32 + lane]);
-    const uint32_t cl = __ballot_sync(~0u, force || bl != border0[64 + lane]);
-    const uint32_t cr = __ballot_sync(~0u, force || br != border0[96 + lane]);
-    act |= cl ? 1u : 0u;
-    act |= cr ? 2u : 0u;
-    act |= ct ? 4u : 0u;
-    act |= cb ? 8u : 0u;
-    act |= (ct & 1u) ? 16u : 0u;
-    act |= (ct >> (TILE - 1)) & 1u ? 32u : 0u;
-    act |= (cb & 1u) ? 64u : 0u;
-    act |= (cb >> (TILE - 1)) & 1u ? 128u : 0u;
-    act &= nexist;
-    if (act) {
-      const uint32_t kl = __reduce_min_sync(~0u, __float_as_uint(bl));
-      const uint32_t kr = __reduce_min_sync(~0u, __float_as_uint(br));
-      const uint32_t kt = __reduce_min_sync(~0u, __float_as_uint(bt));
-      const uint32_t kb = __reduce_min_sync(~0u, __float_as_uint(bb));
-      const float corner = lane == 4 ? T[0] : lane == 5 ? T[TILE - 1] : lane == 6 ? T[(TILE - 1) * S_STRIDE]
-                                                                                    : T[(TILE - 1) * S_STRIDE + TILE - 1];
-      key = lane == 0 ? __uint_as_float(kl) : lane == 1 ? __uint_as_float(kr) : lane == 2 ? __uint_as_float(kt)
-          : lane == 3 ? __uint_as_float(kb) : corner;
+    if constexpr (Sched::any_change) {
+      const uint32_t ct = __ballot_sync(~0u, seed || T[lane] != sm.B0[E_TOP + lane]);
+      const uint32_t cb = __ballot_sync(~0u, seed || T[(TILE - 1) * RS + lane] != sm.B0[E_BOTTOM + lane]);
+      const uint32_t cl = __ballot_sync(~0u, seed || T[lane * RS] != sm.B0[E_LEFT + lane]);
+      const uint32_t cr = __ballot_sync(~0u, seed || T[lane * RS + TILE - 1] != sm.B0[E_RIGHT + lane]);
+      act = (cl ? 1u : 0u) | (cr ? 2u : 0u) | (ct ? 4u : 0u) | (cb ? 8u : 0u) | ((ct & 1u) ? 16u : 0u) |
+            ((ct >> (TILE - 1)) & 1u ? 32u : 0u) | ((cb & 1u) ? 64u : 0u) | ((cb >> (TILE - 1)) & 1u ? 128u : 0u);
+    } else {
+      const uint32_t k = ref_border_keys<FMA>(re, T, sm.E, h);
+      act = __ballot_sync(~0u, k != KEY_NONE);
+      key = __uint_as_float(k);
     }
+    act &= nexist;
   }
 
-  if (any || first) {
+  if (any || first || seed) {
     if (lane < vw) {
       uint8_t* wb = dist_base(dd, y0, x0 + lane, nph);
-#pragma unroll
+#pragma unroll 4
       for (int y = 0; y < TILE; ++y)
-        if (y < vh) *reinterpret_cast<float*>(wb + (int64_t)y * dd.dist_pitch) = T[y * S_STRIDE + lane];
+        if (y < vh) *reinterpret_cast<float*>(wb + (int64_t)y * dd.dist_pitch) = T[y * RS + lane];
     }
   }
   fence_acq_rel();
@@ -902,28 +1000,33 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
 
 // MODE is fixed per kernel instantiation: a launch covers images of one weight mode (and, in ref-mode, one
 // rounding) only, so no kernel's register allocation is inflated by another mode's code.
+template <int MODE>
+using TileSmem = std::conditional_t<MODE == MODE_NS, WarpSmem, RefTile>;  // a warp's shared memory
+
 template <int MODE, class Sched>
 __device__ __forceinline__ void visit_tile(const ImgDesc& dd, const CUtensorMap* tmaps, uint32_t img, uint32_t tile,
-                                           uint32_t old_state, WarpSmem& sm, uint32_t& parity, const Sched& sch,
+                                           uint32_t old_state, TileSmem<MODE>& sm, uint32_t& parity, const Sched& sch,
                                            WarpStats& ws, bool rerun = false) {
   const CUtensorMap* tm_img = tmaps + 2 * img;
   const CUtensorMap* tm_mask = tmaps + 2 * img + 1;
   uint32_t nph, nact;
-  if (MODE == MODE_NS)
+  if constexpr (MODE == MODE_NS)
     visit_ns<false>(dd, tm_img, tm_mask, tile, old_state, visit_bufs(sm, parity), sch, &nph, &nact, rerun);
-  else if (MODE == MODE_REF)
+  else if constexpr (MODE == MODE_REF)
     visit_ref<true>(dd, tm_img, tm_mask, tile, old_state, sm, parity, sch, &nph, &nact, rerun);
   else
     visit_ref<false>(dd, tm_img, tm_mask, tile, old_state, sm, parity, sch, &nph, &nact, rerun);
   count_visit(ws, sch.q, nph, nact);
 }
 
-__device__ __forceinline__ WarpSmem& warp_slot(uint8_t* smem_raw) {
+template <class Smem = WarpSmem>
+__device__ __forceinline__ Smem& warp_slot(uint8_t* smem_raw) {
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  return reinterpret_cast<WarpSmem*>(base)[threadIdx.x >> 5];
+  return reinterpret_cast<Smem*>(base)[threadIdx.x >> 5];
 }
 
-__device__ __forceinline__ void warp_slot_init(WarpSmem& sm) {
+template <class Smem>
+__device__ __forceinline__ void warp_slot_init(Smem& sm) {
   if ((threadIdx.x & 31) == 0) {
     mbar_init(&sm.bar, 1);
     fence_mbar_init();

@@ -68,3 +68,28 @@ def test_both_sides_of_the_size_rule_are_fixpoints():
         va, vb, _ = ns_fixpoint_violations(ti, tm, gamma, 1e10, d)
         assert (va, vb) == (0, 0), "side %d: %d pixels could fall, %d have no source" % (side, va, vb)
         c.close()
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 65), (33, 31), (63, 64), (64, 64), (65, 129), (96, 160), (193, 257)])
+@pytest.mark.parametrize("lam", [0.0, 0.3, 1.0])
+def test_ref_mode_blocks_tiles_and_rounds(fresh, h, w, lam):
+    """Reference weight: the block kernel, the tile kernel (a context with a tuning of its own) and the host-driven rounds,
+    with and without FMA, from seeds in each corner (fronts that cross blocks over their corners) and none."""
+    rng = np.random.default_rng(h * 1000 + w)
+    tiles = dtb.Context(0)
+    tiles.set_tuning(ctas_per_sm=2)
+    for kind in ("noise", "flat", "steps"):
+        img = (rng.integers(0, 256, (h, w)) if kind == "noise" else np.zeros((h, w)) if kind == "flat"
+               else np.add.outer(np.arange(h) // 7 * 40, np.arange(w) // 5 * 30) % 256).astype(np.uint8)
+        for y, x, v in ((0, 0, 1e10), (h - 1, 0, 1e10), (0, w - 1, 60.0), (h - 1, w - 1, 1e10), (-1, -1, 5.0)):
+            mask = np.zeros((h, w), np.uint8)
+            if y >= 0:
+                mask[y, x] = 1
+            ti, tm = torch.from_numpy(img).cuda(), torch.from_numpy(mask).cuda()
+            for fma in (True, False):
+                want = orc.ggdt_ref(img, mask, lam, v, fma)
+                what = "%s %dx%d lambda %g seed (%d, %d) fma %d: " % (kind, h, w, lam, y, x, fma)
+                assert_images_eq(dtb.generalised_distance_transform_task(ti, tm, lam, v, ctx=fresh, fma=fma), want, what + "blocks of tiles")
+                assert_images_eq(dtb.generalised_distance_transform_task(ti, tm, lam, v, ctx=tiles, fma=fma), want, what + "tiles")
+                assert_images_eq(dtb.generalised_distance_transform_blocks(ti, tm, lam, v, ctx=fresh, fma=fma), want, what + "rounds")
+    tiles.close()
