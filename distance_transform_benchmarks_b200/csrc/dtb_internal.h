@@ -18,6 +18,7 @@ namespace dtb {
 
 constexpr int PERSIST_WPC = 4;   // warps per CTA of the persistent tile kernel
 constexpr int ROUND_WPC = 4;
+constexpr int ROUND_BATCH = 8;   // host-driven rounds enqueued per synchronisation
 constexpr size_t PERSIST_SMEM = PERSIST_WPC * sizeof(WarpSmem) + 128;
 constexpr size_t PERSIST_SMEM_AHEAD = PERSIST_WPC * sizeof(WarpSmemP) + 128;
 constexpr size_t ROUND_SMEM = ROUND_WPC * sizeof(WarpSmem) + 128;
@@ -48,6 +49,12 @@ inline int ns_variant_of(int ctas, bool ahead, int wpc = PERSIST_WPC) {
 }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// What a rounds call reads back per batch.
+struct RoundStatus {
+  uint32_t changed[ROUND_BATCH];  // whether round k activated a tile
+  uint32_t error, progress;
+};
 
 // One image of a call, resolved to device memory.
 struct Job {
@@ -173,6 +180,7 @@ struct dtb_context_s {
   int32_t* dround_counts = nullptr;
   size_t dround_counts_size = 0;
   bool count_rounds = false;
+  dtb::RoundStatus* hrounds = nullptr;
   // dtb_debug_inject_queue_stall: no-progress limit of the next persistent run (0 = no injection, one-shot).
   uint64_t inject_stall_ns = 0;
   std::mutex mu;
