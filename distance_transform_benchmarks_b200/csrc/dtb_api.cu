@@ -477,6 +477,10 @@ uint32_t count_blocks(const std::vector<Job>& jobs) {
   return (uint32_t)t;
 }
 
+static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t) {
+  return std::max<uint32_t>(1u, (uint32_t)(ctx->num_sms * BLOCK_CTAS) * (uint32_t)t.grid_percent / 100u);
+}
+
 // Whether a run takes the block kernel: under the default tuning, up to as many blocks as its CTAs may own (9472 on 148
 // SMs, 38 Mpx).  Up to there chains of dependent visits bound the run.  ns-mode: the block kernel is faster or as fast
 // (tile against block kernel: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze 4.2 / 4.1,
@@ -484,13 +488,12 @@ uint32_t count_blocks(const std::vector<Job>& jobs) {
 // images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5).  ref-mode, lambda 0 / 0.5 / 1: 1023x777 0.40 / 0.69 / 0.91 ms
 // against 0.23 / 0.56 / 0.80, 3648x2432 1.21 / 2.02 / 1.74 against 0.98 / 2.30 / 1.67, 6000^2 2.8 / 4.7 / 3.2 against 2.3 / 5.9 / 2.5.
 bool use_blocks(dtb_context ctx, int mode, const LaunchTuning& t, uint32_t blocks) {
-  return !t.chosen && blocks > 0 &&
-         blocks <= std::min((uint32_t)(ctx->num_sms * BLOCK_CTAS * BLOCK_OWNED_MAX), BLOCK_RUN_MAX);
+  (void)mode;
+  return !t.chosen && blocks > 0 && blocks <= std::min(block_grid(ctx, t) * (uint32_t)BLOCK_OWNED_MAX, BLOCK_RUN_MAX);
 }
 
-// A run of the block kernel: one memset (header, block states, keys) and one launch.
-static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, cudaStream_t stream, cudaEvent_t ev0,
-                                 cudaEvent_t ev1) {
+dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
+                          cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1) {
   const uint64_t stall_ns = ctx->inject_stall_ns;
   ctx->inject_stall_ns = 0;
   const ImgDesc* ddesc = reinterpret_cast<const ImgDesc*>(dbase + L.o_desc);
@@ -510,7 +513,7 @@ static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchL
   }
   if (ev0) DTB_CUDA(ctx, cudaEventRecord(ev0, stream));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, (uint32_t)(ctx->num_sms * BLOCK_CTAS)));
+  cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, block_grid(ctx, t)));
   cfg.blockDim = dim3(BLOCK_WARPS * 32);
   cfg.dynamicSmemBytes = mode == MODE_NS ? BLOCK_SMEM<MODE_NS> : BLOCK_SMEM<MODE_REF>;
   cfg.stream = stream;
@@ -530,7 +533,13 @@ static dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchL
 
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
                               cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, QueueHdr* fold) {
-  if (!fold && L.total && use_blocks(ctx, mode, t, L.blocks)) return enqueue_blocks(ctx, dbase, L, mode, stream, ev0, ev1);
+  if (L.total && use_blocks(ctx, mode, t, L.blocks)) {
+    const dtb_status bs = enqueue_blocks(ctx, dbase, L, mode, t, stream, ev0, ev1);
+    if (bs != DTB_OK || !fold) return bs;
+    ggdt_finalize<<<1, 32, 0, stream>>>(nullptr, nullptr, 0, 0, nullptr, reinterpret_cast<const QueueHdr*>(dbase + L.o_hdr), fold);
+    DTB_CUDA(ctx, cudaGetLastError());
+    return DTB_OK;
+  }
   const uint64_t stall_ns = ctx->inject_stall_ns;
   ctx->inject_stall_ns = 0;
   Queue q = make_queue(dbase, L, stall_ns ? stall_ns : DEFAULT_TIMEOUT_NS, &t);

@@ -141,6 +141,7 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&descs[ctl.owned_img[__shfl_sync(~0u, pick, win)]]);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&ctl.desc);
         for (int i = lane; i < (int)(sizeof(ImgDesc) / 4); i += 32) dst[i] = src[i];
+        __syncwarp();
       }
       if (lane == win) {
         atomicAdd(&a.hdr->pending.v, (uint32_t)SIDES);
@@ -152,11 +153,12 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
           ctl.seen[s][pick] = got[s] >> 1;
         }
         const uint32_t bit = 1u << (pick & 31u), seed = ctl.seeded[pick >> 5] & bit;
-        ctl.nvis = nvis;
+        const bool warm = ctl.desc.warm != 0;
+        ctl.nvis = warm ? ~0u : nvis;
         ctl.next = pick;
         ctl.tokens = (uint32_t)SIDES + fresh + (seed ? 1u : 0u);
         ctl.seed = seed ? 1u : 0u;
-        ctl.first = (ctl.visited[pick >> 5] & bit) ? 0u : 1u;
+        ctl.first = warm || (ctl.visited[pick >> 5] & bit) ? 0u : 1u;
         ctl.rerun = pick == prev && !seed ? 1u : 0u;
         ctl.visited[pick >> 5] |= bit;
         ctl.seeded[pick >> 5] &= ~bit;
@@ -330,8 +332,14 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
         for (int y = 0; y < TILE; ++y)
           pb[y * W_STRIDE] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
       } else {
+        bool low = false;  // a seed on a pixel that is 0 already asks for nothing
 #pragma unroll
-        for (int y = 0; y < TILE; ++y) pb[y * W_STRIDE] = ((seeds >> y) & 1u) ? 0.0f : d[y];
+        for (int y = 0; y < TILE; ++y) {
+          const bool s = ((seeds >> y) & 1u) != 0u;
+          low |= s && d[y] > 0.0f;
+          pb[y * W_STRIDE] = s ? 0.0f : d[y];
+        }
+        todo = changed = __any_sync(~0u, low);
       }
       if (first) flags |= BLOCK_UNSAVED;
     }
@@ -511,8 +519,14 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
         for (int y = 0; y < TILE; ++y) T[y * RS + lane] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
         flags |= BLOCK_UNSAVED;
       } else {
+        bool low = false;
 #pragma unroll
-        for (int y = 0; y < TILE; ++y) T[y * RS + lane] = ((seeds >> y) & 1u) ? 0.0f : d[y];
+        for (int y = 0; y < TILE; ++y) {
+          const bool s = ((seeds >> y) & 1u) != 0u;
+          low |= s && d[y] > 0.0f;
+          T[y * RS + lane] = s ? 0.0f : d[y];
+        }
+        todo = changed = __any_sync(~0u, low);
       }
     }
   }
@@ -649,6 +663,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
     const uint32_t blk = first + (uint32_t)i * step;
     if ((sm.ctl.visited[i >> 5] >> (i & 31)) & 1u) continue;
     const ImgDesc& dd = descs[sm.ctl.owned_img[i]];
+    if (dd.warm) continue;
     const uint32_t local = blk - dd.block_base;
     const int x0 = (int)(local % (uint32_t)dd.blocks_x) * BLOCK_W + (warp % BLOCK_TX) * TILE;
     const int y0 = (int)(local / (uint32_t)dd.blocks_x) * BLOCK_H + (warp / BLOCK_TX) * TILE;

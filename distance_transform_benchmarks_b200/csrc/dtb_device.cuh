@@ -72,6 +72,7 @@ struct alignas(64) ImgDesc {
   int32_t ref_fma;  // ref-mode: 1 = fma(l_grad, dI, fma(l_eucl, d, D)), 0 = left-to-right rounding
   int32_t blocks_x, blocks_y;  // block kernel: blocks of 4 x 4 tiles
   uint32_t block_base;
+  int32_t warm;  // block kernel: the map holds a fixpoint of some of the seeds already (serving: a seed edit)
 };
 
 // Counters live on separate 128-byte lines.

@@ -229,11 +229,14 @@ dtb_status count_tiles(dtb_context ctx, const std::vector<Job>& jobs, uint32_t* 
 // Resident warps of the tile kernel of `mode` under `t`.
 uint32_t resident_workers(dtb_context ctx, int mode, const LaunchTuning& t);
 // Enqueues queue reset, seed scan, the persistent tile kernel and finalize on `stream` (capturable); or the block
-// kernel, where use_blocks says so and there is nothing to fold.
+// kernel, where use_blocks says so.
 // ev0 / ev1 (optional) are recorded around the tile kernel; `fold` (optional) receives the run's status and
 // counters, added by finalize.
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
                               cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, QueueHdr* fold = nullptr);
+// Enqueues a run of the block kernel: one memset (header and messages) and one launch.
+dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
+                          cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1);
 // Enqueues the cooperative persistent tile kernel of `mode` under `t` (grid: resident_workers / PERSIST_WPC).
 dtb_status launch_tile_kernel(dtb_context ctx, int mode, const LaunchTuning& t, const ImgDesc* descs,
                               const CUtensorMap* tmaps, uint32_t* states, const Queue& q, cudaStream_t stream);

@@ -504,7 +504,9 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
   if ((s2 = count_tiles(ctx, jobs, &total)) != DTB_OK) return s2;
   LaunchTuning tuning = ctx->tuning;
   tuning.buckets = (int)std::min<uint32_t>((uint32_t)tuning.buckets, s->nb);
-  const ScratchLayout L = layout_for(n, total, s->workers, false, s->nb);
+  ScratchLayout L = layout_for(n, total, s->workers, false, s->nb);
+  L.blocks = count_blocks(jobs);
+  const bool blocks = total > 0 && use_blocks(ctx, MODE_NS, tuning, L.blocks);
   size_t o_warm = 0, o_disks = 0, o_items = 0;
   const size_t off = wave_scratch_bytes(L, n, disks.size(), items.size(), &o_warm, &o_disks, &o_items);
   if (off > ws.scratch_size)  // admission keeps a wave within the slot's scratch
@@ -512,6 +514,7 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
   uint8_t* sc = static_cast<uint8_t*>(ws.scratch);
   std::vector<uint8_t> tab;
   if ((s2 = build_tables(ctx, jobs, L, tab)) != DTB_OK) return s2;
+  for (int i = 0; i < n; ++i) reinterpret_cast<ImgDesc*>(tab.data())[i].warm = warm[i];
   // Tables, warm flags, disks and repitch items: one upload from the slot's pinned buffer (free: the slot's
   // previous wave has ended), so that the copy does not wait for the other wave's work.
   const size_t hbytes = off - L.o_desc;
@@ -530,8 +533,10 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
   DTB_CUDA(ctx, cudaEventRecord(ws.ev_in, s->s_in));
   DTB_CUDA(ctx, cudaStreamWaitEvent(st, ws.ev_in, 0));
   DTB_CUDA(ctx, cudaEventRecord(ws.t_run0, st));
-  const dtb_status qs = reset_queue(ctx, sc, L, st);
-  if (qs != DTB_OK) return qs;
+  if (!blocks) {
+    const dtb_status qs = reset_queue(ctx, sc, L, st);
+    if (qs != DTB_OK) return qs;
+  }
   const ImgDesc* ddesc = reinterpret_cast<const ImgDesc*>(sc + L.o_desc);
   const CUtensorMap* dtm = reinterpret_cast<const CUtensorMap*>(sc + L.o_tmap);
   const uint32_t* dbase = reinterpret_cast<const uint32_t*>(sc + L.o_base);
@@ -539,7 +544,7 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
   // dtb_debug_inject_queue_stall on the server's context applies to the next wave with tiles (one-shot; the
   // caller holds ctx->mu).
   uint64_t stall_ns = 0;
-  if (total > 0) {
+  if (total > 0 && !blocks) {
     stall_ns = ctx->inject_stall_ns;
     ctx->inject_stall_ns = 0;
   }
@@ -556,9 +561,13 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
                                                                              (int)disks.size());
     DTB_CUDA(ctx, cudaGetLastError());
   }
-  if (total > 0) {
-    const uint32_t blocks = std::min<uint32_t>((total + 3) / 4, (uint32_t)ctx->num_sms * 16);
-    serve_wave_init<<<blocks, 128, 0, st>>>(ddesc, dbase, sc + o_warm, n, total, states, q);
+  if (blocks) {
+    // The block kernel scans the masks itself: a warm image's old seeds are 0 in its map already and ask for nothing.
+    const dtb_status bs = enqueue_blocks(ctx, sc, L, MODE_NS, tuning, st, nullptr, nullptr);
+    if (bs != DTB_OK) return bs;
+  } else if (total > 0) {
+    const uint32_t scan_blocks = std::min<uint32_t>((total + 3) / 4, (uint32_t)ctx->num_sms * 16);
+    serve_wave_init<<<scan_blocks, 128, 0, st>>>(ddesc, dbase, sc + o_warm, n, total, states, q);
     DTB_CUDA(ctx, cudaGetLastError());
     if (!disks.empty()) {
       serve_seed_tiles<<<std::min<int>((int)disks.size(), 4096), 32, 0, st>>>(
@@ -571,7 +580,7 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
     }
     const dtb_status ls = launch_tile_kernel(ctx, MODE_NS, tuning, ddesc, dtm, states, q, st);
     if (ls != DTB_OK) return ls;
-    ggdt_finalize<<<blocks, 128, 0, st>>>(ddesc, dbase, n, total, states, nullptr, nullptr);
+    ggdt_finalize<<<scan_blocks, 128, 0, st>>>(ddesc, dbase, n, total, states, nullptr, nullptr);
     DTB_CUDA(ctx, cudaGetLastError());
   }
   DTB_CUDA(ctx, cudaEventRecord(ws.t_run1, st));

@@ -93,3 +93,44 @@ def test_ref_mode_blocks_tiles_and_rounds(fresh, h, w, lam):
                 assert_images_eq(dtb.generalised_distance_transform_task(ti, tm, lam, v, ctx=tiles, fma=fma), want, what + "tiles")
                 assert_images_eq(dtb.generalised_distance_transform_blocks(ti, tm, lam, v, ctx=fresh, fma=fma), want, what + "rounds")
     tiles.close()
+
+
+@pytest.mark.parametrize("tuned", [False, True])
+def test_wave_edits_through_either_kernel(tuned):
+    """Serve waves run the block kernel under the default tuning and the tile kernel under one of the caller's: new images
+    and repeated seed edits (inside, across blocks, on old seeds, outside the picture) equal cold runs on all seeds."""
+    c = dtb.Context(0)
+    if tuned:
+        c.set_tuning(ctas_per_sm=2)
+    srv = dtb.Server(1 << 28, ctx=c)
+    rng = np.random.default_rng(4)
+    imgs = [rng.integers(0, 256, (150, 333, 3), dtype=np.uint8), rng.integers(0, 256, (64, 65), dtype=np.uint8)]
+    masks = [np.zeros(i.shape[:2], np.uint8) for i in imgs]
+    masks[0][5, 7] = masks[1][63, 0] = 1
+
+    def ask(n, outs):
+        for _ in range(n):
+            for a in srv.poll(8, wait_ms=5000):
+                assert a["status"] == 0
+                n -= 1
+            if n <= 0:
+                break
+        for k, o in outs:
+            assert_images_eq(o, orc.ggdt_ns(imgs[k], masks[k], 0.2), "image %d tuned %d" % (k, tuned))
+
+    outs = [(k, torch.empty(imgs[k].shape[:2])) for k in range(2)]
+    for k, o in outs:
+        srv.submit_image(k, imgs[k], masks[k], 0.2, o)
+    ask(2, outs)
+    for disks in ([(330, 149, 2)], [(64, 63, 3)], [(7, 5, 0)], [(500, 500, 4)], [(0, 0, 1), (63, 64, 2)]):
+        outs = []
+        for k in range(2):
+            h, w = masks[k].shape
+            yy, xx = np.mgrid[:h, :w]
+            for x, y, r in disks:
+                masks[k][(xx - x) ** 2 + (yy - y) ** 2 <= r * r] = 1
+            outs.append((k, torch.empty((h, w))))
+            srv.submit_edit(k, disks, outs[-1][1])
+        ask(2, outs)
+    srv.close()
+    c.close()
