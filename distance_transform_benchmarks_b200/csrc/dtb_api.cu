@@ -796,6 +796,14 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
   }
 
   ctx->last_hdr = reinterpret_cast<QueueHdr*>(dbase + L.o_hdr);
+  // The status follows the work on its stream into pinned memory, so a synchronous call waits for the GPU once (a
+  // separate read after the wait cost 18 us of the 83 of a 97x61 call).
+  if (!ctx->hhdr && cudaHostAlloc((void**)&ctx->hhdr, sizeof(QueueHdr), cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->hhdr = nullptr;
+    return fail(ctx, DTB_ERR_OUT_OF_MEMORY, "cudaHostAlloc of the status header failed");
+  }
+  DTB_CUDA(ctx, cudaMemcpyAsync(ctx->hhdr, ctx->last_hdr, sizeof(QueueHdr), cudaMemcpyDeviceToHost, stream));
   ctx->last_stream = stream;
   ctx->stats = dtb_stats{};
   ctx->stats.tiles = total;
@@ -819,6 +827,10 @@ void tuning_to_abi(dtb_context ctx, const LaunchTuning& lt, dtb_tuning* t) {
 dtb_status read_device_status(dtb_context ctx, const QueueHdr* hdr_dev, dtb_stats* st) {
   QueueHdr h;
   DTB_CUDA(ctx, cudaMemcpy(&h, hdr_dev, sizeof(QueueHdr), cudaMemcpyDeviceToHost));
+  return status_of(ctx, h, st);
+}
+
+dtb_status status_of(dtb_context ctx, const QueueHdr& h, dtb_stats* st) {
   st->tile_visits = h.progress.v;
   st->phases = h.phases.v;
   st->activations = h.activations.v;
@@ -977,6 +989,7 @@ DTB_API void dtb_context_destroy(dtb_context ctx) {
   if (ctx->dscratch) cudaFree(ctx->dscratch);
   if (ctx->dround_counts) cudaFree(ctx->dround_counts);
   if (ctx->hrounds) cudaFreeHost(ctx->hrounds);
+  if (ctx->hhdr) cudaFreeHost(ctx->hhdr);
   for (int i = 0; i < 2; ++i) {
     if (ctx->hpin[i]) cudaFreeHost(ctx->hpin[i]);
     if (ctx->hpin_ev[i]) cudaEventDestroy(ctx->hpin_ev[i]);
@@ -1051,7 +1064,9 @@ DTB_API dtb_status dtb_sync(dtb_context ctx, void* stream) {
   }
   if (!ctx->async_pending) return DTB_OK;
   ctx->async_pending = false;
-  const dtb_status s = read_device_status(ctx, ctx->last_hdr, &ctx->stats);
+  // The call's header came back on its own stream (run_jobs); another stream's synchronisation says nothing about it.
+  const dtb_status s = st == ctx->last_stream ? status_of(ctx, *ctx->hhdr, &ctx->stats)
+                                              : read_device_status(ctx, ctx->last_hdr, &ctx->stats);
   if (ctx->timed) {
     float ms = 0.0f;
     DTB_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));

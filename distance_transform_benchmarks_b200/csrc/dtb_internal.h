@@ -144,6 +144,7 @@ struct dtb_context_s {
   dtb_stats stats{};
   // Asynchronous bookkeeping: header of the last enqueued run and the stream it ran on.
   dtb::QueueHdr* last_hdr = nullptr;
+  dtb::QueueHdr* hhdr = nullptr;  // pinned copy of it, written on that stream
   cudaStream_t last_stream = nullptr;
   bool async_pending = false;
   cudaEvent_t ev[2] = {nullptr, nullptr};  // DTB_FLAG_TIMING: around the tile kernel
@@ -277,6 +278,8 @@ bool valid_policy(int buckets, float bucket_tiles);
 // Workload key of the autotuner cache: image count and tile count, each rounded to a power of two.
 uint64_t tuning_key(int n, uint32_t total);
 dtb_status read_device_status(dtb_context ctx, const QueueHdr* hdr, dtb_stats* stats);
+// Counters and status of a run from its queue header.
+dtb_status status_of(dtb_context ctx, const QueueHdr& h, dtb_stats* stats);
 // Autotuner cache file of the context (ctx->tune_cache_path): load this GPU's entries into ctx->tuned; write
 // one entry.  The caller holds ctx->mu.
 dtb_status load_tuning_cache(dtb_context ctx);
