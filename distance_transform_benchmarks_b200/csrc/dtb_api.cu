@@ -88,12 +88,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
       sm.keep = POP_NONE;
     }
     prev = t;
-    uint32_t old = 0;
-    if (lane == 0) {
-      old = atomicXor(&states[t], ST_PENDING | ST_RUNNING);
-      if (q.keys) q.keys[t] = KEY_NONE;  // activations from here on belong to the next queue entry
-    }
-    old = __shfl_sync(~0u, old, 0);
+    const uint32_t old = sch.claim(t);
     const uint32_t img = old >> ST_IMG_SHIFT;
     if constexpr (MODE == MODE_NS) {
       const ImgDesc dd = descs[img];
@@ -131,12 +126,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
   while (cur != POP_NONE) {
     uint32_t nxt = queue_try_pop(q);
     if (nxt != POP_NONE) stage_ahead(descs, tmaps, states, nxt, sm.box[k ^ 1u], &sm.bar[k ^ 1u]);
-    uint32_t old = 0;
-    if (lane == 0) {
-      old = atomicXor(&states[cur], ST_PENDING | ST_RUNNING);
-      if (q.keys) q.keys[cur] = KEY_NONE;  // activations from here on belong to the next queue entry
-    }
-    old = __shfl_sync(~0u, old, 0);
+    const uint32_t old = sch.claim(cur);
     const uint32_t img = old >> ST_IMG_SHIFT;
     const ImgDesc dd = descs[img];
     const VisitBufs vb{sm.box[k], sm.Wh, sm.Wv, sm.E, &sm.bar[k], &sm.mbar, 1u << k, 4u, &pbits};

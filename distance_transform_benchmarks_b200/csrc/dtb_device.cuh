@@ -377,28 +377,28 @@ __device__ __forceinline__ uint32_t queue_pop(const Queue& q) {
   PopWatch w{globaltimer(), 0u};
   if (lane == 0) w.seen = ld_volatile(&q.hdr->progress.v);
   for (;;) {
-    uint32_t base = 0, m = 0;
+    uint32_t base = 0, b = 0;
     if (q.nb_mask) {
-      if (lane == 0) base = ld_volatile(&q.hdr->base.v);
-      base = __shfl_sync(~0u, base, 0);
-      const uint32_t bl = (base + (uint32_t)lane) & q.nb_mask;
+      // Lane l reads bucket l; the hint and all buckets in one trip.
+      base = ld_volatile(&q.hdr->base.v);
       bool avail = false;
       if ((uint32_t)lane <= q.nb_mask)
-        avail = (int32_t)(ld_volatile(&q.hdr->tails[bl].v) - ld_volatile(&q.hdr->heads[bl].v)) > 0;
-      m = __ballot_sync(~0u, avail);
+        avail = (int32_t)(ld_volatile(&q.hdr->tails[lane].v) - ld_volatile(&q.hdr->heads[lane].v)) > 0;
+      const uint32_t m = __ballot_sync(~0u, avail);
+      const uint32_t b0 = base & q.nb_mask;
+      b = b0;
+      if (m) {
+        const uint32_t up = m >> b0;  // buckets b0, b0 + 1, .. first, then the ones that wrapped
+        const uint32_t f = up ? (uint32_t)__ffs(up) - 1u : (uint32_t)__ffs(m) - 1u + q.nb_mask + 1u - b0;
+        if (f > 0 && lane == 0) atomicCAS(&q.hdr->base.v, base, base + f);  // the lower buckets are empty: move the hint up
+        b = (b0 + f) & q.nb_mask;
+      }
     }
     uint32_t res = POP_NONE;
     if (lane == 0) {
-      uint32_t b = base & q.nb_mask;
-      if (m) {
-        const uint32_t f = (uint32_t)(__ffs(m) - 1);
-        if (f > 0) atomicCAS(&q.hdr->base.v, base, base + f);  // the lower buckets are empty: move the hint up
-        b = (base + f) & q.nb_mask;
-      }
       const uint32_t h = atomicAdd(&q.hdr->heads[b].v, 1u);
-      // No fence and no checks between the ticket and the slot: with work queued the item is usually in the
-      // slot already, and the end of the queue (done, an error, nothing pending) is noticed by slot_take's
-      // periodic checks within POLL_CHECK_NS even when the ticket came after signal_done_warp read the heads.
+      // No fence and no checks between the ticket and the slot: with work queued the item is usually in the slot
+      // already, and the end of the queue (an error, nothing pending) is noticed by slot_take's periodic checks.
       res = slot_take(q, b, h, w);
     }
     res = __shfl_sync(~0u, res, 0);

@@ -39,69 +39,65 @@ struct QueueSched {
   // visits it next, which saves the ring's push and pop (two to five L2 round trips) and reuses the halo just
   // written.  It stays counted in `pending` like a queued tile.  nullptr: every tile goes through the ring.
   uint32_t* keep_out = nullptr;
+  // Start of a visit (whole warp): PENDING -> RUNNING; returns the state before.  Activations from here on belong to
+  // the next queue entry.  `pending` takes as many tokens as the visit may activate neighbours, without waiting.
+  static constexpr uint32_t TOKENS = 8;
+  __device__ __forceinline__ uint32_t claim(uint32_t tile) const {
+    uint32_t old = 0;
+    if ((threadIdx.x & 31) == 0) {
+      old = atomicXor(&states[tile], ST_PENDING | ST_RUNNING);
+      if (q.keys) q.keys[tile] = KEY_NONE;
+      atomicAdd(&q.hdr->pending.v, TOKENS);
+    }
+    return __shfl_sync(~0u, old, 0);
+  }
   // Warp-level end of a visit.  Lanes with `want` ask for a re-run of neighbour `item`, bringing activation
   // value `key` (distance units; bucket width 1 / inv_width): idle -> queued; running -> running with a re-run
   // requested; queued -> unchanged.  Lane 31 clears RUNNING of the own tile (and sets / clears the xor_bits);
-  // a re-run requested meanwhile re-queues it at the smallest value its activators left in keys[].  `pending`
-  // moves by (pushes - 1) in one atomic performed before any push is visible; the visit that brings it to 0
-  // ends the queue.
-  // The own-tile update comes first and, when it sets VISITED, is fenced before the activations: a woken
-  // neighbour takes this tile's distances as halo only if it sees VISITED, and otherwise reads v in their
-  // place.  Seeing the activation without the bit would consume the wake-up without the new distances.
+  // a re-run requested meanwhile re-queues it at the smallest value its activators left in keys[].
+  // The tokens taken by claim() cover the pushes, so `pending` counts an item before it can be popped, and what is left
+  // goes back without waiting; waiting workers look at `pending` themselves.  (A count before the pushes, its fence and
+  // its result cost each visit three L2 round trips of 17.)
+  // On a first visit the own-tile update is fenced before the activations: a woken neighbour takes this tile's
+  // distances as halo only if it sees VISITED, and otherwise reads v in their place.  Seeing the activation without
+  // the bit would consume the wake-up without the new distances.  Otherwise the two are in flight together.
   __device__ __forceinline__ void complete(uint32_t tile, uint32_t xor_bits, bool want, uint32_t want_item,
                                            float key = 0.0f, float inv_width = 0.0f) const {
     const int lane = threadIdx.x & 31;
-    bool push = false;
-    uint32_t item = 0;
-    float pkey = key;
-    if (lane == 31) {
-      const uint32_t old = atomicXor(&states[tile], xor_bits | ST_RUNNING);
-      push = (old & ST_PENDING) != 0u;
-      item = tile;
-      if (push && q.keys) {
-        const uint32_t kb = ld_volatile(&q.keys[tile]);
-        pkey = kb == KEY_NONE ? 0.0f : __uint_as_float(kb);
-      }
-      if (xor_bits & ST_VISITED) fence_acq_rel();
+    const uint32_t base = q.nb_mask ? ld_volatile(&q.hdr->base.v) : 0u;
+    uint32_t own = 0, other = 0;
+    if (lane == 31) own = atomicXor(&states[tile], xor_bits | ST_RUNNING);
+    if (xor_bits & ST_VISITED) {
+      fence_acq_rel();
+      __syncwarp();
     }
-    __syncwarp();
+    if (want && want_item >= q.total_tiles) {
+      set_error(q, DERR_BAD_TILE, want_item);
+      want = false;
+    }
     if (want) {
-      if (want_item >= q.total_tiles) {
-        set_error(q, DERR_BAD_TILE, want_item);
-      } else {
-        if (q.keys) {
-          const uint32_t prev = atomicMin(&q.keys[want_item], __float_as_uint(key));
-          pkey = fminf(key, __uint_as_float(prev == KEY_NONE ? __float_as_uint(key) : prev));
-        }
-        const uint32_t old = atomicOr(&states[want_item], ST_PENDING);
-        push = !(old & (ST_PENDING | ST_RUNNING));
-        item = want_item;
-      }
+      if (q.keys) atomicMin(&q.keys[want_item], __float_as_uint(key));
+      other = atomicOr(&states[want_item], ST_PENDING);
+    }
+    const bool again = lane == 31 && (own & ST_PENDING) != 0u;
+    const bool push = again || (want && !(other & (ST_PENDING | ST_RUNNING)));
+    const uint32_t item = lane == 31 ? tile : want_item;
+    float pkey = key;
+    if (again && q.keys && !keep_out) {
+      const uint32_t kb = ld_volatile(&q.keys[tile]);
+      pkey = kb == KEY_NONE ? 0.0f : __uint_as_float(kb);
     }
     const uint32_t m = __ballot_sync(~0u, push);
-    const uint32_t k = __popc(m);
-    uint32_t last = 0;
-    if (lane == 0) {
-      if (k == 0) {
-        last = atomicSub(&q.hdr->pending.v, 1u) == 1u ? 1u : 0u;
-      } else if (k > 1) {
-        atomicAdd(&q.hdr->pending.v, k - 1u);
-      }
-      fence_acq_rel();
-    }
-    __syncwarp();
-    uint32_t base = 0;
-    if (q.nb_mask) base = ld_volatile(&q.hdr->base.v);
     const uint32_t b = push ? bucket_at(q, pkey, inv_width, base) : 0u;
     int kept = -1;
-    if (keep_out) {
-      // The own tile first (lane 31 re-queues it when its halo dropped during the visit): its re-run reuses the
-      // weights and distances in this warp's shared memory.  Else the smallest activation value.
-      const bool elig = push && b == (base & q.nb_mask);
-      const uint32_t em = __ballot_sync(~0u, elig);
-      if (__ballot_sync(~0u, push) >> 31) {  // the own tile, whatever its bucket: its re-run is cheap
+    if (keep_out && m) {
+      // The own tile first, whatever its bucket (lane 31 re-queues it when its halo dropped during the visit): its
+      // re-run reuses the weights and distances in this warp's shared memory.  Else the smallest activation value
+      // in the lowest bucket.
+      if (m >> 31) {
         kept = 31;
       } else {
+        const bool elig = push && b == (base & q.nb_mask);
         const uint32_t kmin = __reduce_min_sync(~0u, elig ? __float_as_uint(pkey) : 0xFFFFFFFFu);
         const uint32_t cand = __ballot_sync(~0u, elig && __float_as_uint(pkey) == kmin);
         if (cand) kept = __ffs(cand) - 1;
@@ -110,7 +106,7 @@ struct QueueSched {
     }
     if (push && lane != kept) slot_write(q, b, atomicAdd(&q.hdr->tails[b].v, 1u), item);
     __syncwarp();
-    if (__shfl_sync(~0u, last, 0)) signal_done_warp(q);
+    if (lane == 0) atomicSub(&q.hdr->pending.v, TOKENS + 1u - __popc(m));
   }
 };
 
@@ -189,6 +185,15 @@ __device__ __forceinline__ bool mask_row_any(const ImgDesc& dd, int x0, int y, i
   bool nz = false;
   for (int c = 0; c < vw; ++c) nz |= row[c] != 0;
   return nz;
+}
+
+// 1 / bucket width of an image: one tile-width of path cost in bucket_tiles parts, 32 x the mean internal edge weight
+// seen so far by first visits.
+__device__ __forceinline__ float bucket_inv_width(const Queue& q, uint32_t img) {
+  if (!q.wacc) return 0.0f;
+  const volatile float* wa = q.wacc + 2 * img;
+  const float s = wa[0], c = wa[1], w = q.bucket_tiles * (float)TILE;
+  return (c > 0.0f && s > 0.0f) ? c / (w * s) : 1.0f / w;
 }
 
 // Waits for the TMA transactions on `bar`; its phase parity is bit `pmask` of `pbits`.  Bounded: after
@@ -461,22 +466,15 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   }
   __syncwarp();
 
-  // Bucket width of this image: one tile-width of path cost, 32 x the mean internal edge weight seen so far by
-  // first visits (each first visit adds its column edges).
-  float inv_width = 0.0f;
-  if (sch.q.wacc) {
+  // The image's mean edge weight, for its bucket width: each first visit adds its column edges.
+  if (sch.q.wacc && first) {
     float* wa = sch.q.wacc + 2 * img_idx;
-    if (first) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(~0u, wsum, o);
-      if (lane == 0 && vh > 1) {
-        atomicAdd(&wa[0], wsum);
-        atomicAdd(&wa[1], (float)(vw * (vh - 1)));
-      }
+    for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(~0u, wsum, o);
+    if (lane == 0 && vh > 1) {
+      atomicAdd(&wa[0], wsum);
+      atomicAdd(&wa[1], (float)(vw * (vh - 1)));
     }
-    const float s_ = *(volatile float*)&wa[0], c_ = *(volatile float*)&wa[1];
-    const float bt = sch.q.bucket_tiles;
-    inv_width = (c_ > 0.0f && s_ > 0.0f) ? c_ / (bt * (float)TILE * s_) : 1.0f / (bt * (float)TILE);
   }
 
   // The tile buffer B overlays the image box, which is no longer needed.  Relax the halo edges in it: top and bottom
@@ -562,6 +560,9 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     act &= nexist;
     act_key = __uint_as_float(lane == 0 ? kl : lane == 1 ? kr : lane == 2 ? kt : kbm);
   }
+
+  // The bucket width, read here so that the write-back covers the trip.
+  const float inv_width = bucket_inv_width(sch.q, img_idx);
 
   // Write back (column layout: each row is one coalesced 128-byte store).
   if (any || first) {
@@ -935,22 +936,15 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
     __syncwarp();
   }
 
-  // Bucket width of this image (priority queue): half a tile-width of the mean axial edge cost
-  // l_eucl + l_grad * |dI| seen by first visits (vertical edges of the tile).
-  float inv_width = 0.0f;
-  if (sch.q.wacc) {
+  // The image's mean axial edge cost, for its bucket width: each first visit adds its vertical edges.
+  if (sch.q.wacc && first) {
     float* wa = sch.q.wacc + 2 * (old_state >> ST_IMG_SHIFT);
-    if (first) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(~0u, wsum, o);
-      if (lane == 0 && vh > 1) {
-        atomicAdd(&wa[0], wsum);
-        atomicAdd(&wa[1], (float)(vw * (vh - 1)));
-      }
+    for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(~0u, wsum, o);
+    if (lane == 0 && vh > 1) {
+      atomicAdd(&wa[0], wsum);
+      atomicAdd(&wa[1], (float)(vw * (vh - 1)));
     }
-    const float s_ = *(volatile float*)&wa[0], c_ = *(volatile float*)&wa[1];
-    const float bt = sch.q.bucket_tiles;
-    inv_width = (c_ > 0.0f && s_ > 0.0f) ? c_ / (bt * (float)TILE * s_) : 1.0f / (bt * (float)TILE);
   }
 
   bool any = ref_halo_relax<FMA>(re, T, sm.E, h, vw, vh);
@@ -981,6 +975,7 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
     act &= nexist;
   }
 
+  const float inv_width = bucket_inv_width(sch.q, old_state >> ST_IMG_SHIFT);
   if (any || first || seed) {
     if (lane < vw) {
       uint8_t* wb = dist_base(dd, y0, x0 + lane, nph);

@@ -91,15 +91,12 @@ __global__ void __launch_bounds__(NOALLOC_WPC * 32, NOALLOC_MINB) noalloc_persis
   const Queue q = na_queue(max_visits, tiles);
   uint32_t* states = na_states();
   const QueueSched sch{q, states};
-  const int lane = threadIdx.x & 31;
   uint32_t parity = 0;
   WarpStats ws;
   for (;;) {
     const uint32_t t = queue_pop(q);  // one FIFO ring: this scratch holds no priority buckets
     if (t == POP_NONE) break;
-    uint32_t old = 0;
-    if (lane == 0) old = atomicXor(&states[t], ST_PENDING | ST_RUNNING);
-    old = __shfl_sync(~0u, old, 0);
+    const uint32_t old = sch.claim(t);
     const ImgDesc dd = *na_desc();
     visit_tile<MODE_NS>(dd, na_tmaps(), 0u, t, old, sm, parity, sch, ws);
   }
