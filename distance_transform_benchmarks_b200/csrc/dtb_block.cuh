@@ -260,6 +260,99 @@ __device__ __forceinline__ void block_store_tile(const ImgDesc& dd, const BlockP
   }
 }
 
+// Writes the lines of the warp's tile that lie on the block's border (`outer`: left, right, top, bottom) to memory.
+__device__ __forceinline__ void block_store_border(const ImgDesc& dd, const BlockPlace& p, uint32_t outer, const float* B, int stride) {
+  const int lane = threadIdx.x & 31;
+  if (lane < p.vh) {
+    float* row = dist_row(dd, p.y0 + lane) + p.x0;
+    if (outer & 1u) row[0] = B[lane * stride];
+    if (outer & 2u) row[TILE - 1] = B[lane * stride + TILE - 1];
+  }
+  if (lane < p.vw) {
+    if (outer & 4u) dist_row(dd, p.y0)[p.x0 + lane] = B[lane];
+    if (outer & 8u) dist_row(dd, p.y0 + TILE - 1)[p.x0 + lane] = B[(TILE - 1) * stride + lane];
+  }
+}
+
+// Fills the warp's tile (distances, weights) from the boxes stage_tile has issued; whether a seed lowered a pixel.
+__device__ __forceinline__ bool block_fill_ns(const ImgDesc& dd, const BlockPlace& p, BlockTile& t, bool first, bool seed,
+                                              uint32_t blk, uint32_t& flags, const Queue& q) {
+  const int lane = threadIdx.x & 31;
+  const float INF = f_inf();
+  float d[TILE];
+  if (!first) {
+    const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
+    const int64_t pitch = dd.dist_pitch;
+#pragma unroll
+    for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : INF;
+  }
+  const bool staged = tma_wait(&t.bar, flags, 1u, q, blk);
+  uint32_t seeds = 0;  // this lane's column of the mask tile
+  if (seed && staged) {
+    const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.Wv);
+#pragma unroll 4
+    for (int y = 0; y < TILE; ++y) seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
+  }
+  __syncwarp();
+  tile_weights(dd.g2, dd.channels == 3, p.vw, p.vh, t.img, t.Wh, t.Wv, t.E);
+  __syncwarp();
+  float* pb = reinterpret_cast<float*>(t.img) + lane;
+  if (first) {
+    const float v = dd.v;
+#pragma unroll 4
+    for (int y = 0; y < TILE; ++y)
+      pb[y * W_STRIDE] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
+    return __any_sync(~0u, seeds != 0u);
+  }
+  bool low = false;  // a seed on a pixel that is 0 already asks for nothing
+#pragma unroll
+  for (int y = 0; y < TILE; ++y) {
+    const bool s = ((seeds >> y) & 1u) != 0u;
+    low |= s && d[y] > 0.0f;
+    pb[y * W_STRIDE] = s ? 0.0f : d[y];
+  }
+  return __any_sync(~0u, low);
+}
+
+template <bool FMA>
+__device__ __forceinline__ bool block_fill_ref(const RefEdge<FMA>& re, const ImgDesc& dd, const BlockPlace& p, RefTile& t, bool first,
+                                               bool seed, uint32_t blk, uint32_t& flags, const Queue& q) {
+  const int lane = threadIdx.x & 31;
+  const float INF = f_inf();
+  float* T = reinterpret_cast<float*>(t.img);
+  float d[TILE];
+  if (!first) {
+    const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
+    const int64_t pitch = dd.dist_pitch;
+#pragma unroll
+    for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : INF;
+  }
+  const bool staged = tma_wait(&t.bar, flags, 1u, q, blk);
+  uint32_t seeds = 0;  // this lane's column of the mask tile
+  if (seed && staged) {
+    const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.V);
+#pragma unroll 4
+    for (int y = 0; y < TILE; ++y) seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
+  }
+  __syncwarp();
+  ref_tile_weights<FMA>(re, p.vw, p.vh, t);
+  __syncwarp();
+  if (first) {
+    const float v = dd.v;
+#pragma unroll 4
+    for (int y = 0; y < TILE; ++y) T[y * RS + lane] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
+    return __any_sync(~0u, seeds != 0u);
+  }
+  bool low = false;
+#pragma unroll
+  for (int y = 0; y < TILE; ++y) {
+    const bool s = ((seeds >> y) & 1u) != 0u;
+    low |= s && d[y] > 0.0f;
+    T[y * RS + lane] = s ? 0.0f : d[y];
+  }
+  return __any_sync(~0u, low);
+}
+
 // A warp's flags: bit 0 the phase parity of its mbarrier; its tile of the block visited last differs from memory.
 constexpr uint32_t BLOCK_UNSAVED = 2u;
 
@@ -271,7 +364,8 @@ constexpr uint32_t BLOCK_UNSAVED = 2u;
 // only after an iteration in which no tile changed.  Only the lines on the block's border are written to memory; the
 // tiles stay in shared memory and are written when the CTA turns to another block (BLOCK_UNSAVED) or ends.
 __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem<MODE_NS>& sm,
-                                               uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q) {
+                                               uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, float (&wh)[TILE],
+                                               float (&wv)[TILE], int& loaded) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float INF = f_inf();
   const ImgDesc& dd = sm.ctl.desc;
@@ -304,49 +398,12 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
       t.H[E_TOP + lane] = top;
       t.H[E_BOTTOM + lane] = bot;
     }
-    if (exists && !rerun) {
-      float d[TILE];
-      if (!first) {
-        const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
-        const int64_t pitch = dd.dist_pitch;
-#pragma unroll
-        for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : INF;
-      }
-      const bool staged = tma_wait(&t.bar, flags, 1u, q, blk);
-      uint32_t seeds = 0;  // this lane's column of the mask tile
-      if (seed && staged) {
-        const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.Wv);
-#pragma unroll 4
-        for (int y = 0; y < TILE; ++y)
-          seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
-        todo = __any_sync(~0u, seeds != 0u);
-        changed = todo;
-      }
-      __syncwarp();
-      tile_weights(dd.g2, dd.channels == 3, p.vw, p.vh, t.img, t.Wh, t.Wv, t.E);
-      __syncwarp();
-      float* pb = B + lane;
-      if (first) {
-        const float v = dd.v;
-#pragma unroll 4
-        for (int y = 0; y < TILE; ++y)
-          pb[y * W_STRIDE] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
-      } else {
-        bool low = false;  // a seed on a pixel that is 0 already asks for nothing
-#pragma unroll
-        for (int y = 0; y < TILE; ++y) {
-          const bool s = ((seeds >> y) & 1u) != 0u;
-          low |= s && d[y] > 0.0f;
-          pb[y * W_STRIDE] = s ? 0.0f : d[y];
-        }
-        todo = changed = __any_sync(~0u, low);
-      }
-      if (first) flags |= BLOCK_UNSAVED;
-    }
+    if (exists && !rerun) todo = changed = block_fill_ns(dd, p, t, first, seed, blk, flags, q);
+    if (first) flags |= BLOCK_UNSAVED;
+    if (!rerun) loaded = -1;
   }
   uint32_t nph = 0;
-  int loaded = -1;  // layout of the weights in registers
-  float d[TILE], wh[TILE], wv[TILE];
+  float d[TILE];
   __syncthreads();  // every tile of the block is in place
   for (uint32_t it = 0;; ++it) {
     bool layout_a = true;
@@ -404,6 +461,9 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
       } while (todo && ++r < BLOCK_ROUNDS);
       changed = true;
       store_skew(B + lane * W_STRIDE, off, d);
+      // The border lines go out at once: the checks that end the visit cover their way to L2.
+      __syncwarp();
+      block_store_border(dd, block_place(dd, blk), sides >> 8, B, W_STRIDE);
     }
     if (it >= (uint32_t)PHASE_LIMIT) {
       if (threadIdx.x == 0) set_error(q, DERR_PHASE_LIMIT, blk);
@@ -412,23 +472,13 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
     __syncthreads();
   }
 
-  // What the block's border can bring to its neighbours, and the border lines to memory.
-  const bool first = sm.ctl.first != 0u;
+  // What the block's border can bring to its neighbours, and the border lines that were never written.
   const uint32_t outer = (sides >> 8) & 15u;
   if (changed) flags |= BLOCK_UNSAVED;
-  if (outer && (changed || first)) {
-    const BlockPlace p = block_place(dd, blk);
+  if (outer && (changed || sm.ctl.first)) {
+    if (!nph) block_store_border(dd, block_place(dd, blk), outer, B, W_STRIDE);
     const float* E = t.E;
     const float bl = B[lane * W_STRIDE], br = B[lane * W_STRIDE + TILE - 1], bt = B[lane], bb = B[(TILE - 1) * W_STRIDE + lane];
-    if (lane < p.vh) {
-      float* row = dist_row(dd, p.y0 + lane) + p.x0;
-      if (outer & 1u) row[0] = bl;
-      if (outer & 2u) row[TILE - 1] = br;
-    }
-    if (lane < p.vw) {
-      if (outer & 4u) dist_row(dd, p.y0)[p.x0 + lane] = bt;
-      if (outer & 8u) dist_row(dd, p.y0 + TILE - 1)[p.x0 + lane] = bb;
-    }
     const float vl = __fadd_rn(bl, E[E_LEFT + lane]), vr = __fadd_rn(br, E[E_RIGHT + lane]);
     const float vt = __fadd_rn(bt, E[E_TOP + lane]), vbm = __fadd_rn(bb, E[E_BOTTOM + lane]);
     const uint32_t kl = __reduce_min_sync(~0u, vl < t.H[E_LEFT + lane] ? __float_as_uint(vl) : KEY_NONE);
@@ -462,6 +512,8 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
   const bool first = sm.ctl.first != 0u;
   const BlockPlace p = block_place(dd, blk);
   const bool exists = (p.sides >> 12) != 0u;
+  // The lines that neighbouring blocks read: the sides with one beyond, and (corners) the whole left and top border.
+  const uint32_t outer = ((p.sides >> 8) & 15u) | (wx == 0 ? 1u : 0u) | (wy == 0 ? 4u : 0u);
   bool todo = false, changed = false;
   // Side k of the tile: the neighbouring tile in this block, or the side of the block it lies beyond.
   auto in_block = [&](int k) {
@@ -492,43 +544,8 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
       t.H[E_BOTTOM + lane] = hb;
       if (lane < 4) t.H[4 * TILE + lane] = hc;
     }
-    if (exists && !rerun) {
-      float d[TILE];
-      if (!first) {
-        const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
-        const int64_t pitch = dd.dist_pitch;
-#pragma unroll
-        for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : INF;
-      }
-      const bool staged = tma_wait(&t.bar, flags, 1u, q, blk);
-      uint32_t seeds = 0;  // this lane's column of the mask tile
-      if (seed && staged) {
-        const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.V);
-#pragma unroll 4
-        for (int y = 0; y < TILE; ++y)
-          seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
-        todo = __any_sync(~0u, seeds != 0u);
-        changed = todo;
-      }
-      __syncwarp();
-      ref_tile_weights<FMA>(re, p.vw, p.vh, t);
-      __syncwarp();
-      if (first) {
-        const float v = dd.v;
-#pragma unroll 4
-        for (int y = 0; y < TILE; ++y) T[y * RS + lane] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
-        flags |= BLOCK_UNSAVED;
-      } else {
-        bool low = false;
-#pragma unroll
-        for (int y = 0; y < TILE; ++y) {
-          const bool s = ((seeds >> y) & 1u) != 0u;
-          low |= s && d[y] > 0.0f;
-          T[y * RS + lane] = s ? 0.0f : d[y];
-        }
-        todo = changed = __any_sync(~0u, low);
-      }
-    }
+    if (exists && !rerun) todo = changed = block_fill_ref<FMA>(re, dd, p, t, first, seed, blk, flags, q);
+    if (first) flags |= BLOCK_UNSAVED;
   }
   uint32_t nph = 0;
   bool col = true;
@@ -556,6 +573,7 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
       changed = true;
       bool fell = false;
       todo = ref_solve<FMA>(re, t, col, BLOCK_PHASES, nph, fell);
+      block_store_border(dd, p, outer, T, RS);  // at once, as in block_visit_ns
     }
     if (it >= (uint32_t)PHASE_LIMIT) {
       if (threadIdx.x == 0) set_error(q, DERR_PHASE_LIMIT, blk);
@@ -567,16 +585,7 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
   // What the block's border can bring to its neighbours, and the border lines to memory.
   if (changed) flags |= BLOCK_UNSAVED;
   if (exists && (changed || first)) {
-    const uint32_t outer = (p.sides >> 8) & 15u;
-    if (lane < p.vh) {
-      float* row = dist_row(dd, p.y0 + lane) + p.x0;
-      if (wx == 0) row[0] = T[lane * RS];
-      if (outer & 2u) row[TILE - 1] = T[lane * RS + TILE - 1];
-    }
-    if (lane < p.vw) {
-      if (wy == 0) dist_row(dd, p.y0)[p.x0 + lane] = T[lane];
-      if (outer & 8u) dist_row(dd, p.y0 + TILE - 1)[p.x0 + lane] = T[(TILE - 1) * RS + lane];
-    }
+    if (!nph) block_store_border(dd, p, outer, T, RS);
     // Neighbours in the block have an INF halo in H: every finite value would beat it, so they are masked out.
     const RefHalo h{t.H[E_LEFT + lane], t.H[E_RIGHT + lane], t.H[E_TOP + lane],  t.H[E_BOTTOM + lane],
                     t.H[4 * TILE],      t.H[4 * TILE + 1],   t.H[4 * TILE + 2], t.H[4 * TILE + 3]};
@@ -640,6 +649,39 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
     if (lane == 0) atomicSub(&a.hdr->pending.v, (uint32_t)count - seeded);
   }
   uint32_t flags = 0, prev = POP_NONE;
+  float wh[TILE], wv[TILE];  // ns-mode: the tile's weights, in the layout `loaded`
+  int loaded = -1;
+  // The first block without seeds is filled before anything activates it, so that its first visit finds it in place: with
+  // one block per CTA that takes 8,000 (gray) to 12,000 (rgb8) cycles off every step of the front into new blocks.
+  {
+    int i = 0;
+    while (i < count && ((sm.ctl.seeded[i >> 5] >> (i & 31)) & 1u)) ++i;
+    if (i < count) {
+      const uint32_t img = sm.ctl.owned_img[i], blk = first + (uint32_t)i * step;
+      const ImgDesc& src = descs[img];
+      if (!src.warm) {
+        if (threadIdx.x < sizeof(ImgDesc) / 4) reinterpret_cast<uint32_t*>(&sm.ctl.desc)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&src)[threadIdx.x];
+        __syncthreads();
+        const ImgDesc& dd = sm.ctl.desc;
+        const BlockPlace p = block_place(dd, blk);
+        auto& t = sm.tile[warp];
+        if (p.vw > 0 && p.vh > 0) {
+          if constexpr (MODE == MODE_NS) {
+            const VisitBufs vb{t.img, t.Wh, t.Wv, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
+            stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, dd.channels == 3, false, p.x0, p.y0);
+            block_fill_ns(dd, p, t, true, false, blk, flags, q);
+          } else {
+            const RefEdge<MODE == MODE_REF> re(dd.l_eucl, dd.l_grad);
+            const VisitBufs vb{t.img, t.V, t.V, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
+            stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, false, false, p.x0, p.y0);
+            block_fill_ref<MODE == MODE_REF>(re, dd, p, t, true, false, blk, flags, q);
+          }
+        }
+        prev = (uint32_t)i;
+        __syncthreads();  // ctl.desc is block_next's from here on
+      }
+    }
+  }
   for (;;) {
     if (warp == 0) block_next<BLOCK_SIDES<MODE>>(a, descs, sm.ctl, first, step, count, prev);
     __syncthreads();
@@ -653,7 +695,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
     }
     if (next == POP_NONE) break;
     if constexpr (MODE == MODE_NS)
-      block_visit_ns(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q);
+      block_visit_ns(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, wh, wv, loaded);
     else
       block_visit_ref<MODE == MODE_REF>(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q);
     prev = next;
