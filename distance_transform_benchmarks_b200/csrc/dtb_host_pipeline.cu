@@ -149,15 +149,22 @@ dtb_status run_host_pipeline(dtb_context ctx, std::vector<Job> jobs, const dtb_i
   ctx->pset_cur ^= 1;
 
   // ---- chunks of about host_chunk_px pixels, the first ones smaller (1/8, 1/4, 1/2) so that the first maps
-  //      start their way back early ----
+  //      start their way back early, and in a synchronous call the last ones half of what is left (down to 1/8), since
+  //      nothing overlaps the last chunk's run and copy out (64 images of 24 Mpx: 3.3 -> 3.0 ms; asynchronous calls
+  //      overlap the next one's and would lose 1 %) ----
   std::vector<int> cut{0};
-  uint64_t acc = 0, target = std::max<uint64_t>(ctx->host_chunk_px / 8, 1);
+  const uint64_t least = std::max<uint64_t>(ctx->host_chunk_px / 8, 1);
+  uint64_t left = 0, acc = 0, target = least;
+  for (int i = 0; i < n; ++i) left += (uint64_t)jobs[i].width * jobs[i].height;
   for (int i = 0; i < n; ++i) {
-    acc += (uint64_t)jobs[i].width * jobs[i].height;
+    const uint64_t px = (uint64_t)jobs[i].width * jobs[i].height;
+    acc += px;
+    left -= px;
     if (acc >= target && i + 1 < n) {
       cut.push_back(i + 1);
       acc = 0;
       target = std::min<uint64_t>(2 * target, ctx->host_chunk_px);
+      if (!(flags & DTB_FLAG_ASYNC)) target = std::min(target, std::max(least, left / 2));
     }
   }
   cut.push_back(n);
