@@ -244,8 +244,7 @@ DTB_API dtb_status dtb_plan_create(dtb_context ctx, int32_t n, const dtb_image* 
   p->L = layout_for(n, total, workers, false, NBUCKET_MAX);  // room for every queue policy of the autotuner
   p->L.blocks = count_blocks(p->jobs);
   p->key = tuning_key(n, total);
-  auto it = ctx->tuned.find(p->key);
-  p->tuning = it != ctx->tuned.end() ? it->second : ctx->tuning;
+  p->tuning = tuning_for(ctx, n, total);
   if (cudaSetDevice(ctx->device) != cudaSuccess) return bail(DTB_ERR_CUDA);
   cudaError_t e = cudaMalloc((void**)&p->dbase, p->L.bytes);
   if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaMalloc(plan scratch)"));

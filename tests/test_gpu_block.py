@@ -134,3 +134,26 @@ def test_wave_edits_through_either_kernel(tuned):
         ask(2, outs)
     srv.close()
     c.close()
+
+
+def test_large_batch_defaults_are_fixpoints():
+    """A plan above the size at which untuned batches change their launch shape and queue policy (96k tiles, 32 images):
+    every map passes the fixpoint check, and a call on the same images gives the same maps."""
+    specs = wl.config3_specs(9, 260, 512, 2048)
+    c = dtb.Context(0)
+    batch = [wl.make_image(s) for s in specs]
+    assert sum(-(-b[1].shape[0] // 32) * -(-b[1].shape[1] // 32) for b in batch) >= 96 * 1024
+    imgs, masks = [dtb.pitched_from(b[0]) for b in batch], [dtb.pitched_from(b[1]) for b in batch]
+    gam = [b[2] for b in batch]
+    dists = [dtb.pitched_empty(b[1].shape[0], b[1].shape[1], 1, torch.float32) for b in batch]
+    plan = dtb.BatchPlan(imgs, masks, gam, dists=dists, ctx=c)
+    plan.run()
+    assert plan.wait()["device_error"] == 0
+    first = [d.clone() for d in dists]
+    for k in range(len(batch)):
+        assert ns_fixpoint_violations(imgs[k], masks[k], gam[k], 1e10, dists[k])[:2] == (0, 0), k
+        dists[k].fill_(-1.0)
+    dtb.geodesic_distance_transform_batch(imgs, masks, gam, dists=dists, ctx=c)
+    assert all(torch.equal(a, b) for a, b in zip(first, dists))
+    plan.close()
+    c.close()
