@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
   WarpStats ws;
   uint32_t prev = POP_NONE;  // the tile this warp visited last
   for (;;) {
-    uint32_t t = sm.keep;
+    uint32_t t = uniform(sm.keep);
     __syncwarp();
     const bool again = t != POP_NONE && t == prev;  // kept its own tile: its weights and distances are in smem
     if (t == POP_NONE) {
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(WPC * 32)
   if (!__shfl_sync(~0u, run, 0)) return;
   warp_slot_init(sm);
   uint32_t parity = 0;
-  const uint32_t old = ld_volatile(&states[t]);
+  const uint32_t old = uniform(ld_volatile(&states[t]));
   const uint32_t img = old >> ST_IMG_SHIFT;
   const RoundSched sch{q, states, next_active, changed};
   const ImgDesc dd = descs[img];

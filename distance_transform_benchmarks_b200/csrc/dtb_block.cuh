@@ -231,7 +231,7 @@ struct BlockPlace {
   uint32_t sides;
 };
 __device__ __forceinline__ BlockPlace block_place(const ImgDesc& dd, uint32_t blk) {
-  const int warp = threadIdx.x >> 5, wx = warp % BLOCK_TX, wy = warp / BLOCK_TX;
+  const int warp = (int)uniform(threadIdx.x >> 5), wx = warp % BLOCK_TX, wy = warp / BLOCK_TX;
   const uint32_t local = blk - dd.block_base;
   BlockPlace p;
   p.x0 = (int)(local % (uint32_t)dd.blocks_x) * BLOCK_W + wx * TILE;
@@ -274,27 +274,29 @@ __device__ __forceinline__ void block_store_border(const ImgDesc& dd, const Bloc
   }
 }
 
-// Fills the warp's tile (distances, weights) from the boxes stage_tile has issued; whether a seed lowered a pixel.
+// The warp's tile from memory (lane = x).
+__device__ __forceinline__ void block_load_tile(const ImgDesc& dd, const BlockPlace& p, float (&d)[TILE]) {
+  const int lane = threadIdx.x & 31;
+  const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
+  const int64_t pitch = dd.dist_pitch;
+#pragma unroll
+  for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : f_inf();
+}
+
+// Fills the warp's tile (distances, weights) from its staged boxes and, unless `first`, its distances d; whether a seed
+// lowered a pixel.
 __device__ __forceinline__ bool block_fill_ns(const ImgDesc& dd, const BlockPlace& p, BlockTile& t, bool first, bool seed,
-                                              uint32_t blk, uint32_t& flags, const Queue& q) {
+                                              const float (&d)[TILE]) {
   const int lane = threadIdx.x & 31;
   const float INF = f_inf();
-  float d[TILE];
-  if (!first) {
-    const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
-    const int64_t pitch = dd.dist_pitch;
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : INF;
-  }
-  const bool staged = tma_wait(&t.bar, flags, 1u, q, blk);
   uint32_t seeds = 0;  // this lane's column of the mask tile
-  if (seed && staged) {
+  if (seed) {
     const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.Wv);
 #pragma unroll 4
     for (int y = 0; y < TILE; ++y) seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
   }
   __syncwarp();
-  tile_weights(dd.g2, dd.channels == 3, p.vw, p.vh, t.img, t.Wh, t.Wv, t.E);
+  tile_weights(dd.g2, uniform(dd.channels == 3), p.vw, p.vh, t.img, t.Wh, t.Wv, t.E);
   __syncwarp();
   float* pb = reinterpret_cast<float*>(t.img) + lane;
   if (first) {
@@ -316,20 +318,12 @@ __device__ __forceinline__ bool block_fill_ns(const ImgDesc& dd, const BlockPlac
 
 template <bool FMA>
 __device__ __forceinline__ bool block_fill_ref(const RefEdge<FMA>& re, const ImgDesc& dd, const BlockPlace& p, RefTile& t, bool first,
-                                               bool seed, uint32_t blk, uint32_t& flags, const Queue& q) {
+                                               bool seed, const float (&d)[TILE]) {
   const int lane = threadIdx.x & 31;
   const float INF = f_inf();
   float* T = reinterpret_cast<float*>(t.img);
-  float d[TILE];
-  if (!first) {
-    const uint8_t* lb = dist_base(dd, p.y0, p.x0 + lane, 0u);
-    const int64_t pitch = dd.dist_pitch;
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = (lane < p.vw && y < p.vh) ? ld_dist_at(lb, pitch, y) : INF;
-  }
-  const bool staged = tma_wait(&t.bar, flags, 1u, q, blk);
   uint32_t seeds = 0;  // this lane's column of the mask tile
-  if (seed && staged) {
+  if (seed) {
     const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.V);
 #pragma unroll 4
     for (int y = 0; y < TILE; ++y) seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
@@ -356,7 +350,7 @@ __device__ __forceinline__ bool block_fill_ref(const RefEdge<FMA>& re, const Img
 // A warp's flags: bit 0 the phase parity of its mbarrier; its tile of the block visited last differs from memory.
 constexpr uint32_t BLOCK_UNSAVED = 2u;
 
-// One visit of a block by its CTA (all warps; the barriers are CTA-wide).  Tile (wx, wy) of the block is warp
+// One visit of a block by its CTA (all warps; the barriers are CTA-wide); with `fill_only` it ends once the tiles are filled.  Tile (wx, wy) of the block is warp
 // wy * BLOCK_TX + wx's.  The tiles relax their halo edges from their neighbours in the block (shared memory) and, on
 // the block's border, from the halo read at the start; a tile whose border was lowered, or which had not converged,
 // runs up to BLOCK_ROUNDS rounds (skew_round); this repeats until no tile has anything to do.  A tile may read a
@@ -365,8 +359,8 @@ constexpr uint32_t BLOCK_UNSAVED = 2u;
 // tiles stay in shared memory and are written when the CTA turns to another block (BLOCK_UNSAVED) or ends.
 __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem<MODE_NS>& sm,
                                                uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, float (&wh)[TILE],
-                                               float (&wv)[TILE], int& loaded) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                                               float (&wv)[TILE], int& loaded, bool fill_only) {
+  const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
   const float INF = f_inf();
   const ImgDesc& dd = sm.ctl.desc;
   BlockTile& t = sm.tile[warp];
@@ -375,10 +369,10 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
   bool todo = false;     // the tile has rounds to run whatever its halo
   bool changed = false;  // a value of the tile fell in this visit
   {
-    const bool first = sm.ctl.first != 0u, seed = sm.ctl.seed != 0u, rerun = sm.ctl.rerun != 0u;
+    const bool first = uniform(sm.ctl.first != 0u), seed = uniform(sm.ctl.seed != 0u), rerun = uniform(sm.ctl.rerun != 0u);
     const BlockPlace p = block_place(dd, blk);
-    sides = p.sides;
-    const bool exists = p.vw > 0 && p.vh > 0;
+    sides = uniform(p.sides);
+    const bool exists = (sides & 0x1000u) != 0u;
     const VisitBufs vb{t.img, t.Wh, t.Wv, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
     if (exists && !rerun) stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, dd.channels == 3, seed, p.x0, p.y0);
     {
@@ -398,9 +392,17 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
       t.H[E_TOP + lane] = top;
       t.H[E_BOTTOM + lane] = bot;
     }
-    if (exists && !rerun) todo = changed = block_fill_ns(dd, p, t, first, seed, blk, flags, q);
-    if (first) flags |= BLOCK_UNSAVED;
+    const bool fill = exists && !rerun;
+    float td[TILE];
+    if (fill && !first) block_load_tile(dd, p, td);
+    tma_wait(&t.bar, flags, 1u, q, blk, fill);
+    if (uniform(fill)) todo = changed = block_fill_ns(dd, p, t, first, seed, td);
     if (!rerun) loaded = -1;
+    if (fill_only) {
+      __syncthreads();  // ctl is block_next's from here on
+      return;
+    }
+    if (first) flags |= BLOCK_UNSAVED;
   }
   uint32_t nph = 0;
   float d[TILE];
@@ -436,7 +438,7 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
       B[lane * W_STRIDE] = dl;
       B[lane * W_STRIDE + TILE - 1] = dr;
       todo |= __any_sync(~0u, low);
-      if (todo) {
+      if (uniform(todo)) {
         const float tl = fminf(dt, dl), br = fminf(db, dr);
         const uint32_t ka = __reduce_min_sync(~0u, __float_as_uint(lane < TILE / 2 ? tl : br));
         const uint32_t kb = __reduce_min_sync(~0u, __float_as_uint(lane < TILE / 2 ? br : tl));
@@ -445,7 +447,7 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
       __syncwarp();
     }
     if (!__syncthreads_or(todo ? 1 : 0)) break;
-    if (todo) {
+    if (uniform(todo)) {
       const int off = layout_a ? (TILE - lane) % TILE : lane;
       const int src_f = (layout_a ? lane + TILE - 1 : lane + 1) % TILE, src_r = (layout_a ? lane + 1 : lane + TILE - 1) % TILE;
       if (loaded != (layout_a ? 1 : 0)) {
@@ -455,6 +457,7 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
       }
       load_skew(d, B + lane * W_STRIDE, off);
       int r = 0;
+#pragma unroll 1
       do {
         todo = __any_sync(~0u, skew_round(d, wh, wv, src_f, src_r));
         ++nph;
@@ -475,7 +478,7 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
   // What the block's border can bring to its neighbours, and the border lines that were never written.
   const uint32_t outer = (sides >> 8) & 15u;
   if (changed) flags |= BLOCK_UNSAVED;
-  if (outer && (changed || sm.ctl.first)) {
+  if (uniform(outer && (changed || sm.ctl.first))) {
     if (!nph) block_store_border(dd, block_place(dd, blk), outer, B, W_STRIDE);
     const float* E = t.E;
     const float bl = B[lane * W_STRIDE], br = B[lane * W_STRIDE + TILE - 1], bt = B[lane], bb = B[(TILE - 1) * W_STRIDE + lane];
@@ -501,17 +504,17 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
 // of them (one per layout) before the neighbours look again.
 template <bool FMA>
 __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem<MODE_REF>& sm,
-                                                uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                                                uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, bool fill_only) {
+  const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
   const int wx = warp % BLOCK_TX, wy = warp / BLOCK_TX;
   const float INF = f_inf();
   const ImgDesc& dd = sm.ctl.desc;
   const RefEdge<FMA> re(dd.l_eucl, dd.l_grad);
   RefTile& t = sm.tile[warp];
   float* T = reinterpret_cast<float*>(t.img);
-  const bool first = sm.ctl.first != 0u;
+  const bool first = uniform(sm.ctl.first != 0u);
   const BlockPlace p = block_place(dd, blk);
-  const bool exists = (p.sides >> 12) != 0u;
+  const bool exists = uniform((p.sides >> 12) != 0u);
   // The lines that neighbouring blocks read: the sides with one beyond, and (corners) the whole left and top border.
   const uint32_t outer = ((p.sides >> 8) & 15u) | (wx == 0 ? 1u : 0u) | (wy == 0 ? 4u : 0u);
   bool todo = false, changed = false;
@@ -521,7 +524,7 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
     return nx >= 0 && nx < BLOCK_TX && ny >= 0 && ny < BLOCK_TY;
   };
   {
-    const bool seed = sm.ctl.seed != 0u, rerun = sm.ctl.rerun != 0u;
+    const bool seed = uniform(sm.ctl.seed != 0u), rerun = uniform(sm.ctl.rerun != 0u);
     const VisitBufs vb{t.img, t.V, t.V, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
     if (exists && !rerun) stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, false, seed, p.x0, p.y0);
     {
@@ -544,7 +547,15 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
       t.H[E_BOTTOM + lane] = hb;
       if (lane < 4) t.H[4 * TILE + lane] = hc;
     }
-    if (exists && !rerun) todo = changed = block_fill_ref<FMA>(re, dd, p, t, first, seed, blk, flags, q);
+    const bool fill = exists && !rerun;
+    float td[TILE];
+    if (fill && !first) block_load_tile(dd, p, td);
+    tma_wait(&t.bar, flags, 1u, q, blk, fill);
+    if (uniform(fill)) todo = changed = block_fill_ref<FMA>(re, dd, p, t, first, seed, td);
+    if (fill_only) {
+      __syncthreads();
+      return;
+    }
     if (first) flags |= BLOCK_UNSAVED;
   }
   uint32_t nph = 0;
@@ -569,7 +580,7 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
       if (ref_halo_relax<FMA>(re, T, t.E, h, p.vw, p.vh)) todo = true;
     }
     if (!__syncthreads_or(todo ? 1 : 0)) break;
-    if (todo) {
+    if (uniform(todo)) {
       changed = true;
       bool fell = false;
       todo = ref_solve<FMA>(re, t, col, BLOCK_PHASES, nph, fell);
@@ -584,7 +595,7 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
 
   // What the block's border can bring to its neighbours, and the border lines to memory.
   if (changed) flags |= BLOCK_UNSAVED;
-  if (exists && (changed || first)) {
+  if (uniform(exists && (changed || first))) {
     if (!nph) block_store_border(dd, p, outer, T, RS);
     // Neighbours in the block have an INF halo in H: every finite value would beat it, so they are masked out.
     const RefHalo h{t.H[E_LEFT + lane], t.H[E_RIGHT + lane], t.H[E_TOP + lane],  t.H[E_BOTTOM + lane],
@@ -614,7 +625,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
   extern __shared__ uint8_t smem_raw[];
   constexpr int KIND = MODE == MODE_NS ? MODE_NS : MODE_REF;
   BlockSmem<KIND>& sm = *reinterpret_cast<BlockSmem<KIND>*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
   const uint32_t first = blockIdx.x, step = gridDim.x;
   const int count = (int)((a.total - first + step - 1) / step);
   Queue q{};  // the header's error words only
@@ -653,39 +664,25 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
   int loaded = -1;
   // The first block without seeds is filled before anything activates it, so that its first visit finds it in place: with
   // one block per CTA that takes 8,000 (gray) to 12,000 (rgb8) cycles off every step of the front into new blocks.
-  {
-    int i = 0;
-    while (i < count && ((sm.ctl.seeded[i >> 5] >> (i & 31)) & 1u)) ++i;
-    if (i < count) {
-      const uint32_t img = sm.ctl.owned_img[i], blk = first + (uint32_t)i * step;
-      const ImgDesc& src = descs[img];
-      if (!src.warm) {
-        if (threadIdx.x < sizeof(ImgDesc) / 4) reinterpret_cast<uint32_t*>(&sm.ctl.desc)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&src)[threadIdx.x];
-        __syncthreads();
-        const ImgDesc& dd = sm.ctl.desc;
-        const BlockPlace p = block_place(dd, blk);
-        auto& t = sm.tile[warp];
-        if (p.vw > 0 && p.vh > 0) {
-          if constexpr (MODE == MODE_NS) {
-            const VisitBufs vb{t.img, t.Wh, t.Wv, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
-            stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, dd.channels == 3, false, p.x0, p.y0);
-            block_fill_ns(dd, p, t, true, false, blk, flags, q);
-          } else {
-            const RefEdge<MODE == MODE_REF> re(dd.l_eucl, dd.l_grad);
-            const VisitBufs vb{t.img, t.V, t.V, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
-            stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, false, false, p.x0, p.y0);
-            block_fill_ref<MODE == MODE_REF>(re, dd, p, t, true, false, blk, flags, q);
-          }
-        }
-        prev = (uint32_t)i;
-        __syncthreads();  // ctl.desc is block_next's from here on
+  int early = 0;
+  while (early < count && ((sm.ctl.seeded[early >> 5] >> (early & 31)) & 1u)) ++early;
+  if (uniform(early < count && descs[sm.ctl.owned_img[min(early, count - 1)]].warm == 0)) {
+    if (warp == 0) {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(&descs[sm.ctl.owned_img[early]]);
+      for (int i = lane; i < (int)(sizeof(ImgDesc) / 4); i += 32) reinterpret_cast<uint32_t*>(&sm.ctl.desc)[i] = src[i];
+      if (lane == 0) {
+        sm.ctl.next = (uint32_t)early;
+        sm.ctl.first = 1u;
+        sm.ctl.seed = sm.ctl.rerun = sm.ctl.nvis = 0u;
       }
     }
+  } else {
+    early = -1;
   }
   for (;;) {
-    if (warp == 0) block_next<BLOCK_SIDES<MODE>>(a, descs, sm.ctl, first, step, count, prev);
+    if (early < 0 && warp == 0) block_next<BLOCK_SIDES<MODE>>(a, descs, sm.ctl, first, step, count, prev);
     __syncthreads();
-    const uint32_t next = sm.ctl.next;
+    const uint32_t next = uniform(sm.ctl.next);
     if (next != prev && (flags & BLOCK_UNSAVED)) {
       const ImgDesc& dd = descs[sm.ctl.owned_img[prev]];
       block_store_tile(dd, block_place(dd, first + prev * step), reinterpret_cast<const float*>(sm.tile[warp].img),
@@ -695,10 +692,11 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
     }
     if (next == POP_NONE) break;
     if constexpr (MODE == MODE_NS)
-      block_visit_ns(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, wh, wv, loaded);
+      block_visit_ns(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, wh, wv, loaded, early >= 0);
     else
-      block_visit_ref<MODE == MODE_REF>(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q);
+      block_visit_ref<MODE == MODE_REF>(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, early >= 0);
     prev = next;
+    early = -1;
   }
   // Blocks never reached keep uninitialised memory: write v there.
   for (int i = 0; i < count; ++i) {

@@ -177,6 +177,12 @@ __device__ __forceinline__ uint64_t globaltimer() {
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *(const volatile uint32_t*)p; }
 
+// A value that is the same in every lane, in a form that the compiler knows to be so.  Warp-wide operations under a
+// branch whose condition it cannot prove uniform (a word from shared memory, a flag from a loop) compile to a guarded
+// sequence of about ten instructions each: a round of sweeps took 1020 instructions instead of 350.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(~0u, x, 0); }
+__device__ __forceinline__ bool uniform(bool x) { return __any_sync(~0u, x) != 0; }
+
 // Acquire-release fence at GPU scope: the release (data before a flag or counter update) and acquire (a flag
 // or counter read before the data) points of the tile visit and the queue.  Lighter than __threadfence()'s
 // sequentially consistent fence, which only the end-of-queue handshake (a store then a load of another word,

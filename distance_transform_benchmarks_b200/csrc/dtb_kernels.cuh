@@ -201,17 +201,21 @@ __device__ __forceinline__ float bucket_inv_width(const Queue& q, uint32_t img) 
 // to land before the warp leaves; after that the wait gives up, and a copy may then still be pending.  The
 // error word ends the launch: every later pop returns POP_NONE, so the warp issues no further copy and never
 // waits on this barrier again.
-__device__ __forceinline__ bool tma_wait(uint64_t* bar, uint32_t& pbits, uint32_t pmask, const Queue& q, uint32_t tile) {
+// `need`: false returns at once.  The wait is called outside of branches with that flag instead of inside of one: its
+// loop has no exit that the compiler knows to be uniform, and a branch around it would make it guard every warp-wide
+// operation that follows (see `uniform`).
+__device__ __forceinline__ bool tma_wait(uint64_t* bar, uint32_t& pbits, uint32_t pmask, const Queue& q, uint32_t tile,
+                                         bool need = true) {
   const uint32_t parity = (pbits & pmask) ? 1u : 0u;
   const uint64_t t0 = globaltimer();
   bool ok = true;
-  while (!mbar_try_wait(bar, parity)) {
+  while (need && !mbar_try_wait(bar, parity)) {
     const uint64_t dt = globaltimer() - t0;
     if (ok && dt > TMA_TIMEOUT_NS) { set_error(q, DERR_TMA_TIMEOUT, tile); ok = false; }
     if (dt > 2 * TMA_TIMEOUT_NS) break;
   }
-  pbits ^= pmask;
-  return ok;
+  if (need) pbits ^= pmask;
+  return __all_sync(~0u, ok);
 }
 
 // Shared memory of one visit.  A self-staging visit loads its image box and seed-mask box on `bar`; a visit
@@ -399,9 +403,10 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   const int tx = (int)(local % (uint32_t)dd.tiles_x), ty = (int)(local / (uint32_t)dd.tiles_x);
   const int x0 = tx * TILE, y0 = ty * TILE;
   const int vw = min(TILE, dd.width - x0), vh = min(TILE, dd.height - y0);
+  rerun = uniform(rerun);
   const bool first = !(old_state & ST_VISITED);
   const bool seed = (old_state & ST_SEED) != 0;
-  const bool rgb = dd.channels == 3;
+  const bool rgb = uniform(dd.channels == 3);
   const float v = dd.v;
   *nph_out = 0;
   *nact_out = 0;
@@ -446,8 +451,8 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
   }
 
-  if (!rerun && !tma_wait(vb.bar, *vb.pbits, vb.pmask, sch.q, tile)) return;
-  if (PRESTAGED && seed && !tma_wait(vb.mbar, *vb.pbits, vb.mmask, sch.q, tile)) return;
+  if (!tma_wait(vb.bar, *vb.pbits, vb.pmask, sch.q, tile, !rerun)) return;
+  if (PRESTAGED && !tma_wait(vb.mbar, *vb.pbits, vb.mmask, sch.q, tile, seed)) return;
 
   // Seeds first: the mask box shares memory with Wv.
   uint32_t seeds = 0;  // this lane's column of the mask tile
@@ -528,6 +533,7 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
       load_skew(d, B + lane * W_STRIDE, off);
       bool ch;
       int r = 0;
+#pragma unroll 1  // one copy of the round: the kernel's code is fetched through small instruction caches
       do {
         ch = __any_sync(~0u, skew_round(d, wh, wv, src_f, src_r));
         any |= ch;
@@ -864,6 +870,7 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
   const int tx = (int)(local % (uint32_t)dd.tiles_x), ty = (int)(local / (uint32_t)dd.tiles_x);
   const int x0 = tx * TILE, y0 = ty * TILE;
   const int vw = min(TILE, dd.width - x0), vh = min(TILE, dd.height - y0);
+  rerun = uniform(rerun);
   const bool first = !(old_state & ST_VISITED);
   const bool seed = (old_state & ST_SEED) != 0;
   const float v = dd.v;
@@ -902,14 +909,14 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
 
   float* T = reinterpret_cast<float*>(sm.img);  // overlays the image box once the edge words are computed
   float wsum = 0.0f;
-  if (!rerun) {
-    float d[TILE];
-    if (!first) {
-      const uint8_t* lb = dist_base(dd, y0, x0 + lane, 0u);
+  float d[TILE];
+  if (!rerun && !first) {
+    const uint8_t* lb = dist_base(dd, y0, x0 + lane, 0u);
 #pragma unroll
-      for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
-    }
-    if (!tma_wait(&sm.bar, parity, 1u, sch.q, tile)) return;
+    for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
+  }
+  if (!tma_wait(&sm.bar, parity, 1u, sch.q, tile, !rerun)) return;
+  if (!rerun) {
     uint32_t seeds = 0;  // this lane's column of the mask tile (its box shares memory with V)
     if (seed) {
       const uint8_t* mbox = reinterpret_cast<const uint8_t*>(sm.V);
