@@ -483,8 +483,12 @@ uint32_t count_blocks(const std::vector<Job>& jobs) {
   return (uint32_t)t;
 }
 
-static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t) {
-  return std::max<uint32_t>(1u, (uint32_t)(ctx->num_sms * BLOCK_CTAS) * (uint32_t)t.grid_percent / 100u);
+// CTAs per SM of the block kernel: with many images (fronts of their own) more blocks in flight pay, with few they only
+// visit blocks too early (2 against 3 CTAs: 48 images of 7 Mpx 0.72 / 0.62 ms, 40 of 15 Mpx 1.44 / 1.25, 24 0.45 / 0.43, 16
+// small ones 0.228 / 0.232, 1333x1999 rgb8 0.43 / 0.44, 4096^2 maze 3.6 / 4.4, a serving burst of 24 2.06 / 2.16).
+static int block_ctas(int mode, int n) { return mode == MODE_NS && n >= 32 ? BLOCK_CTAS_MANY : BLOCK_CTAS; }
+static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t, int ctas) {
+  return std::max<uint32_t>(1u, (uint32_t)(ctx->num_sms * ctas) * (uint32_t)t.grid_percent / 100u);
 }
 
 // Whether a run takes the block kernel: under the default tuning, up to as many blocks as its CTAs may own (9472 on 148
@@ -495,7 +499,7 @@ static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t) {
 // against 0.23 / 0.56 / 0.80, 3648x2432 1.21 / 2.02 / 1.74 against 0.98 / 2.30 / 1.67, 6000^2 2.8 / 4.7 / 3.2 against 2.3 / 5.9 / 2.5.
 bool use_blocks(dtb_context ctx, int mode, const LaunchTuning& t, uint32_t blocks) {
   (void)mode;
-  return !t.chosen && blocks > 0 && blocks <= std::min(block_grid(ctx, t) * (uint32_t)BLOCK_OWNED_MAX, BLOCK_RUN_MAX);
+  return !t.chosen && blocks > 0 && blocks <= std::min(block_grid(ctx, t, BLOCK_CTAS) * (uint32_t)BLOCK_OWNED_MAX, BLOCK_RUN_MAX);
 }
 
 dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
@@ -519,7 +523,8 @@ dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& 
   }
   if (ev0) DTB_CUDA(ctx, cudaEventRecord(ev0, stream));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, block_grid(ctx, t)));
+  const int ctas = block_ctas(mode, L.n);
+  cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, block_grid(ctx, t, ctas)));
   cfg.blockDim = dim3(BLOCK_WARPS * 32);
   cfg.dynamicSmemBytes = mode == MODE_NS ? BLOCK_SMEM<MODE_NS> : BLOCK_SMEM<MODE_REF>;
   cfg.stream = stream;
@@ -528,9 +533,10 @@ dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& 
   attr[0].val.cooperative = 1;  // all CTAs resident: a CTA waits for blocks that the others activate
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const void* fn = mode == MODE_NS ? (const void*)ggdt_block<MODE_NS>
-                   : mode == MODE_REF ? (const void*)ggdt_block<MODE_REF>
-                                      : (const void*)ggdt_block<MODE_REF_NOFMA>;
+  const void* fn = mode == MODE_NS ? (ctas == BLOCK_CTAS ? (const void*)ggdt_block<MODE_NS, BLOCK_CTAS>
+                                                         : (const void*)ggdt_block<MODE_NS, BLOCK_CTAS_MANY>)
+                   : mode == MODE_REF ? (const void*)ggdt_block<MODE_REF, BLOCK_CTAS>
+                                      : (const void*)ggdt_block<MODE_REF_NOFMA, BLOCK_CTAS>;
   void* args[3] = {(void*)&ddesc, (void*)&dtm, (void*)&a};
   DTB_CUDA(ctx, cudaLaunchKernelExC(&cfg, fn, args));
   if (ev1) DTB_CUDA(ctx, cudaEventRecord(ev1, stream));
@@ -935,13 +941,15 @@ DTB_API dtb_status dtb_context_create(int32_t device, dtb_context* out) {
   const struct {
     const void* fn;
     size_t smem;
-  } block_fns[3] = {{(const void*)ggdt_block<MODE_NS>, BLOCK_SMEM<MODE_NS>},
-                    {(const void*)ggdt_block<MODE_REF>, BLOCK_SMEM<MODE_REF>},
-                    {(const void*)ggdt_block<MODE_REF_NOFMA>, BLOCK_SMEM<MODE_REF>}};
+    int ctas;
+  } block_fns[4] = {{(const void*)ggdt_block<MODE_NS, BLOCK_CTAS>, BLOCK_SMEM<MODE_NS>, BLOCK_CTAS},
+                    {(const void*)ggdt_block<MODE_NS, BLOCK_CTAS_MANY>, BLOCK_SMEM<MODE_NS>, BLOCK_CTAS_MANY},
+                    {(const void*)ggdt_block<MODE_REF, BLOCK_CTAS>, BLOCK_SMEM<MODE_REF>, BLOCK_CTAS},
+                    {(const void*)ggdt_block<MODE_REF_NOFMA, BLOCK_CTAS>, BLOCK_SMEM<MODE_REF>, BLOCK_CTAS}};
   for (const auto& f : block_fns) {
     int bps = 0;
     ok = ok && cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, f.fn, BLOCK_WARPS * 32, f.smem) == cudaSuccess && bps >= BLOCK_CTAS;
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, f.fn, BLOCK_WARPS * 32, f.smem) == cudaSuccess && bps >= f.ctas;
   }
   int ref_bps_nofma = 0;
   ok = ok && cudaFuncSetAttribute(kref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REF_SMEM) == cudaSuccess &&

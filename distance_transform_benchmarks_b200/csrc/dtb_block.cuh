@@ -61,7 +61,7 @@ struct BlockSmem {
 };
 template <int MODE>
 constexpr size_t BLOCK_SMEM = sizeof(BlockSmem<MODE>) + 128;
-static_assert(BLOCK_CTAS * (BLOCK_SMEM<MODE_NS> + 1024) <= 228 * 1024 && BLOCK_CTAS * (BLOCK_SMEM<MODE_REF> + 1024) <= 228 * 1024,
+static_assert(BLOCK_CTAS_MANY * (BLOCK_SMEM<MODE_NS> + 1024) <= 228 * 1024 && BLOCK_CTAS * (BLOCK_SMEM<MODE_REF> + 1024) <= 228 * 1024,
               "the blocks of an SM must fit its shared memory");
 
 // Device words of a run.
@@ -619,8 +619,8 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
   if (warp == 0) block_complete<BLOCK_SIDES<MODE_REF>>(a, sm.ctl, blk);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(BLOCK_WARPS * 32, BLOCK_CTAS)
+template <int MODE, int CTAS>
+__global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
     ggdt_block(const ImgDesc* __restrict__ descs, const CUtensorMap* __restrict__ tmaps, BlockRun a) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int KIND = MODE == MODE_NS ? MODE_NS : MODE_REF;

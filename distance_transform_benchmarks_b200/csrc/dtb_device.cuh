@@ -24,11 +24,11 @@ constexpr int GRAY_LUT_OFFSET = 2304;
 static_assert(GRAY_LUT_OFFSET >= IMG_BOX_ROWS * IMG_BOX_GRAY && GRAY_LUT_OFFSET + 1024 <= IMG_BOX_ROWS * IMG_BOX_RGB,
               "gray weight table must fit the unused part of the image box");
 
-// Block kernel: tiles of a block (one warp each), its size in pixels, and CTAs per SM.  Two CTAs of four warps leave
-// 255 registers a thread, so a warp holds its tile and weights without spills; measured against 3 CTAs of 2x2, and one
-// of 4x2, 4x3 and 4x4 tiles, on 512^2 gray, 2048^2 gray and 4096^2 rgb8: 0.17 / 0.45 / 1.10 ms against 0.19 / 0.51 / 1.18,
+// Block kernel: tiles of a block (one warp each), its size in pixels, and CTAs per SM for runs of few and of many images.
+// Two CTAs of four warps leave 255 registers a thread, three 168; measured when it was chosen against 3 CTAs of 2x2, and
+// one of 4x2, 4x3 and 4x4 tiles, on 512^2 gray, 2048^2 gray and 4096^2 rgb8: 0.17 / 0.45 / 1.10 ms against 0.19 / 0.51 / 1.18,
 // 0.17 / 0.46 / 1.13, 0.20 / 0.53 / 1.14 and 0.25 / 0.69 / 1.34 ms.
-constexpr int BLOCK_TX = 2, BLOCK_TY = 2, BLOCK_CTAS = 2;
+constexpr int BLOCK_TX = 2, BLOCK_TY = 2, BLOCK_CTAS = 2, BLOCK_CTAS_MANY = 3;
 constexpr int BLOCK_W = BLOCK_TX * TILE, BLOCK_H = BLOCK_TY * TILE;
 
 // Tile state word: flags in the low byte, image index of the tile in the upper 24 bits.
