@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
     const uint32_t old = sch.claim(cur);
     const uint32_t img = old >> ST_IMG_SHIFT;
     const ImgDesc dd = descs[img];
-    const VisitBufs vb{sm.box[k], sm.Wh, sm.Wv, sm.E, &sm.bar[k], &sm.mbar, 1u << k, 4u, &pbits};
+    const VisitBufs vb{sm.box[k], sm.t.Wv, &sm.t, &sm.bar[k], &sm.mbar, 1u << k, 4u, &pbits};
     uint32_t nph, nact;
     visit_ns<true>(dd, tmaps + 2 * img, tmaps + 2 * img + 1, cur, old, vb, sch, &nph, &nact);
     count_visit(ws, q, nph, nact);
@@ -430,16 +430,22 @@ uint64_t tuning_key(int n, uint32_t total) {
   return ((uint64_t)next_pow2((uint32_t)std::max(n, 1)) << 32) | next_pow2(std::max<uint32_t>(total, 1));
 }
 
-// Many images of together 96k tiles or more keep 12 warps an SM busy with fronts of their own, and then finer buckets pay:
-// 512 images of 200k tiles 5.31 -> 4.90 ms, 2000 of 100k 3.12 -> 2.74.  A single large picture has fewer fronts than
-// workers, and more workers only visit tiles too early (8192x6400 maze 8.2 -> 10.1 ms, 8192x7000 gray 2.40 -> 2.56), and
-// 128 images of 57k tiles are even (2.41, 2.35).
-LaunchTuning tuning_for(dtb_context ctx, int n, uint32_t total) {
+// The tile kernel's launch shape and queue policy by default.  12 warps an SM instead of 8 hide more of a visit's round
+// trips but visit more tiles too early: they pay where many images bring many fronts (128 images of 57k tiles 2.46 -> 1.98
+// ms, 512 of 200k 5.20 -> 4.14), and on rgb8, whose visits are longer (8192^2 1.70 -> 1.44), not on one large gray picture
+// (8192x7000 gray 2.33 -> 2.57, 8192x6400 maze 7.5 -> 7.7).  Finer buckets need a long queue to choose from (512 images 4.14 ->
+// 4.10 ms, 2000 small ones of 100k tiles 2.88 -> 2.74, but 128 images 1.98 -> 2.05).
+LaunchTuning tuning_for(dtb_context ctx, const std::vector<Job>& jobs, uint32_t total) {
+  const int n = (int)jobs.size();
   auto it = ctx->tuned.find(tuning_key(n, total));
   if (it != ctx->tuned.end()) return it->second;
   LaunchTuning t = ctx->tuning;
-  if (!t.chosen && n >= 32 && total >= 96u * 1024u) {
-    t.variant = ns_variant_of(3, false);
+  if (t.chosen) return t;
+  uint64_t rgb = 0;
+  for (const Job& j : jobs)
+    if (j.channels == 3) rgb += (uint64_t)j.tiles_x() * j.tiles_y();
+  if (n >= 32 || 2 * rgb >= total) t.variant = ns_variant_of(3, false);
+  if (n >= 32 && total >= 96u * 1024u) {
     t.buckets = 16;
     t.bucket_tiles = 0.1f;
   }
@@ -768,7 +774,7 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
       return fail(ctx, DTB_ERR_INVALID_ARG, "one call covers images of one weight mode");
   // Kernel mode: ref-mode calls with left-to-right rounding run their own kernels.
   const int mode = n == 0 ? MODE_NS : (jobs[0].mode == MODE_REF && !jobs[0].ref_fma) ? MODE_REF_NOFMA : jobs[0].mode;
-  const LaunchTuning tuning = tuning_for(ctx, n, total);
+  const LaunchTuning tuning = tuning_for(ctx, jobs, total);
   ScratchLayout L = layout_for(n, total, resident_workers(ctx, mode, tuning), rounds,
                                rounds ? 1u : (uint32_t)tuning.buckets);
   L.blocks = count_blocks(jobs);

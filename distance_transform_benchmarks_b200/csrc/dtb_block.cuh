@@ -296,7 +296,7 @@ __device__ __forceinline__ bool block_fill_ns(const ImgDesc& dd, const BlockPlac
     for (int y = 0; y < TILE; ++y) seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
   }
   __syncwarp();
-  tile_weights(dd.g2, uniform(dd.channels == 3), p.vw, p.vh, t.img, t.Wh, t.Wv, t.E);
+  tile_weights<2>(dd.g2, uniform(dd.channels == 3), p.vw, p.vh, t.img, t.Wh, t.Wv, t.E);
   __syncwarp();
   float* pb = reinterpret_cast<float*>(t.img) + lane;
   if (first) {
@@ -373,7 +373,7 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
     const BlockPlace p = block_place(dd, blk);
     sides = uniform(p.sides);
     const bool exists = (sides & 0x1000u) != 0u;
-    const VisitBufs vb{t.img, t.Wh, t.Wv, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
+    const VisitBufs vb{t.img, t.Wv, nullptr, &t.bar, &t.bar, 1u, 1u, &flags};
     if (exists && !rerun) stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, dd.channels == 3, seed, p.x0, p.y0);
     {
       float top = INF, bot = INF, lft = INF, rgt = INF;
@@ -525,7 +525,7 @@ __device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtenso
   };
   {
     const bool seed = uniform(sm.ctl.seed != 0u), rerun = uniform(sm.ctl.rerun != 0u);
-    const VisitBufs vb{t.img, t.V, t.V, t.E, &t.bar, &t.bar, 1u, 1u, &flags};
+    const VisitBufs vb{t.img, t.V, nullptr, &t.bar, &t.bar, 1u, 1u, &flags};
     if (exists && !rerun) stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, false, seed, p.x0, p.y0);
     {
       // The halo on the block's border.

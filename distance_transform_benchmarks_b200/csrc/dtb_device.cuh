@@ -9,6 +9,7 @@
 // combines two edge weights before adding them to a distance.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -112,24 +113,27 @@ struct Queue {
 };
 constexpr uint32_t KEY_NONE = 0xFFFFFFFFu;
 
-// Per-warp shared memory slot (13.4 KB: 16 warps per SM fit in 228 KB).
-// Weight and tile buffers keep 34 floats a row: a lane-per-column access ([k * 34 + lane]) is conflict-free, and so
-// is the sweeps' diagonal access ([lane * 34 + ((k +- lane) & 31)]: consecutive lanes are 33 or 35 words apart);
-// a lane-per-row access of one column, used only at the tile's borders, costs two wavefronts.
+// Shared memory of a tile.  Weight and distance buffers keep 34 floats a row: a lane-per-column access ([k * 34 + lane])
+// is conflict-free, and so is the sweeps' diagonal access ([lane * 34 + ((k +- lane) & 31)]: consecutive lanes are 33 or
+// 35 words apart); a lane-per-row access of one column, used only at the tile's borders, costs two wavefronts.
 constexpr int W_STRIDE = TILE + 2;
 constexpr int TILE_BUF_BYTES = TILE * W_STRIDE * 4;
 constexpr int IMG_REGION = IMG_BOX_ROWS * IMG_BOX_RGB > TILE_BUF_BYTES ? IMG_BOX_ROWS * IMG_BOX_RGB : TILE_BUF_BYTES;
 // Halo edge weights: 32 floats a side.
 constexpr int E_LEFT = 0, E_RIGHT = TILE, E_TOP = 2 * TILE, E_BOTTOM = 3 * TILE;
+struct alignas(128) TileBufs {
+  float B[TILE * W_STRIDE];         // distances B[y * 34 + x]
+  float Wh[TILE * W_STRIDE];        // Wh[y * 34 + x] = weight of edge (x-1, x) on row y; INF at x = 0
+  float Wv[(TILE + 1) * W_STRIDE];  // Wv[y * 34 + x] = weight of edge (y-1, y) on column x; INF at y = 0 and in row 32;
+                                    // its first 1 KB receives the seed-mask TMA box before the weights
+  float E[4 * TILE];                // weights of the edges to the halo, per side
+};
+// Per-warp shared memory of the ns-mode tile kernels (17.8 KB: 12 warps per SM fit in 228 KB).
 struct alignas(128) WarpSmem {
-  uint8_t img[IMG_REGION];                   // TMA destination of the image box (gray uses IMG_BOX_ROWS x 64); once
-                                             // the weights are computed, the tile buffer B[y * 34 + x]
-  float Wh[TILE * W_STRIDE];                 // ns-mode: Wh[y * 34 + x] = weight of edge (x-1, x) on row y; INF at x = 0
-  float Wv[TILE * W_STRIDE];                 // ns-mode: Wv[y * 34 + x] = weight of edge (y-1, y) on column x; INF at
-                                             // y = 0; its first 1 KB receives the seed-mask TMA box before the weights
-  float E[4 * TILE];                         // ns-mode: weights of the edges to the halo, per side
-  uint64_t bar;                              // TMA mbarrier
-  uint32_t keep;                             // tile this warp keeps for its next visit (POP_NONE: none)
+  uint8_t img[IMG_BOX_ROWS * IMG_BOX_RGB];  // TMA destination of the image box (gray uses IMG_BOX_ROWS x 64)
+  TileBufs t;
+  uint64_t bar;                             // TMA mbarrier
+  uint32_t keep;                            // tile this warp keeps for its next visit (POP_NONE: none)
 };
 
 // Per-warp shared memory of a ref-mode visit (23.6 KB: 8 warps per SM).  The edge words (|dI|, or l_grad * |dI| without
@@ -150,19 +154,14 @@ struct alignas(128) RefTile {
 };
 static_assert(sizeof(RefTile::img) >= IMG_BOX_ROWS * IMG_BOX_GRAY, "the gray image box must fit");
 
-// Per-warp shared memory of the staged-ahead tile kernel (18 KB: 12 warps per SM fit in 228 KB): the image
-// boxes of the tile being visited and of the warp's next tile, each the tile buffer B of its own visit once its
-// weights are computed; the weights; a barrier per box and one for the seed-mask box.
-constexpr int IMG_BOX_BYTES = IMG_REGION;
+// Per-warp shared memory of the staged-ahead tile kernel (22 KB): the image boxes of the tile being visited and of the
+// warp's next tile, a barrier per box and one for the seed-mask box.
 struct alignas(128) WarpSmemP {
-  uint8_t box[2][IMG_BOX_BYTES];
-  float Wh[TILE * W_STRIDE];
-  float Wv[TILE * W_STRIDE];         // its first 1 KB receives the seed-mask TMA box before the weights
-  float E[4 * TILE];
-  uint64_t bar[2];                   // image box k
-  uint64_t mbar;                     // seed-mask box
+  uint8_t box[2][IMG_BOX_ROWS * IMG_BOX_RGB];
+  TileBufs t;
+  uint64_t bar[2];  // image box k
+  uint64_t mbar;    // seed-mask box
 };
-static_assert(TILE * W_STRIDE * 4 <= IMG_BOX_BYTES, "the tile buffer must fit an image box");
 
 // ------------------------------------------------------------------------------------------------------
 // PTX helpers
@@ -215,6 +214,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// Copies 4 bytes from global to shared memory asynchronously (generic proxy; complete after cp_async_wait).
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void tmap_acquire(const CUtensorMap* map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
 }
@@ -525,6 +529,20 @@ __device__ __forceinline__ void load_skew(float (&r)[TILE], const float* row, in
   const float* p = row + off;
 #pragma unroll
   for (int j = 0; j < TILE; ++j) r[j] = (off >= TILE - j ? p - TILE : p)[j];
+}
+// The tile and its weights in layout A or B: one address per register for all three arrays.
+__device__ __forceinline__ void load_skew_tile(float (&d)[TILE], float (&wh)[TILE], float (&wv)[TILE], const TileBufs& t, int lane,
+                                               int off, bool layout_a) {
+  constexpr int OH = offsetof(TileBufs, Wh) / 4, OV = offsetof(TileBufs, Wv) / 4;
+  const float* p = t.B + lane * W_STRIDE + off;
+  const int dv = layout_a ? 0 : W_STRIDE;  // layout B: the edges to the row below
+#pragma unroll
+  for (int j = 0; j < TILE; ++j) {
+    const float* q = off >= TILE - j ? p - TILE : p;
+    d[j] = q[j];
+    wh[j] = q[j + OH];
+    wv[j] = (q + dv)[j + OV];
+  }
 }
 __device__ __forceinline__ void store_skew(float* row, int off, const float (&r)[TILE]) {
   asm("" : "+r"(off) : "f"(r[0]));  // or the addresses of the loads would be kept in registers through the rounds

@@ -277,9 +277,9 @@ Queue make_queue(uint8_t* dbase, const ScratchLayout& L, uint64_t timeout_ns = D
 bool valid_policy(int buckets, float bucket_tiles);
 // Workload key of the autotuner cache: image count and tile count, each rounded to a power of two.
 uint64_t tuning_key(int n, uint32_t total);
-// The tuning of a call or plan of n images and `total` tiles: the autotuner's result for its size class, else the
-// context's, or by default the one for its size.
-LaunchTuning tuning_for(dtb_context ctx, int n, uint32_t total);
+// The tuning of a call or plan of `total` tiles: the autotuner's result for its size class, else the context's, or by
+// default one for its size and kind.
+LaunchTuning tuning_for(dtb_context ctx, const std::vector<Job>& jobs, uint32_t total);
 dtb_status read_device_status(dtb_context ctx, const QueueHdr* hdr, dtb_stats* stats);
 // Counters and status of a run from its queue header.
 dtb_status status_of(dtb_context ctx, const QueueHdr& h, dtb_stats* stats);

@@ -221,10 +221,9 @@ __device__ __forceinline__ bool tma_wait(uint64_t* bar, uint32_t& pbits, uint32_
 // Shared memory of one visit.  A self-staging visit loads its image box and seed-mask box on `bar`; a visit
 // staged ahead finds its image box issued on `bar` already and loads the mask box (seed visits only) on `mbar`.
 struct VisitBufs {
-  uint8_t* box;       // image box (TMA destination), the tile buffer B once the weights are computed
-  float* Wh;
-  float* Wv;          // its first 1 KB receives the seed-mask box before the weights
-  float* E;
+  uint8_t* box;       // image box (TMA destination)
+  void* mask;         // seed-mask box (TMA destination), used before the weights are computed
+  TileBufs* t;
   uint64_t* bar;
   uint64_t* mbar;
   uint32_t pmask;     // bit of *pbits holding bar's phase parity
@@ -233,7 +232,7 @@ struct VisitBufs {
 };
 
 __device__ __forceinline__ VisitBufs visit_bufs(WarpSmem& sm, uint32_t& pbits) {
-  return VisitBufs{sm.img, sm.Wh, sm.Wv, sm.E, &sm.bar, &sm.bar, 1u, 1u, &pbits};
+  return VisitBufs{sm.img, sm.t.Wv, &sm.t, &sm.bar, &sm.bar, 1u, 1u, &pbits};
 }
 
 // Issues one 2-D TMA box into this warp's shared memory on `bar` (whole warp; lane 0 issues).  Orders this
@@ -280,7 +279,7 @@ __device__ __forceinline__ void stage_tile(const VisitBufs& vb, const CUtensorMa
     const uint32_t bytes = (rgb ? IMG_BOX_RGB : IMG_BOX_GRAY) * IMG_BOX_ROWS + (with_mask ? TILE * TILE : 0);
     mbar_arrive_expect_tx(vb.bar, bytes);
     tma_load_2d(vb.box, tm_img, rgb ? 3 * x0 - 16 : x0 - 16, y0 - 1, vb.bar);
-    if (with_mask) tma_load_2d(vb.Wv, tm_mask, x0, y0, vb.bar);
+    if (with_mask) tma_load_2d(vb.mask, tm_mask, x0, y0, vb.bar);
   }
 }
 
@@ -293,7 +292,10 @@ __device__ __forceinline__ uint32_t box_pix(const uint8_t* box, bool rgb, int r,
 }
 
 // Edge weights of a tile from its staged image box into Wh / Wv / E (lane = x; the left and right halo edges
-// lane = y).  Returns this lane's sum of the tile's internal column edges (x < vw, 0 < y < vh).
+// lane = y).  Returns this lane's sum of the tile's internal column edges (x < vw, 0 < y < vh).  UNROLL: rows in flight;
+// the tile kernel, whose warps are all at different places of its code, runs faster with the smallest code (1 against 2:
+// 512-image plan 4.41 against 4.70 ms), the block kernel, whose warps move together, with 2.
+template <int UNROLL>
 __device__ __forceinline__ float tile_weights(float g2, bool rgb, int vw, int vh, uint8_t* box, float* Wh, float* Wv, float* E) {
   const int lane = threadIdx.x & 31;
   const float INF = f_inf();
@@ -304,7 +306,7 @@ __device__ __forceinline__ float tile_weights(float g2, bool rgb, int vw, int vh
     // same bits) costs 8 square roots per lane instead of 65; it sits in the part of the image box that the
     // 64-byte gray rows leave unused.
     float* lut = reinterpret_cast<float*>(box + GRAY_LUT_OFFSET);
-#pragma unroll
+#pragma unroll(UNROLL == 1 ? 2 : 8)
     for (int k = 0; k < 8; ++k) {
       const uint32_t a = (uint32_t)(lane + 32 * k);
       lut[a] = ns_weight_sq(a * a, g2);
@@ -315,7 +317,7 @@ __device__ __forceinline__ float tile_weights(float g2, bool rgb, int vw, int vh
     et = lut[abs(pprev - (int)col[0])];
     Wv[lane] = INF;
     Wh[lane] = lane == 0 ? INF : lut[abs(pprev - (int)col[IMG_BOX_GRAY - 1])];
-#pragma unroll 2
+#pragma unroll UNROLL
     for (int y = 1; y < TILE; ++y) {
       const int pcur = col[(y + 1) * IMG_BOX_GRAY];
       const float w = lut[abs(pcur - pprev)];
@@ -337,7 +339,7 @@ __device__ __forceinline__ float tile_weights(float g2, bool rgb, int vw, int vh
       const float wx = ns_weight(__shfl_up_sync(~0u, pprev, 1), pprev, g2);
       Wh[lane] = lane == 0 ? INF : wx;
     }
-#pragma unroll 2
+#pragma unroll UNROLL
     for (int y = 1; y < TILE; ++y) {
       const uint32_t pcur = box_pix(box, true, y + 1, lane);
       const float w = ns_weight(pprev, pcur, g2);
@@ -387,8 +389,8 @@ __device__ __forceinline__ float tile_weights(float g2, bool rgb, int vw, int vh
 // Returns the number of rounds and activations through *nph / *nact.
 //
 // rerun: the warp visits again the tile it has just visited (its halo dropped while it ran, and the visit kept
-// it).  The warp's shared memory still holds that tile's edge weights (Wh / Wv / E) and its final distances (the
-// tile buffer B, equal to the tile in global memory: no other warp can have visited it in between), so the
+// it).  The warp's shared memory still holds that tile's edge weights (Wh / Wv / E) and its final distances (B, equal
+// to the tile in global memory: no other warp can have visited it in between), so the
 // re-run reloads only the neighbour states and halos: no bulk copy, no weights, no tile loads.
 // ------------------------------------------------------------------------------------------------------
 constexpr int LAYOUT_ROUNDS = 3;
@@ -415,7 +417,7 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   } else if (!PRESTAGED) {
     stage_tile(vb, tm_img, tm_mask, rgb, seed, x0, y0);
   } else if (seed) {
-    stage_box(vb.Wv, vb.mbar, tm_mask, TILE * TILE, x0, y0);
+    stage_box(vb.mask, vb.mbar, tm_mask, TILE * TILE, x0, y0);
   }
 
   // Neighbour states: lane 0 left, 1 right, 2 top, 3 bottom.
@@ -443,31 +445,51 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     if (nexist & 2u) rgt = (nvis & 2u) ? ld_dist(dd, y0 + lane, x0 + TILE) : v;
   }
 
-  // Tile distances (lane = x).
-  float d[TILE];
-  if (!rerun && !first) {
-    const uint8_t* lb = dist_base(dd, y0, x0 + lane, 0u);
-#pragma unroll
-    for (int y = 0; y < TILE; ++y) d[y] = (lane < vw && y < vh) ? ld_dist_at(lb, dd.dist_pitch, y) : INF;
+  // Tile distances (lane = x): v on a first visit, else copied behind the weights' back.  The fence above orders the
+  // copies after what the neighbours' states say, like the halo loads.
+  float* B = vb.t->B;
+  const int rows = lane < vw ? vh : 0;  // this lane's rows of the picture
+  if (!rerun) {
+    const uint8_t* src = dist_base(dd, y0, x0 + lane, 0u);
+#pragma unroll 2
+    for (int y = 0; y < TILE; ++y) {
+      float* dst = B + y * W_STRIDE + lane;
+      if (first || y >= rows) *dst = y < rows ? v : INF;
+      else cp_async4(dst, src + (int64_t)y * dd.dist_pitch);
+    }
   }
 
-  if (!tma_wait(vb.bar, *vb.pbits, vb.pmask, sch.q, tile, !rerun)) return;
-  if (PRESTAGED && !tma_wait(vb.mbar, *vb.pbits, vb.mmask, sch.q, tile, seed)) return;
+  if (!tma_wait(vb.bar, *vb.pbits, vb.pmask, sch.q, tile, !rerun)) {
+    cp_async_wait();
+    return;
+  }
+  if (PRESTAGED && !tma_wait(vb.mbar, *vb.pbits, vb.mmask, sch.q, tile, seed)) {
+    cp_async_wait();
+    return;
+  }
 
   // Seeds first: the mask box shares memory with Wv.
   uint32_t seeds = 0;  // this lane's column of the mask tile
   if (seed) {
-    const uint8_t* mbox = reinterpret_cast<const uint8_t*>(vb.Wv);
-#pragma unroll 4
-    for (int y = 0; y < TILE; ++y) seeds |= (lane < vw && y < vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
+    const uint8_t* mbox = reinterpret_cast<const uint8_t*>(vb.mask);
+#pragma unroll 2
+    for (int y = 0; y < TILE; ++y) seeds |= (y < rows && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
   }
   __syncwarp();
 
   // Edge weights into Wh / Wv / E (lane = x; the left and right halo edges lane = y).  A re-run has them.
   const uint32_t img_idx = old_state >> ST_IMG_SHIFT;
+  const float* E = vb.t->E;
   float wsum = 0.0f;
   if (!rerun) {
-    wsum = tile_weights(dd.g2, rgb, vw, vh, vb.box, vb.Wh, vb.Wv, vb.E);
+    wsum = tile_weights<1>(dd.g2, rgb, vw, vh, vb.box, vb.t->Wh, vb.t->Wv, vb.t->E);
+    vb.t->Wv[TILE * W_STRIDE + lane] = INF;
+    cp_async_wait();
+    if (seed) {
+#pragma unroll 2
+      for (int y = 0; y < TILE; ++y)
+        if ((seeds >> y) & 1u) B[y * W_STRIDE + lane] = 0.0f;
+    }
   }
   __syncwarp();
 
@@ -482,21 +504,7 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     }
   }
 
-  // The tile buffer B overlays the image box, which is no longer needed.  Relax the halo edges in it: top and bottom
-  // lane = x, then left and right lane = y.
-  float* B = reinterpret_cast<float*>(vb.box);
-  const float* E = vb.E;
-  if (!rerun) {
-    float* pb = B + lane;
-    if (first) {
-#pragma unroll 4
-      for (int y = 0; y < TILE; ++y) pb[y * W_STRIDE] = (lane < vw && y < vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
-    } else {
-#pragma unroll
-      for (int y = 0; y < TILE; ++y) pb[y * W_STRIDE] = ((seeds >> y) & 1u) ? 0.0f : d[y];
-    }
-    __syncwarp();
-  }
+  // Relax the halo edges in B: top and bottom lane = x, then left and right lane = y.
   bool any, layout_a;
   {
     const float ct = __fadd_rn(top, E[E_TOP + lane]), cb = __fadd_rn(bot, E[E_BOTTOM + lane]);
@@ -527,10 +535,8 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
     for (;;) {
       const int off = layout_a ? (TILE - lane) % TILE : lane;
       const int src_f = (layout_a ? lane + TILE - 1 : lane + 1) % TILE, src_r = (layout_a ? lane + 1 : lane + TILE - 1) % TILE;
-      float wh[TILE], wv[TILE];
-      load_skew(wh, vb.Wh + lane * W_STRIDE, off);
-      load_skew(wv, vb.Wv + (layout_a ? lane : src_f) * W_STRIDE, off);
-      load_skew(d, B + lane * W_STRIDE, off);
+      float d[TILE], wh[TILE], wv[TILE];
+      load_skew_tile(d, wh, wv, *vb.t, lane, off, layout_a);
       bool ch;
       int r = 0;
 #pragma unroll 1  // one copy of the round: the kernel's code is fetched through small instruction caches
@@ -570,13 +576,14 @@ __device__ __forceinline__ void visit_ns(const ImgDesc& dd, const CUtensorMap* t
   // The bucket width, read here so that the write-back covers the trip.
   const float inv_width = bucket_inv_width(sch.q, img_idx);
 
-  // Write back (column layout: each row is one coalesced 128-byte store).
-  if (any || first) {
-    if (lane < vw) {
+  // Write back (each row is one coalesced 128-byte store).  A seed visit always does: it may have lowered a pixel that
+  // lowers nothing else.
+  if (any || first || seed) {
+    {
       uint8_t* wb = dist_base(dd, y0, x0 + lane, nph);
 #pragma unroll 4
       for (int y = 0; y < TILE; ++y)
-        if (y < vh) *reinterpret_cast<float*>(wb + (int64_t)y * dd.dist_pitch) = B[y * W_STRIDE + lane];
+        if (y < rows) *reinterpret_cast<float*>(wb + (int64_t)y * dd.dist_pitch) = B[y * W_STRIDE + lane];
     }
   }
   fence_acq_rel();  // release: distances before activations and before the VISITED bit
@@ -876,7 +883,7 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
   const float v = dd.v;
   const RefEdge<FMA> re(dd.l_eucl, dd.l_grad);
 
-  const VisitBufs vb{sm.img, sm.V, sm.V, sm.E, &sm.bar, &sm.bar, 1u, 1u, &parity};
+  const VisitBufs vb{sm.img, sm.V, nullptr, &sm.bar, &sm.bar, 1u, 1u, &parity};
   if (!rerun) stage_tile(vb, tm_img, tm_mask, false, seed, x0, y0);
 
   // Neighbour k = lane (0..7): (dx, dy) = L, R, T, B, TL, TR, BL, BR.

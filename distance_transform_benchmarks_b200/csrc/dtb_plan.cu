@@ -244,7 +244,7 @@ DTB_API dtb_status dtb_plan_create(dtb_context ctx, int32_t n, const dtb_image* 
   p->L = layout_for(n, total, workers, false, NBUCKET_MAX);  // room for every queue policy of the autotuner
   p->L.blocks = count_blocks(p->jobs);
   p->key = tuning_key(n, total);
-  p->tuning = tuning_for(ctx, n, total);
+  p->tuning = tuning_for(ctx, p->jobs, total);
   if (cudaSetDevice(ctx->device) != cudaSuccess) return bail(DTB_ERR_CUDA);
   cudaError_t e = cudaMalloc((void**)&p->dbase, p->L.bytes);
   if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaMalloc(plan scratch)"));
