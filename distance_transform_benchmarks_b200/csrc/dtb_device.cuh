@@ -231,8 +231,8 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap* map) {
 //   pop:  a head ticket in the lowest bucket holding work (or in the base bucket when there is none), then the
 //         popper waits on its own slot only (no shared hot line is polled) until an item or the termination
 //         sentinel arrives; in the bucketed queue a waiter whose item is not reserved gives the ticket back
-//         when another bucket holds work.  Termination: the visit whose completion brings pending to 0 sets
-//         `done` and writes the sentinel into every slot that has a waiting popper.
+//         when another bucket holds work.  Termination: a waiter sees pending == 0 in its periodic check
+//         and leaves; `done` and the sentinels of signal_done_warp end the live kernel, whose pending never settles.
 // Items are interchangeable, so a popper that takes an item meant for another ticket of the same slot is
 // harmless: every item is taken exactly once (atomicExch) and no slot is written twice (CAS from 0).  Each
 // ring holds at least 2 * (tiles + workers) slots, more than items and waiting poppers together.

@@ -28,10 +28,12 @@ constexpr uint64_t DEFAULT_TIMEOUT_NS = 2000000000ull;
 constexpr uint32_t BLOCK_RUN_MAX = 16384;  // blocks of a block kernel run at most (room for its messages)
 constexpr int REF_CTAS = 2;  // resident CTAs per SM of the ref-mode tile kernels (the tile and its edges take 128
                              // registers a thread; 94 KB of shared memory a CTA)
-// ns-mode tile kernel variants: CTAs per SM, whether a warp stages its next tile ahead (17 KB of shared memory a
-// warp instead of 13 KB, so at most 3 CTAs of 4 warps per SM), and warps per CTA.  Registers per thread follow
-// the warps per SM: 8 -> 255, 12 -> 168, 16 -> 128.  The 12- and 16-warp shapes come in several CTA sizes
-// (2 x 6, 3 x 4, 6 x 2; 2 x 8, 4 x 4), which differ in how the SM's warps are grouped and scheduled only.
+// ns-mode tile kernel variants: CTAs per SM, whether a warp stages its next tile ahead (22.4 KB of shared memory a
+// warp instead of 17.8 KB), and warps per CTA.  Registers per thread follow the warps per SM: 8 -> 255, 12 -> 168,
+// 16 -> 128.  The 227 KB of an SM hold 12 warps at 17.8 KB and 8 that stage ahead, so of the shapes with 16 warps 12
+// are resident and 3 x 4 ahead runs as 2 x 4: resident_workers sizes the grid by the occupancy, and saved tuning
+// entries stay valid.  The 12- and 16-warp shapes come in several CTA sizes (2 x 6, 3 x 4, 6 x 2; 2 x 8, 4 x 4), which
+// differ in how the SM's warps are grouped and scheduled only.
 struct NsVariant {
   int ctas;
   bool ahead;
