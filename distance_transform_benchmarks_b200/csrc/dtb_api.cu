@@ -334,7 +334,7 @@ ScratchLayout layout_for(int n, uint32_t total, uint32_t workers, bool rounds, u
   L.nb = std::max<uint32_t>(1u, std::min<uint32_t>(next_pow2(std::max<uint32_t>(buckets, 1u)), NBUCKET_MAX));
   size_t off = 0;
   L.o_hdr = off;    off = align_up(off + sizeof(QueueHdr), 256);
-  L.o_msg = off;    off = align_up(off + 64ull * std::min<uint32_t>(total, BLOCK_RUN_MAX), 256);  // right after the header
+  L.o_msg = off;    off = align_up(off + 32ull * std::min<uint32_t>(total, BLOCK_RUN_MAX), 256);  // right after the header
   L.o_states = off; off = align_up(off + 4ull * std::max<uint32_t>(total, 1), 256);
   L.o_ring = off;   off = align_up(off + L.ring_bytes(), 256);
   L.o_keys = off;   off = align_up(off + (L.nb > 1 ? 4ull * std::max<uint32_t>(total, 1) : 0), 256);
@@ -492,7 +492,7 @@ uint32_t count_blocks(const std::vector<Job>& jobs) {
 // CTAs per SM of the block kernel: with many images (fronts of their own) more blocks in flight pay, with few they only
 // visit blocks too early (2 against 3 CTAs: 48 images of 7 Mpx 0.72 / 0.62 ms, 40 of 15 Mpx 1.44 / 1.25, 24 0.45 / 0.43, 16
 // small ones 0.228 / 0.232, 1333x1999 rgb8 0.43 / 0.44, 4096^2 maze 3.6 / 4.4, a serving burst of 24 2.06 / 2.16).
-static int block_ctas(int mode, int n) { return mode == MODE_NS && n >= 32 ? BLOCK_CTAS_MANY : BLOCK_CTAS; }
+static int block_ctas(int n) { return n >= 32 ? BLOCK_CTAS_MANY : BLOCK_CTAS; }
 static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t, int ctas) {
   return std::max<uint32_t>(1u, (uint32_t)(ctx->num_sms * ctas) * (uint32_t)t.grid_percent / 100u);
 }
@@ -501,14 +501,15 @@ static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t, int ctas) {
 // SMs, 38 Mpx).  Up to there chains of dependent visits bound the run.  ns-mode: the block kernel is faster or as fast
 // (tile against block kernel: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze 4.2 / 4.1,
 // 6016^2 rgb8 1.19 / 1.18, 48 images of 7 Mpx 0.80 / 0.75); with more work than warps the tile kernel's finer units win (128
-// images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5).  ref-mode, lambda 0 / 0.5 / 1: 1023x777 0.40 / 0.69 / 0.91 ms
-// against 0.23 / 0.56 / 0.80, 3648x2432 1.21 / 2.02 / 1.74 against 0.98 / 2.30 / 1.67, 6000^2 2.8 / 4.7 / 3.2 against 2.3 / 5.9 / 2.5.
+// images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5). 
+// ns-mode only: a block kernel for eight neighbours was faster on small pictures (1023x777, lambda 0 / 0.5 / 1: 0.23 / 0.56 /
+// 0.80 ms against 0.40 / 0.69 / 0.91), no faster at lambda 0.5 on large ones (3648x2432 2.30 against 2.02), and stopped once
+// with an illegal instruction whose cause reading did not show, so it was taken out.
 bool use_blocks(dtb_context ctx, int mode, const LaunchTuning& t, uint32_t blocks) {
-  (void)mode;
-  return !t.chosen && blocks > 0 && blocks <= std::min(block_grid(ctx, t, BLOCK_CTAS) * (uint32_t)BLOCK_OWNED_MAX, BLOCK_RUN_MAX);
+  return mode == MODE_NS && !t.chosen && blocks > 0 && blocks <= std::min(block_grid(ctx, t, BLOCK_CTAS) * (uint32_t)BLOCK_OWNED_MAX, BLOCK_RUN_MAX);
 }
 
-dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
+dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, const LaunchTuning& t,
                           cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1) {
   const uint64_t stall_ns = ctx->inject_stall_ns;
   ctx->inject_stall_ns = 0;
@@ -522,27 +523,24 @@ dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& 
   a.total = L.blocks;
   a.max_visits = (uint32_t)std::min<uint64_t>(0xF0000000ull, 4096ull * L.total + (1ull << 20));
   a.timeout_ns = stall_ns ? stall_ns : DEFAULT_TIMEOUT_NS;
-  DTB_CUDA(ctx, cudaMemsetAsync(dbase + L.o_hdr, 0, L.o_msg - L.o_hdr + (mode == MODE_NS ? 32ull : 64ull) * L.blocks, stream));
+  DTB_CUDA(ctx, cudaMemsetAsync(dbase + L.o_hdr, 0, L.o_msg - L.o_hdr + 32ull * L.blocks, stream));
   if (stall_ns) {
     ggdt_phantom_pending<<<1, 1, 0, stream>>>(a.hdr);
     DTB_CUDA(ctx, cudaGetLastError());
   }
   if (ev0) DTB_CUDA(ctx, cudaEventRecord(ev0, stream));
   cudaLaunchConfig_t cfg{};
-  const int ctas = block_ctas(mode, L.n);
+  const int ctas = block_ctas(L.n);
   cfg.gridDim = dim3(std::min<uint32_t>(L.blocks, block_grid(ctx, t, ctas)));
   cfg.blockDim = dim3(BLOCK_WARPS * 32);
-  cfg.dynamicSmemBytes = mode == MODE_NS ? BLOCK_SMEM<MODE_NS> : BLOCK_SMEM<MODE_REF>;
+  cfg.dynamicSmemBytes = BLOCK_SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;  // all CTAs resident: a CTA waits for blocks that the others activate
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const void* fn = mode == MODE_NS ? (ctas == BLOCK_CTAS ? (const void*)ggdt_block<MODE_NS, BLOCK_CTAS>
-                                                         : (const void*)ggdt_block<MODE_NS, BLOCK_CTAS_MANY>)
-                   : mode == MODE_REF ? (const void*)ggdt_block<MODE_REF, BLOCK_CTAS>
-                                      : (const void*)ggdt_block<MODE_REF_NOFMA, BLOCK_CTAS>;
+  const void* fn = ctas == BLOCK_CTAS ? (const void*)ggdt_block<BLOCK_CTAS> : (const void*)ggdt_block<BLOCK_CTAS_MANY>;
   void* args[3] = {(void*)&ddesc, (void*)&dtm, (void*)&a};
   DTB_CUDA(ctx, cudaLaunchKernelExC(&cfg, fn, args));
   if (ev1) DTB_CUDA(ctx, cudaEventRecord(ev1, stream));
@@ -552,7 +550,7 @@ dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& 
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
                               cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, QueueHdr* fold) {
   if (L.total && use_blocks(ctx, mode, t, L.blocks)) {
-    const dtb_status bs = enqueue_blocks(ctx, dbase, L, mode, t, stream, ev0, ev1);
+    const dtb_status bs = enqueue_blocks(ctx, dbase, L, t, stream, ev0, ev1);
     if (bs != DTB_OK || !fold) return bs;
     ggdt_finalize<<<1, 32, 0, stream>>>(nullptr, nullptr, 0, 0, nullptr, reinterpret_cast<const QueueHdr*>(dbase + L.o_hdr), fold);
     DTB_CUDA(ctx, cudaGetLastError());
@@ -946,16 +944,13 @@ DTB_API dtb_status dtb_context_create(int32_t device, dtb_context* out) {
   }
   const struct {
     const void* fn;
-    size_t smem;
     int ctas;
-  } block_fns[4] = {{(const void*)ggdt_block<MODE_NS, BLOCK_CTAS>, BLOCK_SMEM<MODE_NS>, BLOCK_CTAS},
-                    {(const void*)ggdt_block<MODE_NS, BLOCK_CTAS_MANY>, BLOCK_SMEM<MODE_NS>, BLOCK_CTAS_MANY},
-                    {(const void*)ggdt_block<MODE_REF, BLOCK_CTAS>, BLOCK_SMEM<MODE_REF>, BLOCK_CTAS},
-                    {(const void*)ggdt_block<MODE_REF_NOFMA, BLOCK_CTAS>, BLOCK_SMEM<MODE_REF>, BLOCK_CTAS}};
+  } block_fns[2] = {{(const void*)ggdt_block<BLOCK_CTAS>, BLOCK_CTAS},
+                    {(const void*)ggdt_block<BLOCK_CTAS_MANY>, BLOCK_CTAS_MANY}};
   for (const auto& f : block_fns) {
     int bps = 0;
-    ok = ok && cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, f.fn, BLOCK_WARPS * 32, f.smem) == cudaSuccess && bps >= f.ctas;
+    ok = ok && cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLOCK_SMEM) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, f.fn, BLOCK_WARPS * 32, BLOCK_SMEM) == cudaSuccess && bps >= f.ctas;
   }
   int ref_bps_nofma = 0;
   ok = ok && cudaFuncSetAttribute(kref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REF_SMEM) == cudaSuccess &&

@@ -20,7 +20,6 @@ constexpr int BLOCK_OWNED_MAX = 32;                // blocks of one CTA at most
 // Rounds a tile runs before its neighbours look at it: two complete a full sweep (1 and 3 were 25 % and 8 % slower on
 // 2048^2 gray).
 constexpr int BLOCK_ROUNDS = 2;
-constexpr uint32_t BLOCK_PHASES = 2;  // ref-mode: likewise, one phase per layout
 
 struct alignas(128) BlockTile {
   uint8_t img[IMG_REGION];   // image box, then the tile buffer B[y * 34 + x]
@@ -30,46 +29,39 @@ struct alignas(128) BlockTile {
   float H[4 * TILE];          // halo of the sides that lie on the block's border (INF on the others), per side
   uint64_t bar;
 };
-// Sides of a block: left, right, top, bottom, and in ref-mode (8 neighbours) the corners tl, tr, bl, br.
-constexpr int BLOCK_SIDES_MAX = 8;
-template <int MODE>
-constexpr int BLOCK_SIDES = MODE == MODE_NS ? 4 : 8;
+constexpr int BLOCK_SIDES = 4;  // left, right, top, bottom
 // Offset to the neighbour on side k (tables as bit masks: no array in local memory), and the side it sees us on.
-__device__ __forceinline__ int side_dx(int k) { return (0xF3 >> k) & 1 ? ((0xA2 >> k) & 1 ? 1 : -1) : 0; }
-__device__ __forceinline__ int side_dy(int k) { return (0xFC >> k) & 1 ? ((0xC8 >> k) & 1 ? 1 : -1) : 0; }
-__device__ __forceinline__ int side_back(int k) { return k < 4 ? k ^ 1 : 11 - k; }
+__device__ __forceinline__ int side_dx(int k) { return (0x3 >> k) & 1 ? ((0x2 >> k) & 1 ? 1 : -1) : 0; }
+__device__ __forceinline__ int side_dy(int k) { return (0xC >> k) & 1 ? ((0x8 >> k) & 1 ? 1 : -1) : 0; }
+__device__ __forceinline__ int side_back(int k) { return k ^ 1; }
 
 struct BlockCtl {
   uint32_t owned_img[BLOCK_OWNED_MAX];
-  uint32_t sent[BLOCK_OWNED_MAX][BLOCK_SIDES_MAX];  // activations sent over each side of the owned blocks
-  uint32_t seen[BLOCK_SIDES_MAX][BLOCK_OWNED_MAX];  // activations answered, per side
+  uint32_t sent[BLOCK_OWNED_MAX][BLOCK_SIDES];  // activations sent over each side of the owned blocks
+  uint32_t seen[BLOCK_SIDES][BLOCK_OWNED_MAX];  // activations answered, per side
   uint32_t visited[BLOCK_OWNED_MAX / 32];  // bit i: owned block i has been visited
   uint32_t seeded[BLOCK_OWNED_MAX / 32];   // bit i: owned block i holds seeds not applied yet
   uint32_t next;       // index of the owned block to visit, or POP_NONE
   uint32_t first, seed, rerun;  // of this visit: no earlier visit; apply seeds; shared memory holds the block
   uint32_t nvis;       // bit k: the neighbouring block on side k holds valid distances
   uint32_t tokens;     // tokens the visit gives back at its end
-  uint32_t side[BLOCK_SIDES_MAX];  // smallest value each side can bring to the neighbouring block (float bits), KEY_NONE if none
+  uint32_t side[BLOCK_SIDES];  // smallest value each side can bring to the neighbouring block (float bits), KEY_NONE if none
   uint32_t visits;     // tiles swept in this visit
   uint32_t phases, activations;  // counters of the run
   ImgDesc desc;        // the block's image
 };
-template <int MODE>
 struct BlockSmem {
-  std::conditional_t<MODE == MODE_NS, BlockTile, RefTile> tile[BLOCK_WARPS];
+  BlockTile tile[BLOCK_WARPS];
   BlockCtl ctl;
 };
-template <int MODE>
-constexpr size_t BLOCK_SMEM = sizeof(BlockSmem<MODE>) + 128;
-static_assert(BLOCK_CTAS_MANY * (BLOCK_SMEM<MODE_NS> + 1024) <= 228 * 1024 && BLOCK_CTAS * (BLOCK_SMEM<MODE_REF> + 1024) <= 228 * 1024,
-              "the blocks of an SM must fit its shared memory");
+constexpr size_t BLOCK_SMEM = sizeof(BlockSmem) + 128;
+static_assert(BLOCK_CTAS_MANY * (BLOCK_SMEM + 1024) <= 228 * 1024, "the blocks of an SM must fit its shared memory");
 
 // Device words of a run.
 struct BlockRun {
   QueueHdr* hdr;         // pending: tokens in use less `total`; the run has ended when all are back.  Every block starts
                          // out with one token, every activation under way carries one, and a visit holds four more
-                         // (ref-mode: eight) from its start for those it may send: so the count never reaches zero
-                         // early.
+                         // from its start for those it may send: so the count never reaches zero early.
   uint2* msg;            // per block and side, from the neighbour there: x = 2 * activations sent + 1 (0: the neighbour
                          // has not been visited), y = the smallest value the last one brings (float bits)
   const uint32_t* base;  // block prefix of the images
@@ -88,7 +80,6 @@ __device__ __forceinline__ uint4 ld_volatile4(const uint4* p) {
 // Waits until one of the CTA's blocks is to be visited and claims it (warp 0).  The block visited last comes first
 // (its visit needs no staging), then the one with the smallest activation value.  Bounded: end of the run / error /
 // watchdog.
-template <int SIDES>
 __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __restrict__ descs, BlockCtl& ctl, uint32_t first,
                                            uint32_t step, int count, uint32_t prev) {
   const int lane = threadIdx.x & 31;
@@ -96,14 +87,14 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
   uint32_t last = ld_volatile(&a.hdr->progress.v);
   for (;;) {
     // Each lane looks at every 32nd block: its best one, and the messages of that.
-    uint32_t key = KEY_NONE, pick = POP_NONE, got[SIDES] = {};
+    uint32_t key = KEY_NONE, pick = POP_NONE, got[BLOCK_SIDES] = {};
     bool stop = ld_volatile(&a.hdr->pending.v) + a.total == 0u;
 #pragma unroll 4
     for (int i = lane; i < count; i += 32) {
-      const uint4* mine = reinterpret_cast<const uint4*>(a.msg + (uint64_t)SIDES * (first + (uint32_t)i * step));
-      uint4 m[SIDES / 2];
+      const uint4* mine = reinterpret_cast<const uint4*>(a.msg + (uint64_t)BLOCK_SIDES * (first + (uint32_t)i * step));
+      uint4 m[BLOCK_SIDES / 2];
 #pragma unroll
-      for (int s = 0; s < SIDES / 2; ++s) m[s] = ld_volatile4(mine + s);
+      for (int s = 0; s < BLOCK_SIDES / 2; ++s) m[s] = ld_volatile4(mine + s);
       uint32_t k = KEY_NONE;
       bool ready = false;
       auto side = [&](uint32_t x, uint32_t y, int s) {
@@ -113,7 +104,7 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
         }
       };
 #pragma unroll
-      for (int s = 0; s < SIDES / 2; ++s) {
+      for (int s = 0; s < BLOCK_SIDES / 2; ++s) {
         side(m[s].x, m[s].y, 2 * s);
         side(m[s].z, m[s].w, 2 * s + 1);
       }
@@ -125,7 +116,7 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
         key = k;
         pick = (uint32_t)i;
 #pragma unroll
-        for (int s = 0; s < SIDES / 2; ++s) {
+        for (int s = 0; s < BLOCK_SIDES / 2; ++s) {
           got[2 * s] = m[s].x;
           got[2 * s + 1] = m[s].z;
         }
@@ -144,10 +135,10 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
         __syncwarp();
       }
       if (lane == win) {
-        atomicAdd(&a.hdr->pending.v, (uint32_t)SIDES);
+        atomicAdd(&a.hdr->pending.v, (uint32_t)BLOCK_SIDES);
         uint32_t fresh = 0, nvis = 0;
 #pragma unroll
-        for (int s = 0; s < SIDES; ++s) {
+        for (int s = 0; s < BLOCK_SIDES; ++s) {
           fresh += (got[s] >> 1) - ctl.seen[s][pick];
           nvis |= (got[s] ? 1u : 0u) << s;
           ctl.seen[s][pick] = got[s] >> 1;
@@ -156,7 +147,7 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
         const bool warm = ctl.desc.warm != 0;
         ctl.nvis = warm ? ~0u : nvis;
         ctl.next = pick;
-        ctl.tokens = (uint32_t)SIDES + fresh + (seed ? 1u : 0u);
+        ctl.tokens = (uint32_t)BLOCK_SIDES + fresh + (seed ? 1u : 0u);
         ctl.seed = seed ? 1u : 0u;
         ctl.first = warm || (ctl.visited[pick >> 5] & bit) ? 0u : 1u;
         ctl.rerun = pick == prev && !seed ? 1u : 0u;
@@ -196,14 +187,13 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
 
 // End of a visit of block `blk` (warp 0, after the CTA's barrier): each side's lane tells the neighbouring block there, if
 // there is one, that this block has been visited, and activates it if the visit found a value to bring (ctl.side).
-template <int SIDES>
 __device__ __forceinline__ void block_complete(const BlockRun& a, BlockCtl& ctl, uint32_t blk) {
   const int lane = threadIdx.x & 31;
   const ImgDesc& dd = ctl.desc;
   const int bxn = dd.blocks_x, local = (int)(blk - dd.block_base), bx = local % bxn, by = local / bxn;
-  const int nx = bx + side_dx(lane & 7), ny = by + side_dy(lane & 7);
-  const bool exists = lane < SIDES && nx >= 0 && nx < bxn && ny >= 0 && ny < dd.blocks_y;
-  const uint32_t key = lane < SIDES ? ctl.side[lane] : KEY_NONE;
+  const int nx = bx + side_dx(lane & 3), ny = by + side_dy(lane & 3);
+  const bool exists = lane < BLOCK_SIDES && nx >= 0 && nx < bxn && ny >= 0 && ny < dd.blocks_y;
+  const uint32_t key = lane < BLOCK_SIDES ? ctl.side[lane] : KEY_NONE;
   const bool want = exists && key != KEY_NONE;
   fence_acq_rel();  // release: the CTA's distances (and the visit's spare tokens) before the messages
   const uint32_t nsent = __popc(__ballot_sync(~0u, want));
@@ -211,11 +201,11 @@ __device__ __forceinline__ void block_complete(const BlockRun& a, BlockCtl& ctl,
     const uint32_t nb = dd.block_base + (uint32_t)(ny * bxn + nx);
     const uint32_t n = ctl.sent[ctl.next][lane] + (want ? 1u : 0u);
     ctl.sent[ctl.next][lane] = n;
-    asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(a.msg + (uint64_t)SIDES * nb + side_back(lane)), "r"(2u * n + 1u),
+    asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(a.msg + (uint64_t)BLOCK_SIDES * nb + side_back(lane)), "r"(2u * n + 1u),
                  "r"(key)
                  : "memory");
   }
-  if (lane < SIDES) ctl.side[lane] = KEY_NONE;
+  if (lane < BLOCK_SIDES) ctl.side[lane] = KEY_NONE;
   if (lane == 0) {
     atomicSub(&a.hdr->pending.v, ctl.tokens - nsent);
     atomicAdd(&a.hdr->progress.v, max(ctl.visits, 1u));
@@ -316,37 +306,6 @@ __device__ __forceinline__ bool block_fill_ns(const ImgDesc& dd, const BlockPlac
   return __any_sync(~0u, low);
 }
 
-template <bool FMA>
-__device__ __forceinline__ bool block_fill_ref(const RefEdge<FMA>& re, const ImgDesc& dd, const BlockPlace& p, RefTile& t, bool first,
-                                               bool seed, const float (&d)[TILE]) {
-  const int lane = threadIdx.x & 31;
-  const float INF = f_inf();
-  float* T = reinterpret_cast<float*>(t.img);
-  uint32_t seeds = 0;  // this lane's column of the mask tile
-  if (seed) {
-    const uint8_t* mbox = reinterpret_cast<const uint8_t*>(t.V);
-#pragma unroll 4
-    for (int y = 0; y < TILE; ++y) seeds |= (lane < p.vw && y < p.vh && mbox[y * TILE + lane] != 0 ? 1u : 0u) << y;
-  }
-  __syncwarp();
-  ref_tile_weights<FMA>(re, p.vw, p.vh, t);
-  __syncwarp();
-  if (first) {
-    const float v = dd.v;
-#pragma unroll 4
-    for (int y = 0; y < TILE; ++y) T[y * RS + lane] = (lane < p.vw && y < p.vh) ? (((seeds >> y) & 1u) ? 0.0f : v) : INF;
-    return __any_sync(~0u, seeds != 0u);
-  }
-  bool low = false;
-#pragma unroll
-  for (int y = 0; y < TILE; ++y) {
-    const bool s = ((seeds >> y) & 1u) != 0u;
-    low |= s && d[y] > 0.0f;
-    T[y * RS + lane] = s ? 0.0f : d[y];
-  }
-  return __any_sync(~0u, low);
-}
-
 // A warp's flags: bit 0 the phase parity of its mbarrier; its tile of the block visited last differs from memory.
 constexpr uint32_t BLOCK_UNSAVED = 2u;
 
@@ -357,7 +316,7 @@ constexpr uint32_t BLOCK_UNSAVED = 2u;
 // neighbour's border while the neighbour lowers it: values only decrease and each is one word, and the visit ends
 // only after an iteration in which no tile changed.  Only the lines on the block's border are written to memory; the
 // tiles stay in shared memory and are written when the CTA turns to another block (BLOCK_UNSAVED) or ends.
-__device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem<MODE_NS>& sm,
+__device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem& sm,
                                                uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, float (&wh)[TILE],
                                                float (&wv)[TILE], int& loaded, bool fill_only) {
   const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
@@ -497,134 +456,14 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
     atomicAdd(&sm.ctl.phases, nph);
   }
   __syncthreads();
-  if (warp == 0) block_complete<BLOCK_SIDES<MODE_NS>>(a, sm.ctl, blk);
+  if (warp == 0) block_complete(a, sm.ctl, blk);
 }
 
-// The ref-mode visit of a block: as block_visit_ns, with eight neighbours and phases (ref_solve) in place of rounds, two
-// of them (one per layout) before the neighbours look again.
-template <bool FMA>
-__device__ __forceinline__ void block_visit_ref(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem<MODE_REF>& sm,
-                                                uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, bool fill_only) {
-  const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
-  const int wx = warp % BLOCK_TX, wy = warp / BLOCK_TX;
-  const float INF = f_inf();
-  const ImgDesc& dd = sm.ctl.desc;
-  const RefEdge<FMA> re(dd.l_eucl, dd.l_grad);
-  RefTile& t = sm.tile[warp];
-  float* T = reinterpret_cast<float*>(t.img);
-  const bool first = uniform(sm.ctl.first != 0u);
-  const BlockPlace p = block_place(dd, blk);
-  const bool exists = uniform((p.sides >> 12) != 0u);
-  // The lines that neighbouring blocks read: the sides with one beyond, and (corners) the whole left and top border.
-  const uint32_t outer = ((p.sides >> 8) & 15u) | (wx == 0 ? 1u : 0u) | (wy == 0 ? 4u : 0u);
-  bool todo = false, changed = false;
-  // Side k of the tile: the neighbouring tile in this block, or the side of the block it lies beyond.
-  auto in_block = [&](int k) {
-    const int nx = wx + side_dx(k), ny = wy + side_dy(k);
-    return nx >= 0 && nx < BLOCK_TX && ny >= 0 && ny < BLOCK_TY;
-  };
-  {
-    const bool seed = uniform(sm.ctl.seed != 0u), rerun = uniform(sm.ctl.rerun != 0u);
-    const VisitBufs vb{t.img, t.V, nullptr, &t.bar, &t.bar, 1u, 1u, &flags};
-    if (exists && !rerun) stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, false, seed, p.x0, p.y0);
-    {
-      // The halo on the block's border.
-      const uint32_t nvis = sm.ctl.nvis;
-      const float v = dd.v;
-      auto value = [&](int k, int gx, int gy) -> float {
-        if (!exists || in_block(k) || gx < 0 || gy < 0 || gx >= dd.width || gy >= dd.height) return INF;
-        const int nx = wx + side_dx(k), ny = wy + side_dy(k);
-        const int ox = nx < 0 ? -1 : nx >= BLOCK_TX ? 1 : 0, oy = ny < 0 ? -1 : ny >= BLOCK_TY ? 1 : 0;
-        const int side = oy == 0 ? (ox < 0 ? 0 : 1) : ox == 0 ? (oy < 0 ? 2 : 3) : 4 + (oy > 0 ? 2 : 0) + (ox > 0 ? 1 : 0);
-        return ((nvis >> side) & 1u) ? ld_dist(dd, gy, gx) : v;
-      };
-      const float hl = value(0, p.x0 - 1, p.y0 + lane), hr = value(1, p.x0 + TILE, p.y0 + lane);
-      const float ht = value(2, p.x0 + lane, p.y0 - 1), hb = value(3, p.x0 + lane, p.y0 + TILE);
-      const float hc = lane < 4 ? value(4 + lane, p.x0 + ((lane & 1) ? TILE : -1), p.y0 + ((lane & 2) ? TILE : -1)) : INF;
-      t.H[E_LEFT + lane] = hl;
-      t.H[E_RIGHT + lane] = hr;
-      t.H[E_TOP + lane] = ht;
-      t.H[E_BOTTOM + lane] = hb;
-      if (lane < 4) t.H[4 * TILE + lane] = hc;
-    }
-    const bool fill = exists && !rerun;
-    float td[TILE];
-    if (fill && !first) block_load_tile(dd, p, td);
-    tma_wait(&t.bar, flags, 1u, q, blk, fill);
-    if (uniform(fill)) todo = changed = block_fill_ref<FMA>(re, dd, p, t, first, seed, td);
-    if (fill_only) {
-      __syncthreads();
-      return;
-    }
-    if (first) flags |= BLOCK_UNSAVED;
-  }
-  uint32_t nph = 0;
-  bool col = true;
-  __syncthreads();  // every tile of the block is in place
-  for (uint32_t it = 0;; ++it) {
-    if (exists) {
-      // The halo: a neighbour's border in shared memory (tiles outside the image do not exist there either: H is INF), or H.
-      const bool exl = (p.sides & 1u) != 0u, exr = (p.sides & 2u) != 0u, ext = (p.sides & 4u) != 0u, exb = (p.sides & 8u) != 0u;
-      auto tileT = [&](int k) -> const volatile float* {
-        return reinterpret_cast<const volatile float*>(sm.tile[warp + side_dx(k) + side_dy(k) * BLOCK_TX].img);
-      };
-      RefHalo h;
-      h.l = exl && in_block(0) ? tileT(0)[lane * RS + TILE - 1] : t.H[E_LEFT + lane];
-      h.r = exr && in_block(1) ? tileT(1)[lane * RS] : t.H[E_RIGHT + lane];
-      h.t = ext && in_block(2) ? tileT(2)[(TILE - 1) * RS + lane] : t.H[E_TOP + lane];
-      h.b = exb && in_block(3) ? tileT(3)[lane] : t.H[E_BOTTOM + lane];
-      h.tl = exl && ext && in_block(4) ? tileT(4)[(TILE - 1) * RS + TILE - 1] : t.H[4 * TILE];
-      h.tr = exr && ext && in_block(5) ? tileT(5)[(TILE - 1) * RS] : t.H[4 * TILE + 1];
-      h.bl = exl && exb && in_block(6) ? tileT(6)[TILE - 1] : t.H[4 * TILE + 2];
-      h.br = exr && exb && in_block(7) ? tileT(7)[0] : t.H[4 * TILE + 3];
-      if (ref_halo_relax<FMA>(re, T, t.E, h, p.vw, p.vh)) todo = true;
-    }
-    if (!__syncthreads_or(todo ? 1 : 0)) break;
-    if (uniform(todo)) {
-      changed = true;
-      bool fell = false;
-      todo = ref_solve<FMA>(re, t, col, BLOCK_PHASES, nph, fell);
-      block_store_border(dd, p, outer, T, RS);  // at once, as in block_visit_ns
-    }
-    if (it >= (uint32_t)PHASE_LIMIT) {
-      if (threadIdx.x == 0) set_error(q, DERR_PHASE_LIMIT, blk);
-      break;
-    }
-    __syncthreads();
-  }
-
-  // What the block's border can bring to its neighbours, and the border lines to memory.
-  if (changed) flags |= BLOCK_UNSAVED;
-  if (uniform(exists && (changed || first))) {
-    if (!nph) block_store_border(dd, p, outer, T, RS);
-    // Neighbours in the block have an INF halo in H: every finite value would beat it, so they are masked out.
-    const RefHalo h{t.H[E_LEFT + lane], t.H[E_RIGHT + lane], t.H[E_TOP + lane],  t.H[E_BOTTOM + lane],
-                    t.H[4 * TILE],      t.H[4 * TILE + 1],   t.H[4 * TILE + 2], t.H[4 * TILE + 3]};
-    const uint32_t k = ref_border_keys<FMA>(re, T, t.E, h);
-    if (lane < 8 && k != KEY_NONE && !in_block(lane)) {
-      const int gx = p.x0 / TILE + side_dx(lane), gy = p.y0 / TILE + side_dy(lane);
-      if (gx >= 0 && gy >= 0 && gx < dd.tiles_x && gy < dd.tiles_y) {
-        const int nx = wx + side_dx(lane), ny = wy + side_dy(lane);
-        const int ox = nx < 0 ? -1 : nx >= BLOCK_TX ? 1 : 0, oy = ny < 0 ? -1 : ny >= BLOCK_TY ? 1 : 0;
-        const int side = oy == 0 ? (ox < 0 ? 0 : 1) : ox == 0 ? (oy < 0 ? 2 : 3) : 4 + (oy > 0 ? 2 : 0) + (ox > 0 ? 1 : 0);
-        atomicMin(&sm.ctl.side[side], k);
-      }
-    }
-  }
-  if (nph && lane == 0) {
-    atomicAdd(&sm.ctl.visits, 1u);
-    atomicAdd(&sm.ctl.phases, nph);
-  }
-  __syncthreads();
-  if (warp == 0) block_complete<BLOCK_SIDES<MODE_REF>>(a, sm.ctl, blk);
-}
-
-template <int MODE, int CTAS>
+template <int CTAS>
 __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
     ggdt_block(const ImgDesc* __restrict__ descs, const CUtensorMap* __restrict__ tmaps, BlockRun a) {
   extern __shared__ uint8_t smem_raw[];
-  constexpr int KIND = MODE == MODE_NS ? MODE_NS : MODE_REF;
-  BlockSmem<KIND>& sm = *reinterpret_cast<BlockSmem<KIND>*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  BlockSmem& sm = *reinterpret_cast<BlockSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
   const uint32_t first = blockIdx.x, step = gridDim.x;
   const int count = (int)((a.total - first + step - 1) / step);
@@ -634,10 +473,10 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
     mbar_init(&sm.tile[warp].bar, 1);
     fence_mbar_init();
   }
-  for (int i = threadIdx.x; i < BLOCK_OWNED_MAX * BLOCK_SIDES_MAX; i += BLOCK_WARPS * 32) (&sm.ctl.sent[0][0])[i] = (&sm.ctl.seen[0][0])[i] = 0;
+  for (int i = threadIdx.x; i < BLOCK_OWNED_MAX * BLOCK_SIDES; i += BLOCK_WARPS * 32) (&sm.ctl.sent[0][0])[i] = (&sm.ctl.seen[0][0])[i] = 0;
   for (int i = threadIdx.x; i < BLOCK_OWNED_MAX / 32; i += BLOCK_WARPS * 32) sm.ctl.seeded[i] = sm.ctl.visited[i] = 0;
   for (int i = threadIdx.x; i < count; i += BLOCK_WARPS * 32) sm.ctl.owned_img[i] = image_of_tile(a.base, a.n, first + (uint32_t)i * step);
-  if (threadIdx.x < BLOCK_SIDES_MAX) sm.ctl.side[threadIdx.x] = KEY_NONE;
+  if (threadIdx.x < BLOCK_SIDES) sm.ctl.side[threadIdx.x] = KEY_NONE;
   if (threadIdx.x == 0) sm.ctl.visits = sm.ctl.phases = sm.ctl.activations = 0;
   __syncthreads();
   // Seed scan of the owned blocks: one warp per tile, lane = row, the rows of several blocks in flight.
@@ -660,7 +499,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
     if (lane == 0) atomicSub(&a.hdr->pending.v, (uint32_t)count - seeded);
   }
   uint32_t flags = 0, prev = POP_NONE;
-  float wh[TILE], wv[TILE];  // ns-mode: the tile's weights, in the layout `loaded`
+  float wh[TILE], wv[TILE];  // the tile's weights, in the layout `loaded`
   int loaded = -1;
   // The first block without seeds is filled before anything activates it, so that its first visit finds it in place: with
   // one block per CTA that takes 8,000 (gray) to 12,000 (rgb8) cycles off every step of the front into new blocks.
@@ -680,21 +519,17 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
     early = -1;
   }
   for (;;) {
-    if (early < 0 && warp == 0) block_next<BLOCK_SIDES<MODE>>(a, descs, sm.ctl, first, step, count, prev);
+    if (early < 0 && warp == 0) block_next(a, descs, sm.ctl, first, step, count, prev);
     __syncthreads();
     const uint32_t next = uniform(sm.ctl.next);
     if (next != prev && (flags & BLOCK_UNSAVED)) {
       const ImgDesc& dd = descs[sm.ctl.owned_img[prev]];
-      block_store_tile(dd, block_place(dd, first + prev * step), reinterpret_cast<const float*>(sm.tile[warp].img),
-                       MODE == MODE_NS ? W_STRIDE : RS);
+      block_store_tile(dd, block_place(dd, first + prev * step), reinterpret_cast<const float*>(sm.tile[warp].img), W_STRIDE);
       flags &= ~BLOCK_UNSAVED;
       __syncwarp();
     }
     if (next == POP_NONE) break;
-    if constexpr (MODE == MODE_NS)
-      block_visit_ns(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, wh, wv, loaded, early >= 0);
-    else
-      block_visit_ref<MODE == MODE_REF>(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, early >= 0);
+    block_visit_ns(a, tmaps, sm, sm.ctl.owned_img[next], first + next * step, flags, q, wh, wv, loaded, early >= 0);
     prev = next;
     early = -1;
   }

@@ -136,7 +136,7 @@ struct alignas(128) WarpSmem {
   uint32_t keep;                            // tile this warp keeps for its next visit (POP_NONE: none)
 };
 
-// Per-warp shared memory of a ref-mode visit (23.6 KB: 8 warps per SM).  The edge words (|dI|, or l_grad * |dI| without
+// Per-warp shared memory of a ref-mode visit (23.3 KB: 8 warps per SM).  The edge words (|dI|, or l_grad * |dI| without
 // FMA; INF where there is no edge inside the tile) and the tile keep 33 floats a row: conflict-free with a lane per
 // column and with a lane per row.
 constexpr int RS = TILE + 1;
@@ -148,7 +148,6 @@ struct alignas(128) RefTile {
   float DR[(TILE + 1) * RS];    // (x + 1, y - 1) - (x, y)
   float E[12 * TILE];           // edges to the halo: side (as E_LEFT..), offset -1, 0, 1 along it, position
   float B0[4 * TILE];           // host-driven rounds: the border before the visit
-  float H[4 * TILE + 4];        // block kernel: halo on the block's border (INF elsewhere), sides, then corners
   uint64_t bar;
   uint32_t keep;
 };

@@ -238,7 +238,7 @@ uint32_t resident_workers(dtb_context ctx, int mode, const LaunchTuning& t);
 dtb_status enqueue_persistent(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
                               cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, QueueHdr* fold = nullptr);
 // Enqueues a run of the block kernel: one memset (header and messages) and one launch.
-dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, int mode, const LaunchTuning& t,
+dtb_status enqueue_blocks(dtb_context ctx, uint8_t* dbase, const ScratchLayout& L, const LaunchTuning& t,
                           cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1);
 // Enqueues the cooperative persistent tile kernel of `mode` under `t` (grid: resident_workers / PERSIST_WPC).
 dtb_status launch_tile_kernel(dtb_context ctx, int mode, const LaunchTuning& t, const ImgDesc* descs,

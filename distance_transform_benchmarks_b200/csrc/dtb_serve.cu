@@ -563,7 +563,7 @@ dtb_status launch_wave(dtb_server s, InFlight& f) {
   }
   if (blocks) {
     // The block kernel scans the masks itself: a warm image's old seeds are 0 in its map already and ask for nothing.
-    const dtb_status bs = enqueue_blocks(ctx, sc, L, MODE_NS, tuning, st, nullptr, nullptr);
+    const dtb_status bs = enqueue_blocks(ctx, sc, L, tuning, st, nullptr, nullptr);
     if (bs != DTB_OK) return bs;
   } else if (total > 0) {
     const uint32_t scan_blocks = std::min<uint32_t>((total + 3) / 4, (uint32_t)ctx->num_sms * 16);
