@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
       visit_tile<MODE>(descs[img], tmaps, img, t, old, sm, parity, sch, ws,
                        again && (old & ST_VISITED) && !(old & ST_SEED));
     }
+    if (uniform((parity & STAGE_LOST) != 0u)) break;
   }
   flush_stats(ws, q);
 }
@@ -133,6 +134,10 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
     uint32_t nph, nact;
     visit_ns<true>(dd, tmaps + 2 * img, tmaps + 2 * img + 1, cur, old, vb, sch, &nph, &nact);
     count_visit(ws, q, nph, nact);
+    if (uniform((pbits & STAGE_LOST) != 0u)) {
+      if (nxt != POP_NONE) tma_wait(&sm.bar[k ^ 1u], pbits, 2u >> k, q, nxt);  // the box in flight lands before the warp leaves
+      break;
+    }
     if (nxt == POP_NONE) {
       nxt = queue_pop(q);
       if (nxt != POP_NONE) stage_ahead(descs, tmaps, states, nxt, sm.box[k ^ 1u], &sm.bar[k ^ 1u]);

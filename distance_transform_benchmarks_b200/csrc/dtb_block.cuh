@@ -96,7 +96,7 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
     uint32_t key = KEY_NONE, pick = POP_NONE, got[BLOCK_SIDES] = {};
     bool stop = ld_volatile(&a.hdr->pending.v) + a.total == 0u;
     // After an error no block is claimed any more, ready or not.  The word is on a line that nobody writes, so its load
-    // comes back with the messages' (with the check of the image index below, 512^2 gray takes 159.7 us instead of 158.8 and the
+    // comes back with the messages' (with the checks of the visit below, 512^2 gray takes 159.7 us instead of 158.8 and the
     // 4096^2 maze 3.65 ms instead of 3.63).
     const uint32_t failed = ld_volatile(&a.hdr->error.v);
 #pragma unroll 4
@@ -333,7 +333,8 @@ constexpr uint32_t BLOCK_UNSAVED = 2u;
 // neighbour's border while the neighbour lowers it: values only decrease and each is one word, and the visit ends
 // only after an iteration in which no tile changed.  Only the lines on the block's border are written to memory; the
 // tiles stay in shared memory and are written when the CTA turns to another block (BLOCK_UNSAVED) or ends.
-__device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem& sm,
+// Returns false when a copy into the block's tiles did not arrive: the CTA then visits nothing more (STAGE_LOST).
+__device__ __forceinline__ bool block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem& sm,
                                                uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, float (&wh)[TILE],
                                                float (&wv)[TILE], int& loaded, bool fill_only) {
   const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
@@ -371,18 +372,16 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
     const bool fill = exists && !rerun;
     float td[TILE];
     if (fill && !first) block_load_tile(dd, p, td);
-    tma_wait(&t.bar, flags, 1u, q, blk, fill);
-    if (uniform(fill)) todo = changed = block_fill_ns(dd, p, t, first, seed, td);
+    const bool staged = tma_wait(&t.bar, flags, 1u, q, blk, fill);
+    if (uniform(fill) && staged) todo = changed = block_fill_ns(dd, p, t, first, seed, td);
     if (!rerun) loaded = -1;
-    if (fill_only) {
-      __syncthreads();  // ctl is block_next's from here on
-      return;
-    }
+    // Every tile of the block is in place; with fill_only, ctl is block_next's from here on.
+    if (__syncthreads_or(staged ? 0 : 1)) return false;
+    if (fill_only) return true;
     if (first) flags |= BLOCK_UNSAVED;
   }
   uint32_t nph = 0;
   float d[TILE];
-  __syncthreads();  // every tile of the block is in place
   for (uint32_t it = 0;; ++it) {
     bool layout_a = true;
     asm volatile("" : "+r"(sides));  // keeps the addresses below from being held in registers through the rounds
@@ -474,6 +473,7 @@ __device__ __forceinline__ void block_visit_ns(const BlockRun& a, const CUtensor
   }
   __syncthreads();
   if (warp == 0) block_complete(a, sm.ctl, blk);
+  return true;
 }
 
 template <int CTAS>
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
       if (threadIdx.x == 0) block_error(a, DERR_BAD_TILE, next);
       break;
     }
-    block_visit_ns(a, tmaps, sm, img, first + next * step, flags, q, wh, wv, loaded, early >= 0);
+    if (!block_visit_ns(a, tmaps, sm, img, first + next * step, flags, q, wh, wv, loaded, early >= 0)) break;
     prev = next;
     early = -1;
   }

@@ -589,6 +589,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) ggdt_live(LiveArgs a) {
     visit_ns<false>(dd, a.tmaps + 2 * slot, a.tmaps + 2 * slot + 1, it, old, visit_bufs(sm, parity), sch, &nph, &nact,
                     again && (old & ST_VISITED) && !(old & ST_SEED));
     count_visit(ws, a.q, nph, nact);
+    if (uniform((parity & STAGE_LOST) != 0u)) break;
   }
   flush_stats(ws, a.q);
 }

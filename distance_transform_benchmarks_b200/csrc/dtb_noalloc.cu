@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(NOALLOC_WPC * 32, NOALLOC_MINB) noalloc_persis
     const uint32_t old = sch.claim(t);
     const ImgDesc dd = *na_desc();
     visit_tile<MODE_NS>(dd, na_tmaps(), 0u, t, old, sm, parity, sch, ws);
+    if (uniform((parity & STAGE_LOST) != 0u)) break;
   }
   flush_stats(ws, q);
 }

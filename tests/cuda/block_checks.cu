@@ -1,5 +1,5 @@
-// Checks of the block kernel that need its own launch words: runs that begin with an error word or with a small visit cap.
-// Built by tests/test_gpu_block_failure.py.
+// Checks of the block kernel that need its own launch words: runs that begin with an error word or with a small visit cap,
+// and a wait for a copy that nobody issued.  Built by tests/test_gpu_block_failure.py.
 #include <cstdint>
 #include <cstring>
 #include <cuda.h>
@@ -26,6 +26,23 @@ bool encode(CUtensorMap* tm, const void* base, uint64_t w, uint64_t h, uint64_t 
   return fn && fn(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+__global__ void wait_for_nothing(QueueHdr* hdr, uint32_t* out) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+  }
+  __syncwarp();
+  Queue q{};
+  q.hdr = hdr;
+  uint32_t bits = 0;
+  const bool ok = tma_wait(&bar, bits, 1u, q, 77u);
+  if (threadIdx.x == 0) {
+    out[0] = ok;
+    out[1] = bits & STAGE_LOST ? 1u : 0u;
+  }
 }
 
 }  // namespace
@@ -94,5 +111,22 @@ extern "C" __attribute__((visibility("default"))) int block_run(const uint8_t* i
   out[1] = hdr.err_info.v;
   out[2] = hdr.progress.v;
   out[3] = blocks;
+  return 0;
+}
+
+// A wait on a barrier that no copy was issued on; out: its result, STAGE_LOST, error word, its detail.
+extern "C" __attribute__((visibility("default"))) int lost_copy(uint32_t* out) {
+  uint8_t* dev = nullptr;
+  if (cudaMalloc(&dev, sizeof(QueueHdr) + 256) != cudaSuccess) return -4;
+  QueueHdr hdr{};
+  uint32_t* dout = reinterpret_cast<uint32_t*>(dev + sizeof(QueueHdr));
+  bool ok = cudaMemset(dev, 0, sizeof(QueueHdr) + 256) == cudaSuccess;
+  wait_for_nothing<<<1, 32>>>(reinterpret_cast<QueueHdr*>(dev), dout);
+  ok = ok && cudaDeviceSynchronize() == cudaSuccess && cudaMemcpy(&hdr, dev, sizeof(hdr), cudaMemcpyDeviceToHost) == cudaSuccess &&
+       cudaMemcpy(out, dout, 8, cudaMemcpyDeviceToHost) == cudaSuccess;
+  cudaFree(dev);
+  if (!ok) return -5;
+  out[2] = hdr.error.v;
+  out[3] = hdr.err_info.v;
   return 0;
 }

@@ -66,3 +66,9 @@ def test_the_visit_cap_ends_a_run_whose_ctas_never_wait(checks):
     # A CTA looks at the cap at its 16th visit at the latest, and then nobody claims another block.
     assert st["error"] == DERR_VISIT_LIMIT and st["info"] > 64, st
     assert st["visits"] < 4 * 0.75 * st["blocks"], st  # a visit sweeps up to four tiles
+
+
+def test_a_copy_that_does_not_arrive_ends_the_warp(checks):
+    out = (ctypes.c_uint32 * 4)()
+    assert checks.lost_copy(out) == 0
+    assert tuple(out) == (0, 1, DERR_TMA_TIMEOUT, 77)
