@@ -1059,7 +1059,15 @@ DTB_API dtb_status dtb_context_set_tuning(dtb_context ctx, const dtb_tuning* t) 
   nt.grid_percent = pct;
   nt.buckets = buckets;
   nt.bucket_tiles = width;
-  nt.chosen = true;
+  // A launch field selects the tile kernel for every size.  The pipeline's chunk size alone does not, and a call that names
+  // all of them at their defaults (what dtb_context_get_tuning says of a new context) returns to the choice by size.
+  const LaunchTuning def;
+  const bool any = t->ctas_per_sm || t->grid_percent || t->queue_buckets || t->bucket_width_pct || t->staging || t->warps_per_cta;
+  const bool all = t->ctas_per_sm && t->grid_percent && t->queue_buckets && t->bucket_width_pct && t->staging && t->warps_per_cta;
+  if (all && variant == def.variant && pct == def.grid_percent && buckets == def.buckets && width == def.bucket_tiles)
+    nt.chosen = false;
+  else if (any)
+    nt.chosen = true;
   ctx->tuning = nt;
   if (t->host_chunk_kpx > 0) ctx->host_chunk_px = (uint64_t)t->host_chunk_kpx * 1024ull;
   ctx->tuned.clear();

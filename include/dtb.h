@@ -108,8 +108,10 @@ DTB_API dtb_status dtb_sync(dtb_context ctx, void* stream);
  * one tile-width of path cost of the image (32 x its mean edge weight), 1..6400 (default 50);
  * staging: 1 = a visit stages its own tile, 2 = a warp stages the image box of its next tile while it visits
  * the current one (double-buffered shared memory; ctas_per_sm 2 or 3 only).
- * A context whose tuning was never set runs calls and plans of up to about 38 Mpx in another kernel (one CTA per 64 x 64
- * block); setting any field selects the tile kernel for every size. */
+ * A context whose launch fields were never set chooses by size: ns-mode calls, plans, host batches and waves of up to about
+ * 38 Mpx run in another kernel (one CTA per 64 x 64 block), larger ones in the tile kernel.  Setting any field but
+ * host_chunk_kpx selects the tile kernel for every size; naming all of them at their defaults, as
+ * dtb_context_get_tuning gives them for a new context, returns to the choice by size. */
 typedef struct dtb_tuning {
   int32_t ctas_per_sm;
   int32_t grid_percent;
