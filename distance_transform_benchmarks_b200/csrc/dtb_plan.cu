@@ -317,10 +317,10 @@ DTB_API dtb_status dtb_plan_autotune(dtb_plan p, void* stream, int32_t reps, dtb
   };
   // Coordinate search: (1) kernel variant (CTAs per SM x warps per CTA x staging) x grid share under the current
   // queue policy; (2) queue policy (FIFO; 8 or 16 buckets of 1/10, 1/4, 1/2 or 1 tile-width) under the best launch;
-  // (3) the variants again under the best policy.
+  // (3) the variants again under the best policy.  The block kernel knows none of these, so it is timed once, last,
+  // against the best of them, unless the caller chose a tuning; an earlier result of the autotuner does not shut it out.
   static const int kPercent[3] = {100, 75, 50};
   const LaunchTuning start = p->tuning;
-  if (use_blocks(ctx, MODE_NS, start, p->L.blocks)) trial(start);  // the block kernel
   for (int v = 0; v < NS_VARIANTS; ++v)
     for (int pc = 0; pc < 3; ++pc) {
       LaunchTuning t = start;
@@ -351,6 +351,12 @@ DTB_API dtb_status dtb_plan_autotune(dtb_plan p, void* stream, int32_t reps, dtb
       t.variant = v;
       trial(t);
     }
+  }
+  {
+    LaunchTuning blocks = start;  // kept as it was for the runs of this size class that are too large for the block kernel
+    blocks.chosen = false;
+    blocks.grid_percent = 100;
+    if (!ctx->tuning.chosen && use_blocks(ctx, MODE_NS, blocks, p->L.blocks)) trial(blocks);
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);

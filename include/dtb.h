@@ -166,8 +166,8 @@ DTB_API dtb_status dtb_gdt_batch(dtb_context ctx, int32_t n, const dtb_image* im
  * queue policies under the best launch, then the variants again under the best policy.  It keeps the fastest
  * in the plan and, for batches of the same size class (image count and tile count, each rounded up to a power
  * of two), in the context and in its autotuner cache file if one is set; and reports it.  Where the size allows the
- * kernel of one CTA per 64 x 64 block (see dtb_tuning), that one competes too and the report names the tile kernel's
- * unchanged tuning when it wins.  dtb_plan_get_tuning
+ * kernel of one CTA per 64 x 64 block (see dtb_tuning) and the context has no tuning of the caller's, that one competes
+ * too; when it wins, plan and report keep the tuning the plan began with.  dtb_plan_get_tuning
  * reports the plan's current tuning.  No reference counterpart: the reference fixes these choices
  * (dt/src/task_queue.cuh:23, dt/src/generalised_distance_transform_task.cu:184). */
 typedef struct dtb_plan_s* dtb_plan;
