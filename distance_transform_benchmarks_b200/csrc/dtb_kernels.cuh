@@ -720,26 +720,30 @@ __device__ __forceinline__ bool ref_halo_relax(const RefEdge<FMA>& re, float* T,
 }
 
 // The smallest value the tile's border can bring to each neighbour below the halo it was compared with: lane k returns
-// neighbour k's (left, right, top, bottom, then the corners tl, tr, bl, br) as float bits, KEY_NONE if nothing.
+// neighbour k's (left, right, top, bottom, then the corners tl, tr, bl, br) as float bits, KEY_NONE if nothing.  In a
+// tile of vw x vh < 32 pixels the last pixel of a side has no diagonal neighbour after it: its halo is infinite there, and
+// any value would be below it (lane 31's goes to a corner, which exists or not as a whole).
 template <bool FMA>
-__device__ __forceinline__ uint32_t ref_border_keys(const RefEdge<FMA>& re, const float* T, const float* E, const RefHalo& h) {
+__device__ __forceinline__ uint32_t ref_border_keys(const RefEdge<FMA>& re, const float* T, const float* E, const RefHalo& h, int vw,
+                                                    int vh) {
   const int lane = threadIdx.x & 31;
   uint32_t kc[4] = {KEY_NONE, KEY_NONE, KEY_NONE, KEY_NONE};  // tl, tr, bl, br
-  auto side = [&](float hh, float before, float after, const float* e, float px, uint32_t& k0, uint32_t& k2) -> uint32_t {
+  auto side = [&](float hh, float before, float after, const float* e, float px, int len, uint32_t& k0, uint32_t& k2) -> uint32_t {
     float o[3];
     halo3(o, hh, before, after);
     const float c0 = re.grad(e[lane], re.diagonal(px)), c1 = re.grad(e[TILE + lane], re.axial(px)),
                 c2 = re.grad(e[2 * TILE + lane], re.diagonal(px));
     uint32_t k = c1 < o[1] ? __float_as_uint(c1) : KEY_NONE;
-    const uint32_t u0 = c0 < o[0] ? __float_as_uint(c0) : KEY_NONE, u2 = c2 < o[2] ? __float_as_uint(c2) : KEY_NONE;
+    const uint32_t u0 = c0 < o[0] ? __float_as_uint(c0) : KEY_NONE;
+    const uint32_t u2 = c2 < o[2] && (lane + 1 < len || lane == TILE - 1) ? __float_as_uint(c2) : KEY_NONE;
     if (lane == 0) k0 = min(k0, u0); else k = min(k, u0);
     if (lane == TILE - 1) k2 = min(k2, u2); else k = min(k, u2);
     return __reduce_min_sync(~0u, k);
   };
-  const uint32_t kt = side(h.t, h.tl, h.tr, E + E_TOP * 3, T[lane], kc[0], kc[1]);
-  const uint32_t kb = side(h.b, h.bl, h.br, E + E_BOTTOM * 3, T[(TILE - 1) * RS + lane], kc[2], kc[3]);
-  const uint32_t kl = side(h.l, h.tl, h.bl, E + E_LEFT * 3, T[lane * RS], kc[0], kc[2]);
-  const uint32_t kr = side(h.r, h.tr, h.br, E + E_RIGHT * 3, T[lane * RS + TILE - 1], kc[1], kc[3]);
+  const uint32_t kt = side(h.t, h.tl, h.tr, E + E_TOP * 3, T[lane], vw, kc[0], kc[1]);
+  const uint32_t kb = side(h.b, h.bl, h.br, E + E_BOTTOM * 3, T[(TILE - 1) * RS + lane], vw, kc[2], kc[3]);
+  const uint32_t kl = side(h.l, h.tl, h.bl, E + E_LEFT * 3, T[lane * RS], vh, kc[0], kc[2]);
+  const uint32_t kr = side(h.r, h.tr, h.br, E + E_RIGHT * 3, T[lane * RS + TILE - 1], vh, kc[1], kc[3]);
   const uint32_t ktl = __reduce_min_sync(~0u, kc[0]), ktr = __reduce_min_sync(~0u, kc[1]);
   const uint32_t kbl = __reduce_min_sync(~0u, kc[2]), kbr = __reduce_min_sync(~0u, kc[3]);
   return lane == 0 ? kl : lane == 1 ? kr : lane == 2 ? kt : lane == 3 ? kb : lane == 4 ? ktl : lane == 5 ? ktr
@@ -987,7 +991,7 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
       act = (cl ? 1u : 0u) | (cr ? 2u : 0u) | (ct ? 4u : 0u) | (cb ? 8u : 0u) | ((ct & 1u) ? 16u : 0u) |
             ((ct >> (TILE - 1)) & 1u ? 32u : 0u) | ((cb & 1u) ? 64u : 0u) | ((cb >> (TILE - 1)) & 1u ? 128u : 0u);
     } else {
-      const uint32_t k = ref_border_keys<FMA>(re, T, sm.E, h);
+      const uint32_t k = ref_border_keys<FMA>(re, T, sm.E, h, vw, vh);
       act = __ballot_sync(~0u, k != KEY_NONE);
       key = __uint_as_float(k);
     }
