@@ -1,5 +1,4 @@
-"""Which kernel a call takes after which tuning, by the kernels that the profiler sees, and host batches of many chunks
-through either kernel."""
+"""Which kernel a call takes after which tuning, and host batches of many chunks through either kernel."""
 import numpy as np
 import pytest
 import torch
@@ -12,13 +11,11 @@ from tests.helpers import assert_images_eq
 pytestmark = pytest.mark.gpu
 
 
-def kernels_of(fn):
-    """Names of this library's map kernels that `fn` launched."""
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        fn()
-        torch.cuda.synchronize()
-    names = " ".join(e.key for e in prof.key_averages())
-    return {k for k in ("ggdt_block", "ggdt_persistent") if k in names}
+def kernel_of(stats, images):
+    """The kernel that made maps of wholly reached pictures with one seeded tile each: the tile kernel activates every other
+    tile at least once, the block kernel crosses the tiles of its 64 x 64 blocks without (in these tests it needs fewer
+    activations than there are tiles)."""
+    return "blocks" if stats["activations"] < stats["tiles"] - images else "tiles"
 
 
 def set_nothing(c):
@@ -44,21 +41,23 @@ def set_launch_then_chunk(c):
     c.set_tuning(host_chunk_kpx=24)
 
 
-@pytest.mark.parametrize("change,kernel", [(set_nothing, "ggdt_block"), (set_chunk, "ggdt_block"), (set_launch, "ggdt_persistent"),
-                                           (set_and_return, "ggdt_block"), (set_launch_then_chunk, "ggdt_persistent")])
+@pytest.mark.parametrize("change,kernel", [(set_nothing, "blocks"), (set_chunk, "blocks"), (set_launch, "tiles"),
+                                           (set_and_return, "blocks"), (set_launch_then_chunk, "tiles")])
 def test_the_chunk_size_alone_keeps_the_choice_by_size(change, kernel):
     c = dtb.Context(0)
     change(c)
-    img, mask, gamma = wl.config0()
-    ti, tm = torch.from_numpy(img).cuda(), torch.from_numpy(mask).cuda()
-    out = []
-    assert kernels_of(lambda: out.append(dtb.geodesic_distance_transform(ti, tm, gamma, ctx=c))) == {kernel}
-    assert_images_eq(out[0], orc.ggdt_ns(img, mask, gamma), "device call")
-    batch = wl.config3(seed=15, n=9, smin=20, smax=240)
-    hi, hm, hd = dtb.host_batch_arena([b[0] for b in batch], [b[1] for b in batch])
-    assert kernels_of(lambda: dtb.geodesic_distance_transform_batch(hi, hm, [b[2] for b in batch], dists=hd, ctx=c)) == {kernel}
-    for k, (i, m, g) in enumerate(batch):
-        assert_images_eq(hd[k], orc.ggdt_ns(i, m, g), "host image %d" % k)
+    img = wl.blobs_gray(3, 64, 64)
+    mask = np.zeros((64, 64), np.uint8)
+    mask[20, 40] = 1
+    want = orc.ggdt_ns(img, mask, 0.1)
+    d = dtb.geodesic_distance_transform(torch.from_numpy(img).cuda(), torch.from_numpy(mask).cuda(), 0.1, ctx=c)
+    assert_images_eq(d, want, "device call")
+    assert kernel_of(c.stats(), 1) == kernel
+    hi, hm, hd = dtb.host_batch_arena([img] * 9, [mask] * 9)
+    dtb.geodesic_distance_transform_batch(hi, hm, [0.1] * 9, dists=hd, ctx=c)
+    assert kernel_of(c.stats(), 9) == kernel
+    for k in range(9):
+        assert_images_eq(hd[k], want, "host image %d" % k)
     c.close()
 
 
