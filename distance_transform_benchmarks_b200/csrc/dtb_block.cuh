@@ -50,7 +50,8 @@ struct BlockCtl {
   uint32_t visits;     // tiles swept in this visit
   uint32_t done;       // visits of this CTA
   uint32_t phases, activations;  // counters of the run
-  ImgDesc desc;        // the block's image
+  uint32_t img;        // the block's image
+  ImgDesc desc;
 };
 struct BlockSmem {
   BlockTile tile[BLOCK_WARPS];
@@ -96,8 +97,8 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
     uint32_t key = KEY_NONE, pick = POP_NONE, got[BLOCK_SIDES] = {};
     bool stop = ld_volatile(&a.hdr->pending.v) + a.total == 0u;
     // After an error no block is claimed any more, ready or not.  The word is on a line that nobody writes, so its load
-    // comes back with the messages' (with the checks of the visit below, 512^2 gray takes 159.7 us instead of 158.8 and the
-    // 4096^2 maze 3.65 ms instead of 3.63).
+    // comes back with the messages' (with the check of the copies in the visit, 512^2 gray takes 158.2 us instead of 157.9
+    // and the 4096^2 maze 3.61 ms instead of 3.60).
     const uint32_t failed = ld_volatile(&a.hdr->error.v);
 #pragma unroll 4
     for (int i = lane; i < count; i += 32) {
@@ -140,8 +141,16 @@ __device__ __forceinline__ void block_next(const BlockRun& a, const ImgDesc* __r
       const uint32_t own = __ballot_sync(~0u, pick != POP_NONE && pick == prev);
       const int win = __ffs(own ? own : __ballot_sync(~0u, pick != POP_NONE && key == best)) - 1;
       if (!own) {
-        // (an image index out of range ends the run before the visit: ggdt_block)
-        const uint32_t img = min(ctl.owned_img[__shfl_sync(~0u, pick, win)], (uint32_t)a.n - 1u);
+        // The visit's descriptor and tensor maps are read through this index: a map that is none would end in a device fault.
+        const uint32_t img = ctl.owned_img[__shfl_sync(~0u, pick, win)];
+        if (img >= (uint32_t)a.n) {
+          if (lane == win) {
+            block_error(a, DERR_BAD_TILE, pick);
+            ctl.next = POP_NONE;
+          }
+          return;
+        }
+        if (lane == 0) ctl.img = img;
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&descs[img]);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&ctl.desc);
         for (int i = lane; i < (int)(sizeof(ImgDesc) / 4); i += 32) dst[i] = src[i];
@@ -335,7 +344,7 @@ constexpr uint32_t BLOCK_UNSAVED = 2u;
 // tiles stay in shared memory and are written when the CTA turns to another block (BLOCK_UNSAVED) or ends.
 // Returns false when a copy into the block's tiles did not arrive: the CTA then visits nothing more (STAGE_LOST).
 __device__ __forceinline__ bool block_visit_ns(const BlockRun& a, const CUtensorMap* __restrict__ tmaps, BlockSmem& sm,
-                                               uint32_t img, uint32_t blk, uint32_t& flags, const Queue& q, float (&wh)[TILE],
+                                               uint32_t blk, uint32_t& flags, const Queue& q, float (&wh)[TILE],
                                                float (&wv)[TILE], int& loaded, bool fill_only) {
   const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5);
   const float INF = f_inf();
@@ -351,7 +360,7 @@ __device__ __forceinline__ bool block_visit_ns(const BlockRun& a, const CUtensor
     sides = uniform(p.sides);
     const bool exists = (sides & 0x1000u) != 0u;
     const VisitBufs vb{t.img, t.Wv, nullptr, &t.bar, &t.bar, 1u, 1u, &flags};
-    if (exists && !rerun) stage_tile(vb, tmaps + 2 * img, tmaps + 2 * img + 1, dd.channels == 3, seed, p.x0, p.y0);
+    if (exists && !rerun) stage_tile(vb, tmaps + 2 * sm.ctl.img, tmaps + 2 * sm.ctl.img + 1, dd.channels == 3, seed, p.x0, p.y0);
     {
       float top = INF, bot = INF, lft = INF, rgt = INF;
       const float v = dd.v;
@@ -528,6 +537,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
       for (int i = lane; i < (int)(sizeof(ImgDesc) / 4); i += 32) reinterpret_cast<uint32_t*>(&sm.ctl.desc)[i] = src[i];
       if (lane == 0) {
         sm.ctl.next = (uint32_t)early;
+        sm.ctl.img = sm.ctl.owned_img[early];
         sm.ctl.first = 1u;
         sm.ctl.seed = sm.ctl.rerun = sm.ctl.nvis = 0u;
       }
@@ -545,14 +555,11 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
       flags &= ~BLOCK_UNSAVED;
       __syncwarp();
     }
-    if (next == POP_NONE) break;
-    // Whatever a copy reads through comes from these two words: a tensor map that is none would end in a device fault.
-    const uint32_t img = next < (uint32_t)count ? uniform(sm.ctl.owned_img[next]) : POP_NONE;
-    if (img >= (uint32_t)a.n) {
-      if (threadIdx.x == 0) block_error(a, DERR_BAD_TILE, next);
+    if (next >= (uint32_t)count) {  // POP_NONE, or not an index at all
+      if (next != POP_NONE && threadIdx.x == 0) block_error(a, DERR_BAD_TILE, next);
       break;
     }
-    if (!block_visit_ns(a, tmaps, sm, img, first + next * step, flags, q, wh, wv, loaded, early >= 0)) break;
+    if (!block_visit_ns(a, tmaps, sm, first + next * step, flags, q, wh, wv, loaded, early >= 0)) break;
     prev = next;
     early = -1;
   }
