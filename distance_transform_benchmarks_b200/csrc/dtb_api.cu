@@ -118,7 +118,6 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
   WarpSmemP& sm = warp_slot_p(smem_raw);
   warp_slot_init(sm);
   const QueueSched sch{q, states};
-  const int lane = threadIdx.x & 31;
   WarpStats ws;
   uint32_t pbits = 0;  // bit k: phase parity of box k's barrier; bit 2: the mask barrier's
   uint32_t k = 0;      // box of the tile being visited
@@ -504,9 +503,9 @@ static uint32_t block_grid(dtb_context ctx, const LaunchTuning& t, int ctas) {
 
 // Whether a run takes the block kernel: under the default tuning, up to as many blocks as its CTAs may own (9472 on 148
 // SMs, 38 Mpx).  Up to there chains of dependent visits bound the run.  ns-mode: the block kernel is faster or as fast
-// (tile against block kernel: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze 4.2 / 4.1,
+// (tile against block kernel, repeated calls on the same buffers: 512^2 gray 0.30 / 0.17 ms, 2048^2 gray 0.84 / 0.46, 4096^2 rgb8 1.72 / 1.12, 4096^2 maze 4.2 / 4.1,
 // 6016^2 rgb8 1.19 / 1.18, 48 images of 7 Mpx 0.80 / 0.75); with more work than warps the tile kernel's finer units win (128
-// images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5). 
+// images of 58 Mpx 2.8 / 3.2 ms, 512 images of 188 Mpx 5.8 / 7.5).
 // ns-mode only: a block kernel for eight neighbours was faster on small pictures (1023x777, lambda 0 / 0.5 / 1: 0.23 / 0.56 /
 // 0.80 ms against 0.40 / 0.69 / 0.91), no faster at lambda 0.5 on large ones (3648x2432 2.30 against 2.02), and stopped once
 // with an illegal instruction whose cause reading did not show, so it was taken out.

@@ -264,29 +264,29 @@ __device__ __forceinline__ BlockPlace block_place(const ImgDesc& dd, uint32_t bl
   return p;
 }
 
-// Writes the warp's tile, `stride` floats a row, to memory (row by row, coalesced).
-__device__ __forceinline__ void block_store_tile(const ImgDesc& dd, const BlockPlace& p, const float* B, int stride) {
+// Writes the warp's tile to memory (row by row, coalesced).
+__device__ __forceinline__ void block_store_tile(const ImgDesc& dd, const BlockPlace& p, const float* B) {
   const int lane = threadIdx.x & 31;
   if (lane < p.vw) {
     uint8_t* wb = dist_base(dd, p.y0, p.x0 + lane, 0u);
     const int64_t pitch = dd.dist_pitch;
 #pragma unroll 4
     for (int y = 0; y < TILE; ++y)
-      if (y < p.vh) *reinterpret_cast<float*>(wb + (int64_t)y * pitch) = B[y * stride + lane];
+      if (y < p.vh) *reinterpret_cast<float*>(wb + (int64_t)y * pitch) = B[y * W_STRIDE + lane];
   }
 }
 
 // Writes the lines of the warp's tile that lie on the block's border (`outer`: left, right, top, bottom) to memory.
-__device__ __forceinline__ void block_store_border(const ImgDesc& dd, const BlockPlace& p, uint32_t outer, const float* B, int stride) {
+__device__ __forceinline__ void block_store_border(const ImgDesc& dd, const BlockPlace& p, uint32_t outer, const float* B) {
   const int lane = threadIdx.x & 31;
   if (lane < p.vh) {
     float* row = dist_row(dd, p.y0 + lane) + p.x0;
-    if (outer & 1u) row[0] = B[lane * stride];
-    if (outer & 2u) row[TILE - 1] = B[lane * stride + TILE - 1];
+    if (outer & 1u) row[0] = B[lane * W_STRIDE];
+    if (outer & 2u) row[TILE - 1] = B[lane * W_STRIDE + TILE - 1];
   }
   if (lane < p.vw) {
     if (outer & 4u) dist_row(dd, p.y0)[p.x0 + lane] = B[lane];
-    if (outer & 8u) dist_row(dd, p.y0 + TILE - 1)[p.x0 + lane] = B[(TILE - 1) * stride + lane];
+    if (outer & 8u) dist_row(dd, p.y0 + TILE - 1)[p.x0 + lane] = B[(TILE - 1) * W_STRIDE + lane];
   }
 }
 
@@ -450,7 +450,7 @@ __device__ __forceinline__ bool block_visit_ns(const BlockRun& a, const CUtensor
       store_skew(B + lane * W_STRIDE, off, d);
       // The border lines go out at once: the checks that end the visit cover their way to L2.
       __syncwarp();
-      block_store_border(dd, block_place(dd, blk), sides >> 8, B, W_STRIDE);
+      block_store_border(dd, block_place(dd, blk), sides >> 8, B);
     }
     if (it >= (uint32_t)PHASE_LIMIT) {
       if (threadIdx.x == 0) set_error(q, DERR_PHASE_LIMIT, blk);
@@ -463,7 +463,7 @@ __device__ __forceinline__ bool block_visit_ns(const BlockRun& a, const CUtensor
   const uint32_t outer = (sides >> 8) & 15u;
   if (changed) flags |= BLOCK_UNSAVED;
   if (uniform(outer && (changed || sm.ctl.first))) {
-    if (!nph) block_store_border(dd, block_place(dd, blk), outer, B, W_STRIDE);
+    if (!nph) block_store_border(dd, block_place(dd, blk), outer, B);
     const float* E = t.E;
     const float bl = B[lane * W_STRIDE], br = B[lane * W_STRIDE + TILE - 1], bt = B[lane], bb = B[(TILE - 1) * W_STRIDE + lane];
     const float vl = __fadd_rn(bl, E[E_LEFT + lane]), vr = __fadd_rn(br, E[E_RIGHT + lane]);
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(BLOCK_WARPS * 32, CTAS)
     const uint32_t next = uniform(sm.ctl.next);
     if (next != prev && (flags & BLOCK_UNSAVED)) {
       const ImgDesc& dd = descs[sm.ctl.owned_img[prev]];
-      block_store_tile(dd, block_place(dd, first + prev * step), reinterpret_cast<const float*>(sm.tile[warp].img), W_STRIDE);
+      block_store_tile(dd, block_place(dd, first + prev * step), reinterpret_cast<const float*>(sm.tile[warp].img));
       flags &= ~BLOCK_UNSAVED;
       __syncwarp();
     }

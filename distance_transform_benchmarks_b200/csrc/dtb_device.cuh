@@ -71,7 +71,7 @@ struct alignas(64) ImgDesc {
   float l_grad;   // ref-mode: lambda
   int32_t mode;
   int32_t ref_fma;  // ref-mode: 1 = fma(l_grad, dI, fma(l_eucl, d, D)), 0 = left-to-right rounding
-  int32_t blocks_x, blocks_y;  // block kernel: blocks of 4 x 4 tiles
+  int32_t blocks_x, blocks_y;  // block kernel: blocks of BLOCK_TX x BLOCK_TY tiles
   uint32_t block_base;
   int32_t warm;  // block kernel: the map holds a fixpoint of some of the seeds already (serving: a seed edit)
 };
@@ -273,24 +273,12 @@ __device__ __forceinline__ void slot_write(const Queue& q, uint32_t b, uint32_t 
   }
 }
 
-// Bucket of an activation value `key` (distance units) for an image whose bucket width is 1 / inv_width.
-// (Idle workers waiting in another bucket give their tickets back within POLL_CHECK_NS and find the item.)
-__device__ __forceinline__ uint32_t bucket_of(const Queue& q, float key, float inv_width) {
-  if (q.nb_mask == 0) return 0;
-  const uint32_t base = ld_volatile(&q.hdr->base.v);
-  const float r = key * inv_width;  // absolute bucket; NaN / huge values land in the last bucket
-  uint32_t rel = q.nb_mask;
-  if (r < 4.0e9f) {
-    const uint32_t kb = (uint32_t)r;
-    rel = kb <= base ? 0u : min(kb - base, q.nb_mask);
-  }
-  return (base + rel) & q.nb_mask;
-}
-
-// Bucket of an activation value relative to a base the caller read (bucket_of with the base given).
+// Bucket of an activation value `key` (distance units) for an image whose bucket width is 1 / inv_width, relative to a
+// base the caller read.  (Idle workers waiting in another bucket give their tickets back within POLL_CHECK_NS and find
+// the item.)
 __device__ __forceinline__ uint32_t bucket_at(const Queue& q, float key, float inv_width, uint32_t base) {
   if (q.nb_mask == 0) return 0;
-  const float r = key * inv_width;
+  const float r = key * inv_width;  // absolute bucket; NaN / huge values land in the last bucket
   uint32_t rel = q.nb_mask;
   if (r < 4.0e9f) {
     const uint32_t kb = (uint32_t)r;

@@ -30,10 +30,11 @@ constexpr int REF_CTAS = 2;  // resident CTAs per SM of the ref-mode tile kernel
                              // registers a thread; 94 KB of shared memory a CTA)
 // ns-mode tile kernel variants: CTAs per SM, whether a warp stages its next tile ahead (22.4 KB of shared memory a
 // warp instead of 17.8 KB), and warps per CTA.  Registers per thread follow the warps per SM: 8 -> 255, 12 -> 168,
-// 16 -> 128.  The 227 KB of an SM hold 12 warps at 17.8 KB and 8 that stage ahead, so of the shapes with 16 warps 12
-// are resident and 3 x 4 ahead runs as 2 x 4: resident_workers sizes the grid by the occupancy, and saved tuning
-// entries stay valid.  The 12- and 16-warp shapes come in several CTA sizes (2 x 6, 3 x 4, 6 x 2; 2 x 8, 4 x 4), which
-// differ in how the SM's warps are grouped and scheduled only.
+// 16 -> 128.  The 227 KB of an SM hold 12 warps at 17.8 KB and 8 that stage ahead, so 4 x 4 runs as 3 x 4,
+// 2 x 8 as 1 x 8 and 3 x 4 ahead as 2 x 4, the first two with fewer registers than they could have (512 images: 3 x 4 4.33
+// ms, 4 x 4 5.08, 2 x 8 6.27): resident_workers sizes the grid by the occupancy, and saved tuning entries stay valid.
+// The 12-warp shapes come in several CTA sizes (2 x 6, 3 x 4, 6 x 2), which differ in how the SM's warps are grouped and
+// scheduled only.
 struct NsVariant {
   int ctas;
   bool ahead;

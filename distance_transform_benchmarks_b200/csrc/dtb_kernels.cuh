@@ -617,6 +617,7 @@ constexpr float REF_SQ2 = 1.41421354f;  // sqrtf(2.f), reference generalised_dis
 // `diagonal` of the source's distance, then `grad` with the edge's word (|dI|, or l_grad * |dI| rounded by itself
 // without FMA).  An edge that does not exist has an infinite word, so its candidate is infinite, or NaN when l_grad is
 // 0, and fminf and < pass over both.
+// (the host's pass over the constructor, whose arguments do not depend on the template, does not know __fmul_rn)
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 template <bool FMA>
 struct RefEdge {
@@ -783,7 +784,7 @@ __device__ __forceinline__ bool ref_phase(const RefEdge<FMA>& re, float (&d)[TIL
   return __any_sync(~0u, ch);
 }
 
-// Loads the tile (and with `edges` the phase's edge words) in the column or row layout.
+// Loads the tile in the column or row layout.
 __device__ __forceinline__ void ref_load_tile(float (&d)[TILE], const float* T, bool col) {
   const int lane = threadIdx.x & 31;
   if (col) {
@@ -835,32 +836,30 @@ __device__ __forceinline__ bool ref_chain_low(const RefEdge<FMA>& re, const floa
   return __any_sync(~0u, low);
 }
 
-// Runs phases over the tile in t.img (T) until it is converged or `limit` phases have run; `col` is the layout to start
-// with, and to go on with.  Adds the phases to nph; whether the tile is not converged yet.  `changed` is set when a
-// value fell.
+// Runs phases over the tile in t.img (T), a column phase first, until it is converged or PHASE_LIMIT phases have run; nph
+// counts them.  Whether the tile is not converged; `changed` is set when a value fell.
 template <bool FMA>
-__device__ __forceinline__ bool ref_solve(const RefEdge<FMA>& re, RefTile& t, bool& col, uint32_t limit, uint32_t& nph, bool& changed) {
+__device__ __forceinline__ bool ref_solve(const RefEdge<FMA>& re, RefTile& t, uint32_t& nph, bool& changed) {
   const int lane = threadIdx.x & 31;
   float* T = reinterpret_cast<float*>(t.img);
   float d[TILE], c[TILE], p[TILE], n[TILE];
+  bool col = true;
   ref_load_tile(d, T, col);
-  for (uint32_t k = 0;; ) {
+  for (;;) {
     ref_load_edges(c, p, n, t, col);
     const bool ch = ref_phase<FMA>(re, d, c, p, n);
     changed |= ch;
     ++nph;
-    ++k;
     if (ch) {
       ref_store_tile(T, d, col);
       __syncwarp();
     }
     col = !col;
-    if (ch && k >= limit) return true;
     ref_load_tile(d, T, col);
     __syncwarp();
     // A phase without change: the other layout's chain edges decide.
     if (!ch && !ref_chain_low<FMA>(re, d, col ? t.V + lane : t.Hh + lane * RS, col ? RS : 1)) return false;
-    if (k >= limit) return true;
+    if (nph >= (uint32_t)PHASE_LIMIT) return true;
   }
 }
 
@@ -973,8 +972,7 @@ __device__ __forceinline__ void visit_ref(const ImgDesc& dd, const CUtensorMap* 
   bool any = ref_halo_relax<FMA>(re, T, sm.E, h, vw, vh);
   uint32_t nph = 0;
   if (any || seed) {
-    bool col = true;
-    if (ref_solve<FMA>(re, sm, col, (uint32_t)PHASE_LIMIT, nph, any) && lane == 0) set_error(sch.q, DERR_PHASE_LIMIT, tile);
+    if (ref_solve<FMA>(re, sm, nph, any) && lane == 0) set_error(sch.q, DERR_PHASE_LIMIT, tile);
   }
 
   // Neighbours to activate (bit k = neighbour k as in ndx_l / ndy_l) and the value each is activated at: the ones the

@@ -98,8 +98,9 @@ DTB_API dtb_status dtb_sync(dtb_context ctx, void* stream);
  * (dt/src/task_queue.cuh:23, dt/src/block_priority.cu:71-155) and 4 blocks of one warp per SM
  * (dt/src/generalised_distance_transform_task.cu:184).  0 keeps a field's current value.
  * ctas_per_sm and warps_per_cta: the launch shape, one warp per 32 x 32 tile visit; (2, 4), (3, 4), (4, 4),
- * (6, 2), (2, 6) or (2, 8) -- 8, 12 or 16 warps per SM, registers per thread 255 / 168 / 128 (with only
- * ctas_per_sm given, warps_per_cta stays if it fits, else becomes 4);
+ * (6, 2), (2, 6) or (2, 8), built for 8, 12 or 16 warps per SM (255 / 168 / 128 registers per thread); the shared memory
+ * of an SM holds 12 warps (8 with staging 2), so (4, 4) runs as three CTAs, (2, 8) as one, and (3, 4) with staging 2 as
+ * two (with only ctas_per_sm given, warps_per_cta stays if it fits, else becomes 4);
  * grid_percent: share of the co-resident CTAs launched, 1..100 (fewer workers re-visit fewer tiles on
  * narrow fronts); host_chunk_kpx: pixels (in units of 1024) per chunk of the pipeline that serves batches in
  * host memory (host-to-device copies, tile runs on two alternating compute lanes and device-to-host copies of
