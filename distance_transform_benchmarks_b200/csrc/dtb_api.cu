@@ -637,6 +637,9 @@ static dtb_status run_rounds(dtb_context ctx, uint8_t* dbase, const ScratchLayou
   uint8_t* cur = dbase + L.o_act;
   uint8_t* nxt = dbase + L.o_act + total;
   uint32_t* changed = reinterpret_cast<uint32_t*>(dbase + L.o_chg);
+  RoundStatus* st = nullptr;
+  dtb_status s = round_status(ctx, &st);
+  if (s != DTB_OK) return s;
   DTB_CUDA(ctx, cudaMemsetAsync(hdr, 0, sizeof(QueueHdr), stream));
   *nrounds = 0;
   if (total == 0) return DTB_OK;
@@ -648,9 +651,6 @@ static dtb_status run_rounds(dtb_context ctx, uint8_t* dbase, const ScratchLayou
   // dt/src/generalised_distance_transform_blocks.cu:149-151), so per-tile round counters count the same rounds.
   if (mode != MODE_NS) DTB_CUDA(ctx, cudaMemsetAsync(cur, 1, total, stream));
   int32_t* counts = ctx->count_rounds ? ctx->dround_counts : nullptr;
-  RoundStatus* st = nullptr;
-  dtb_status s = round_status(ctx, &st);
-  if (s != DTB_OK) return s;
   const uint32_t blocks = (total + ROUND_WPC - 1) / ROUND_WPC;
   for (bool more = true; more;) {
     DTB_CUDA(ctx, cudaMemsetAsync(changed, 0, 4 * ROUND_BATCH, stream));
@@ -780,6 +780,12 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
   ScratchLayout L = layout_for(n, total, resident_workers(ctx, mode, tuning), rounds,
                                rounds ? 1u : (uint32_t)tuning.buckets);
   L.blocks = count_blocks(jobs);
+  // Every allocation before the first kernel: a call that fails for want of memory leaves none running on its buffers.
+  if (!ctx->hhdr && cudaHostAlloc((void**)&ctx->hhdr, sizeof(QueueHdr), cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->hhdr = nullptr;
+    return fail(ctx, DTB_ERR_OUT_OF_MEMORY, "cudaHostAlloc of the status header failed");
+  }
   if ((s = grow(ctx, &ctx->dscratch, &ctx->dscratch_size, L.bytes)) != DTB_OK) return s;
   uint8_t* dbase = reinterpret_cast<uint8_t*>(ctx->dscratch);
   if ((s = build_tables(ctx, jobs, L, ctx->hstage)) != DTB_OK) return s;
@@ -816,11 +822,6 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
   ctx->last_hdr = reinterpret_cast<QueueHdr*>(dbase + L.o_hdr);
   // The status follows the work on its stream into pinned memory, so a synchronous call waits for the GPU once (a
   // separate read after the wait cost 18 us of the 83 of a 97x61 call).
-  if (!ctx->hhdr && cudaHostAlloc((void**)&ctx->hhdr, sizeof(QueueHdr), cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    ctx->hhdr = nullptr;
-    return fail(ctx, DTB_ERR_OUT_OF_MEMORY, "cudaHostAlloc of the status header failed");
-  }
   DTB_CUDA(ctx, cudaMemcpyAsync(ctx->hhdr, ctx->last_hdr, sizeof(QueueHdr), cudaMemcpyDeviceToHost, stream));
   ctx->last_stream = stream;
   ctx->stats = dtb_stats{};
