@@ -710,7 +710,6 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
   // Serialise with a previous asynchronous call on another stream (the scratch is shared; host-buffer pipeline
   // calls have their own).
   if (ctx->async_pending && ctx->last_stream != stream) DTB_CUDA(ctx, cudaStreamSynchronize(ctx->last_stream));
-  ctx->async_pending = false;
 
   bool all_host = n > 0 && !(flags & DTB_FLAG_ROUNDS);
   for (int i = 0; i < n && all_host; ++i)
@@ -819,16 +818,17 @@ dtb_status run_jobs(dtb_context ctx, const std::vector<Job>& jobs_in, const dtb_
                                     (size_t)u->height, kind, stream));
   }
 
-  ctx->last_hdr = reinterpret_cast<QueueHdr*>(dbase + L.o_hdr);
   // The status follows the work on its stream into pinned memory, so a synchronous call waits for the GPU once (a
   // separate read after the wait cost 18 us of the 83 of a 97x61 call).
-  DTB_CUDA(ctx, cudaMemcpyAsync(ctx->hhdr, ctx->last_hdr, sizeof(QueueHdr), cudaMemcpyDeviceToHost, stream));
+  DTB_CUDA(ctx, cudaMemcpyAsync(ctx->hhdr, dbase + L.o_hdr, sizeof(QueueHdr), cudaMemcpyDeviceToHost, stream));
   ctx->last_stream = stream;
-  ctx->stats = dtb_stats{};
-  ctx->stats.tiles = total;
-  ctx->stats.rounds = nrounds;
+  ctx->call_stats = dtb_stats{};
+  ctx->call_stats.tiles = total;
+  ctx->call_stats.rounds = nrounds;
+  ctx->stats = ctx->call_stats;
   ctx->timed = timed;
   ctx->async_pending = true;
+  ctx->pipe_last = false;
   if ((flags & DTB_FLAG_ASYNC) && !host_io) return DTB_OK;
   return dtb_sync(ctx, stream);
 }
@@ -1084,20 +1084,30 @@ DTB_API dtb_status dtb_sync(dtb_context ctx, void* stream) {
   if (!ctx) return DTB_ERR_INVALID_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   DTB_CUDA(ctx, cudaStreamSynchronize(st));
-  if (ctx->pipe_pending) {
-    DTB_CUDA(ctx, cudaEventSynchronize(ctx->ev_pipe_done));  // the last call's end (copies out run in call order)
-    return finish_pipeline(ctx);
+  // The last device call and the host-buffer batches since the last look may both be open: both are waited for, the first
+  // error is reported, and the statistics are those of whichever came last.
+  dtb_status s = DTB_OK;
+  if (ctx->async_pending) {
+    // The call's header came back on its own stream (run_jobs); another stream's synchronisation says nothing about it.
+    if (st != ctx->last_stream) DTB_CUDA(ctx, cudaStreamSynchronize(ctx->last_stream));
+    ctx->async_pending = false;
+    s = status_of(ctx, *ctx->hhdr, &ctx->call_stats);
+    if (ctx->timed) {
+      float ms = 0.0f;
+      DTB_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
+      ctx->call_stats.kernel_ms = ms;
+      ctx->timed = false;
+    }
+    if (!ctx->pipe_last || !ctx->pipe_pending) ctx->stats = ctx->call_stats;
   }
-  if (!ctx->async_pending) return DTB_OK;
-  ctx->async_pending = false;
-  // The call's header came back on its own stream (run_jobs); another stream's synchronisation says nothing about it.
-  const dtb_status s = st == ctx->last_stream ? status_of(ctx, *ctx->hhdr, &ctx->stats)
-                                              : read_device_status(ctx, ctx->last_hdr, &ctx->stats);
-  if (ctx->timed) {
-    float ms = 0.0f;
-    DTB_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
-    ctx->stats.kernel_ms = ms;
-    ctx->timed = false;
+  if (ctx->pipe_pending) {
+    const dtb_stats call = ctx->stats;
+    const std::string msg = ctx->msg;
+    DTB_CUDA(ctx, cudaEventSynchronize(ctx->ev_pipe_done));  // the last batch's end (copies out run in call order)
+    const dtb_status ps = finish_pipeline(ctx);
+    if (!ctx->pipe_last) ctx->stats = call;
+    if (s == DTB_OK) s = ps;
+    else ctx->msg = msg;
   }
   return s;
 }

@@ -339,7 +339,7 @@ dtb_status run_host_pipeline(dtb_context ctx, std::vector<Job> jobs, const dtb_i
   ctx->pipe_tiles += total_all;
   ctx->pipe_chunks += (uint64_t)nchunks;
   ctx->pipe_pending = true;
-  ctx->async_pending = false;
+  ctx->pipe_last = true;
   if (flags & DTB_FLAG_ASYNC) return DTB_OK;  // dtb_sync(ctx, stream) waits and reports
   DTB_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->ev_pipe_done, 0));
   DTB_CUDA(ctx, cudaStreamSynchronize(stream));

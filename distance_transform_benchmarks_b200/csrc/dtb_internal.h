@@ -145,9 +145,9 @@ struct dtb_context_s {
   std::vector<uint8_t> hstage;
   std::string msg;
   dtb_stats stats{};
-  // Asynchronous bookkeeping: header of the last enqueued run and the stream it ran on.
-  dtb::QueueHdr* last_hdr = nullptr;
-  dtb::QueueHdr* hhdr = nullptr;  // pinned copy of it, written on that stream
+  dtb_stats call_stats{};  // of the last device call, until dtb_sync has its counters
+  // Asynchronous bookkeeping: header of the last enqueued run (pinned, written on its stream) and that stream.
+  dtb::QueueHdr* hhdr = nullptr;
   cudaStream_t last_stream = nullptr;
   bool async_pending = false;
   cudaEvent_t ev[2] = {nullptr, nullptr};  // DTB_FLAG_TIMING: around the tile kernel
@@ -164,6 +164,7 @@ struct dtb_context_s {
   dtb::QueueHdr* dpipe = nullptr;
   cudaEvent_t ev_pipe_done = nullptr;
   bool pipe_pending = false;
+  bool pipe_last = false;  // the last call was one of them, not a device call
   uint64_t pipe_tiles = 0, pipe_chunks = 0, pipe_h2d = 0, pipe_d2h = 0;
   // Host-buffer pipeline: two sets of device staging + chunk scratch used by alternate calls, so that a call's
   // copies in overlap the previous call's copies out; set i is free once ev_pset_free[i] (its last call's end)
