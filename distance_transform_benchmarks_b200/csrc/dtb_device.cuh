@@ -443,7 +443,7 @@ __device__ __forceinline__ uint32_t queue_try_pop(const Queue& q) {
 // Correctly rounded square root of x >= 1 (or infinite), without branches.  The hardware approximation s is within one
 // ulp, and Tuckerman's test picks the right neighbour: the rounded root r is the float with r * pred(r) < x <= r * succ(r),
 // whose two products a fused multiply-add compares with x exactly.  Equal to __fsqrt_rn for every float from 1 up
-// (checked exhaustively); __fsqrt_rn's special cases are a branch per root, which kept the roots of a tile from overlapping
+// (tests/cuda/sqrt_checks.cu compares them all); __fsqrt_rn's special cases are a branch per root, which kept the roots of a tile from overlapping
 // (59 cycles a root in a row of independent ones, 21 here).
 __device__ __forceinline__ float sqrt_ge1(float x) {
   float s;
